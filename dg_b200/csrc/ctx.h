@@ -15,6 +15,7 @@
 #include "device/common.cuh"
 #include "device/limiter_gated.cuh"
 #include "device/sensor.h"
+#include "device/tile2d_cols.cuh"
 
 namespace dgb {
 // Dynamic shared memory above 48 KB is opted into per kernel, and cudaFuncSetAttribute acts on the
@@ -65,7 +66,11 @@ struct dgb_ctx {
   bool rowmajor = false;  // structured row-major grid: tiled limiter passes
   bool chain1d = false;   // 1D elements in chain order: fused residual + limiter stages
   bool fused_lim = false; // row-major grid, hrl / m2l: both limiter passes in one kernel (opt-in)
-  CUtensorMap mapA, mapB, mapC;  // TMA descriptors of the state buffers (tiled kernel)
+  CUtensorMap mapA, mapB, mapC;  // TMA descriptors of the state buffers (mixed, DMMA and many-Y tiles)
+  // structured 2D grids: the residual with one thread per (element, quadrature column)
+  bool cols = false, cols_tma = false;
+  CUtensorMap colA, colB, colC;    // its TMA descriptors
+  dgb::ColTab col_step, col_raw;   // its tables: stage update, residual
   double hx = 0, hy = 0;
   size_t nstate = 0;
   dgb::Consts cs;

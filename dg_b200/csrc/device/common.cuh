@@ -49,7 +49,7 @@ struct DevScalars {
   double dt_fixed;             // fixed step (> 0) or 0 for the CFL step
 };
 
-enum { FLAG_NONFINITE = 1u, FLAG_DT_SMALL = 2u };
+enum { FLAG_NONFINITE = 1u, FLAG_DT_SMALL = 2u, FLAG_TIMEOUT = 4u };
 
 // Programmatic dependent launch (a kernel launched with programmatic stream serialization may be
 // scheduled before its predecessor in the stream has finished): pdl_wait blocks until the

@@ -91,8 +91,6 @@ struct TileDims {
   static_assert(off_tile % 128 == 0 && off_face % 128 == 0, "TMA destinations must be 128-byte aligned");
 };
 
-enum { FLAG_TIMEOUT = 4u };
-
 // Unrolling of the outer quadrature-column loop of the volume terms.  Fully unrolled, the
 // straight-line kernel body outgrows the instruction cache once several warps per scheduler run
 // different parts of it; rolled, the column index is warp-uniform and the tables stay

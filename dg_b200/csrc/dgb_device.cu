@@ -38,6 +38,9 @@ int limit1d_many_y(dgb_ctx* c, const double* in, double* out);
 int residual2d_many_y(dgb_ctx* c, const StageArgs& a, int mode);
 int limit2d_many_y(dgb_ctx* c, double* U);
 int upload_many_y_tables(const Consts& cs, int D, int p);
+// structured 2D grids, up to three mass fractions (dgb_tile.cu)
+int residual2d_cols(dgb_ctx* c, const StageArgs& a, int mode);
+void cols_setup(dgb_ctx* c);
 }  // namespace dgb
 #include "host/host.h"
 #include "ctx.h"
@@ -235,48 +238,16 @@ bool dgb::encode_state_map(dgb_ctx* c, double* ptr, CUtensorMap* map, int tw, in
 
 namespace {
 
-// NY passive mass fractions (1D or tiled 2D, FP64 form; checked at create)
+// NY passive mass fractions in 1D
 template <int MODE, int NY>
 int residual_ny(dgb_ctx* c, const StageArgs& a) {
-  if (c->tile_tma) {  // full tiles, then the strips outside them (if any) with the generic kernel
-#define T2Y(P, F)                                                               \
-  case P * 10 + F:                                                              \
-    launch_tile2d<P, F, MODE, NY>(c, a);                                        \
-    if (c->nleft) launch_res2d<P, F, MODE, NY>(c, a, c->left, c->nleft);        \
-    return 0;
-    switch (c->p * 10 + c->flux) {
-      T2Y(1, 0) T2Y(1, 2) T2Y(2, 0) T2Y(2, 2) T2Y(3, 0) T2Y(3, 2)
-      default: return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (p, flux) with mass fractions");
-    }
-#undef T2Y
-  }
-  if (c->D == 1) {
 #define R1Y(P, F) case P * 10 + F: launch_res1d<P, F, MODE, NY>(c, a); return 0;
-    switch (c->p * 10 + c->flux) {
-      R1Y(1, 0) R1Y(1, 1) R1Y(1, 2) R1Y(2, 0) R1Y(2, 1) R1Y(2, 2) R1Y(3, 0) R1Y(3, 1) R1Y(3, 2)
-      default: break;
-    }
+  switch (c->p * 10 + c->flux) {
+    R1Y(1, 0) R1Y(1, 1) R1Y(1, 2) R1Y(2, 0) R1Y(2, 1) R1Y(2, 2) R1Y(3, 0) R1Y(3, 1) R1Y(3, 2)
+    default: break;
+  }
 #undef R1Y
-  }
   return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (p, flux) with mass fractions");
-}
-
-// the full tiles with the tiled kernel, then the elements outside them (right and top strips of a
-// grid whose extents are not tile multiples) with the generic kernel; disjoint outputs, both read
-// the stage input's neighbours from global memory
-template <int P, int FLUX, int MODE>
-int tiles_then_strips(dgb_ctx* c, const StageArgs& a) {
-  if constexpr (P == 2 && MODE != MODE_RESIDUAL) {
-    if (c->tile_tma && c->tile_dmma) {
-      launch_tile2d_dmma<FLUX, MODE>(c, a);
-      if (c->nleft) launch_res2d<P, FLUX, MODE>(c, a, c->left, c->nleft);
-      return 0;
-    }
-  }
-  if (c->tile_tma) launch_tile2d<P, FLUX, MODE>(c, a);
-  else launch_tile2d<P, FLUX, MODE, 0, false, false>(c, a);
-  if (c->nleft) launch_res2d<P, FLUX, MODE>(c, a, c->left, c->nleft);
-  return 0;
 }
 
 template <int MODE>
@@ -294,19 +265,24 @@ int residual_dispatch(dgb_ctx* c, const StageArgs& a) {
       default: return set_error(DGB_ERR_UNSUPPORTED, "mixed form: p = 1..3 with Rusanov or Roe");
     }
   }
-  if (c->gamcons) {  // GAMCONS: tiled 2D or 1D, FP64 form, no mass fractions (checked at create)
-    if (c->D == 2) {  // full tiles, then the strips outside them (if any) with the generic kernel
-#define T2G(P, F)                                                               \
-  case P * 10 + F:                                                              \
-    launch_tile2d<P, F, MODE, 0, true>(c, a);                                   \
-    if (c->nleft) launch_res2d<P, F, MODE, 0, true>(c, a, c->left, c->nleft);   \
-    return 0;
-      switch (c->p * 10 + c->flux) {
-        T2G(1, 0) T2G(1, 2) T2G(2, 0) T2G(2, 2) T2G(3, 0) T2G(3, 2)
-        default: return set_error(DGB_ERR_UNSUPPORTED, "no GAMCONS residual kernel for this (p, flux)");
+  if (c->cols) {
+    if constexpr (MODE != MODE_RESIDUAL) {
+      if (c->tile_tma && c->tile_dmma && c->p == 2 && c->nmass == 0 && !c->gamcons) {
+        // p = 2 FP64 stages on the FP64 tensor cores (opt-in): the full tiles, then the elements
+        // outside them with the generic kernel
+        if (c->flux == DGB_FLUX_ROE) {
+          launch_tile2d_dmma<2, MODE>(c, a);
+          if (c->nleft) launch_res2d<2, 2, MODE>(c, a, c->left, c->nleft);
+        } else {
+          launch_tile2d_dmma<0, MODE>(c, a);
+          if (c->nleft) launch_res2d<2, 0, MODE>(c, a, c->left, c->nleft);
+        }
+        return 0;
       }
-#undef T2G
     }
+    return residual2d_cols(c, a, MODE);
+  }
+  if (c->gamcons) {  // GAMCONS in 1D, FP64 form, no mass fractions (checked at create)
 #define R1G(P, F) case P * 10 + F: launch_res1d<P, F, MODE, 0, true>(c, a); return 0;
     switch (c->p * 10 + c->flux) {
       R1G(1, 0) R1G(1, 1) R1G(1, 2) R1G(2, 0) R1G(2, 1) R1G(2, 2) R1G(3, 0) R1G(3, 1) R1G(3, 2)
@@ -320,18 +296,6 @@ int residual_dispatch(dgb_ctx* c, const StageArgs& a) {
       case 2: return residual_ny<MODE, 2>(c, a);
       case 3: return residual_ny<MODE, 3>(c, a);
       default: return c->D == 1 ? residual1d_many_y(c, a, MODE) : residual2d_many_y(c, a, MODE);
-    }
-  }
-  if (c->tiled) {
-    const int key = c->p * 10 + c->flux;
-    switch (key) {
-      case 10: return tiles_then_strips<1, 0, MODE>(c, a);
-      case 12: return tiles_then_strips<1, 2, MODE>(c, a);
-      case 20: return tiles_then_strips<2, 0, MODE>(c, a);
-      case 22: return tiles_then_strips<2, 2, MODE>(c, a);
-      case 30: return tiles_then_strips<3, 0, MODE>(c, a);
-      case 32: return tiles_then_strips<3, 2, MODE>(c, a);
-      default: break;
     }
   }
 #define R2(P, F) case P * 10 + F: launch_res2d<P, F, MODE>(c, a); return 0;
@@ -1001,6 +965,8 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
   c->tiled = c->rowmajor && P.p <= 3 && P.nx >= TILE_W && P.ny >= tile_h_for(P.p, P.N_Y);
   c->tile_tma = c->tiled && P.nx % 2 == 0;
   c->tiled_full = c->tile_tma && P.nx % TILE_W == 0 && P.ny % tile_h_for(P.p, P.N_Y) == 0;
+  // structured grids, up to three mass fractions: the residual of tile2d_cols.cuh on any extents
+  c->cols = c->rowmajor && P.p <= 3 && P.N_Y <= 3;
   // opt-in: measured slower than the two tiled passes on 512 x 256, p = 2 (64 vs 55 us per stage)
   c->fused_lim = c->rowmajor && (P.limiter == DGB_LIM_HRL || P.limiter == DGB_LIM_M2L) &&
                  std::getenv("DGB_FUSED_LIMITER") != nullptr && P.N_Y == 0;
@@ -1099,6 +1065,7 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
   std::memset(&c->mapA, 0, sizeof(CUtensorMap));
   std::memset(&c->mapB, 0, sizeof(CUtensorMap));
   std::memset(&c->mapC, 0, sizeof(CUtensorMap));
+  for (CUtensorMap* m : {&c->colA, &c->colB, &c->colC}) std::memset(m, 0, sizeof(CUtensorMap));
   if (c->tile_tma) {
     // row starts must be 16-byte aligned for TMA: nx is even and ld a multiple of 64
     const int th = tile_h_for(P.p, P.N_Y);
@@ -1108,6 +1075,7 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
       c->tile_tma = c->tiled_full = false;  // plain tile loads
     }
   }
+  if (c->cols) cols_setup(c);
   if (c->tiled && !c->tiled_full) {
     // the right strip (rows of the full tiles) and the top strip (all columns), in element order
     const int th = tile_h_for(P.p, P.N_Y), nxt = P.nx / TILE_W * TILE_W, nyt = P.ny / th * th;

@@ -1,0 +1,146 @@
+// The tiled 2D residual of structured row-major grids (device/tile2d_cols.cuh): its tables, its
+// dispatch over order, flux and field set, and its launches.
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "../../include/dgb.h"
+#include "device/kernels.cuh"
+#include "device/tile2d_cols.cuh"
+#include "host/host.h"
+#include "launch.h"
+
+namespace dgb {
+
+// Tables of the problem with constants cs: for the stage update (M1^-1 and 1/J folded in), or for
+// the residual itself (raw: neither).
+ColTab make_col_tab(const Consts& cs, bool raw) {
+  ColTab t;
+  std::memset(&t, 0, sizeof(t));
+  const int n1 = cs.n1, ng1 = cs.ng1;
+  std::vector<double> M((size_t)n1 * n1, 0.0);  // 1D mass matrix of the reference element, inverted
+  for (int i = 0; i < n1; ++i)
+    for (int j = 0; j < n1; ++j) {
+      if (raw) M[i + (size_t)j * n1] = i == j ? 1.0 : 0.0;
+      else
+        for (int g = 0; g < ng1; ++g) M[i + (size_t)j * n1] += cs.wq[g] * cs.Bq[g][i] * cs.Bq[g][j];
+    }
+  if (!raw) invert(M, n1);
+  auto fold = [&](const double* row, int i) {
+    double s = 0;
+    for (int k = 0; k < n1; ++k) s += M[i + (size_t)k * n1] * row[k];
+    return s;
+  };
+  const double jx = raw ? cs.J : 1.0;
+  for (int g = 0; g < ng1; ++g)
+    for (int i = 0; i < n1; ++i) {
+      t.B1[g][i] = cs.Bq[g][i];
+      t.Dx[g][i] = cs.ixx * cs.Dq[g][i];
+      t.Dy[g][i] = cs.iyy * cs.Dq[g][i];
+      t.LB[g][i] = cs.wq[g] * fold(cs.Bq[g], i);
+      t.LD[g][i] = cs.wq[g] * fold(cs.Dq[g], i);
+      t.XD[g][i] = jx * cs.ixx * cs.wq[g] * fold(cs.Dq[g], i);
+      t.XB[g][i] = jx * cs.iyy * cs.wq[g] * fold(cs.Bq[g], i);
+      t.XS[g][i] = jx * cs.wq[g] * fold(cs.Bq[g], i);
+    }
+  for (int g = 0; g < n1; ++g)
+    for (int i = 0; i < n1; ++i) {
+      t.BF[g][i] = cs.Bf[g][i];
+      t.LF[g][i] = 0.5 * cs.wf[g] * fold(cs.Bf[g], i);
+    }
+  const double fx = raw ? cs.JFx : cs.JFx / cs.J, fy = raw ? cs.JFy : cs.JFy / cs.J;
+  for (int i = 0; i < n1; ++i) {
+    t.EX[0][i] = fx * M[i];
+    t.EX[1][i] = -fx * M[i + (size_t)(n1 - 1) * n1];
+    t.EY[0][i] = fy * M[i];
+    t.EY[1][i] = -fy * M[i + (size_t)(n1 - 1) * n1];
+  }
+  return t;
+}
+
+namespace {
+
+template <int P, int FLUX, int NY, bool GC>
+void launch_cols(dgb_ctx* c, const ColArgs& a, const CUtensorMap& map) {
+  using Dm = ColDims<P, NY, GC>;
+  auto k = residual2d_cols_kernel<P, FLUX, NY, GC>;
+  allow_dynamic_smem(k, Dm::smem_bytes);
+  const dim3 grid((c->nx + Dm::TW - 1) / Dm::TW, (c->ny + Dm::TH - 1) / Dm::TH);
+  ProfScope ps(c, KC_RESIDUAL);
+  launch_pdl(c, k, grid, dim3(Dm::NT), Dm::smem_bytes, a, map);
+}
+
+template <int NY, bool GC>
+int dispatch_cols(dgb_ctx* c, const ColArgs& a, const CUtensorMap& map) {
+  switch (c->p * 10 + c->flux) {
+    case 10: launch_cols<1, 0, NY, GC>(c, a, map); return 0;
+    case 12: launch_cols<1, 2, NY, GC>(c, a, map); return 0;
+    case 20: launch_cols<2, 0, NY, GC>(c, a, map); return 0;
+    case 22: launch_cols<2, 2, NY, GC>(c, a, map); return 0;
+    case 30: launch_cols<3, 0, NY, GC>(c, a, map); return 0;
+    case 32: launch_cols<3, 2, NY, GC>(c, a, map); return 0;
+    default: return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (dim, p, flux)");
+  }
+}
+
+}  // namespace
+
+namespace {
+template <int P>
+void tile_of(const dgb_ctx* c, int& tw, int& th) {
+  if (c->gamcons) { tw = ColDims<P, 0, true>::TW; th = ColDims<P, 0, true>::TH; }
+  else if (c->nmass > 0) { tw = ColDims<P, 1, false>::TW; th = ColDims<P, 1, false>::TH; }
+  else { tw = ColDims<P, 0, false>::TW; th = ColDims<P, 0, false>::TH; }
+}
+}  // namespace
+
+// Tables and tensor maps of a structured 2D problem.  Rows must start on 16-byte boundaries for TMA (nx
+// even) and the grid must hold one tile's box; the other grids take plain loads.
+void cols_setup(dgb_ctx* c) {
+  c->col_step = make_col_tab(c->cs, false);
+  c->col_raw = make_col_tab(c->cs, true);
+  int tw = 0, th = 0;
+  if (c->p == 1) tile_of<1>(c, tw, th);
+  else if (c->p == 2) tile_of<2>(c, tw, th);
+  else tile_of<3>(c, tw, th);
+  c->cols_tma = c->nx % 2 == 0 && c->nx >= tw && c->ny >= th && encode_state_map(c, c->A, &c->colA, tw, th) &&
+                encode_state_map(c, c->B, &c->colB, tw, th) && encode_state_map(c, c->C, &c->colC, tw, th);
+}
+
+int residual2d_cols(dgb_ctx* c, const StageArgs& s, int mode) {
+  ColArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.U = s.U;
+  a.out = s.out;
+  a.nbr = s.nbr;
+  a.scal = s.scal;
+  a.errflag = &c->scal->flags;
+  a.polls = c->wait_polls;
+  a.nx = c->nx; a.ny = c->ny; a.ld = c->ld;
+  a.tma = c->cols_tma ? 1 : 0;
+  a.t = mode == MODE_RESIDUAL ? c->col_raw : c->col_step;
+  a.dt = mode == MODE_RESIDUAL ? 1.0 : s.dt_override;
+  if (mode == MODE_SSP) {
+    a.base = s.Ubase;
+    a.k0 = s.a;
+    a.k1 = a.k2 = s.b;
+  } else {
+    a.k2 = 1.0;
+    a.base2 = a.out2 = s.Uacc;
+    a.c2 = s.b;
+  }
+  const CUtensorMap& map = s.U == c->B ? c->colB : s.U == c->C ? c->colC : c->colA;
+  if (c->gamcons) return dispatch_cols<0, true>(c, a, map);
+  switch (c->nmass) {
+    case 0: return dispatch_cols<0, false>(c, a, map);
+    case 1: return dispatch_cols<1, false>(c, a, map);
+    case 2: return dispatch_cols<2, false>(c, a, map);
+    case 3: return dispatch_cols<3, false>(c, a, map);
+    default: return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (dim, p, flux)");
+  }
+}
+
+}  // namespace dgb
