@@ -65,11 +65,11 @@ struct dgb_ctx {
   long long wait_polls = 1ll << 22;  // poll budget of the residual kernels' first wait per tile copy
   bool rowmajor = false;  // structured row-major grid: tiled limiter passes
   bool chain1d = false;   // 1D elements in chain order: fused residual + limiter stages
-  bool fused_lim = false; // row-major grid, hrl / m2l: both limiter passes in one kernel (opt-in)
+  bool lim_out = false;   // row-major grid, hrl / m2l: both limiter passes in one launch, out of place
   CUtensorMap mapA, mapB, mapC;  // TMA descriptors of the state buffers (mixed, DMMA and many-Y tiles)
   // structured 2D grids: the residual with one thread per (element, quadrature column)
   bool cols = false, cols_tma = false;
-  CUtensorMap colA, colB, colC;    // its TMA descriptors
+  CUtensorMap colA, colB, colC, colD;  // its TMA descriptors
   dgb::ColTab col_step, col_raw;   // its tables: stage update, residual
   double hx = 0, hy = 0;
   size_t nstate = 0;

@@ -6,8 +6,7 @@
 // a persistent grid of CTAs walks that list with a fixed stride; all items of a launch cost the
 // same, so the static stride balances.  The arithmetic of an item is that of the single-problem
 // kernels (the same body functions): a 1D case advanced in a batch matches the same case advanced
-// alone bit for bit; in 2D the tile body reads the metric from shared memory instead of kernel
-// parameters and the compiler forms some fused multiply-adds differently (a few ulps).
+// alone bit for bit; in 2D the metric is a factor of its own instead of part of the tables (a few ulps).
 //
 // A case whose scalars carry a flag (an error, or FLAG_DONE once it has reached its end time) is
 // skipped by every item; the test is taken once per item by one thread and shared, so the CTA
@@ -15,7 +14,7 @@
 #pragma once
 #include "kernels.cuh"
 #include "limiter2d_tile.cuh"
-#include "tile2d.cuh"
+#include "tile2d_cols.cuh"
 
 namespace dgb {
 
@@ -29,7 +28,7 @@ struct BatchCase {
   const int* nbr;
   DevScalars* scal;
   int nx, ny, ld, ne;
-  double J, invJ, cx, cy, sx, sy, JFx, JFy;  // metric of the uniform element (2D tile kernel)
+  double sx, sy;  // 2/hx, 2/hy of the uniform element (2D)
   double cfl_scaled;
 };
 
@@ -55,7 +54,7 @@ __device__ __forceinline__ double stage_b(int s) { return s == 0 ? 1.0 : s == 1 
 // case flags of item `it`, read once by thread 0 and shared through `slot`
 __device__ __forceinline__ unsigned item_flags(const BatchCase* cases, int ci, unsigned* slot) {
   __syncthreads();  // the previous item's shared-memory users are done
-  if (threadIdx.x == 0 && threadIdx.y == 0) *slot = *(volatile unsigned*)&cases[ci].scal->flags;
+  if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) *slot = *(volatile unsigned*)&cases[ci].scal->flags;
   __syncthreads();
   return *slot;
 }
@@ -65,16 +64,19 @@ __device__ __forceinline__ unsigned item_flags(const BatchCase* cases, int ci, u
 // ---------------------------------------------------------------------------------------------
 template <int P, int TW, int TH>
 constexpr size_t batch_tile2d_smem_bytes() {
-  return (TileDims<P, TW, TH>::smem_bytes + 127) / 128 * 128 + (sizeof(TileArgs) + 127) / 128 * 128;
+  return (ColDims<P, 0, false, TW, TH>::smem_bytes + 127) / 128 * 128 + (sizeof(ColArgs) + 127) / 128 * 128;
 }
 
-template <int P, int FLUX, int TW, int TH, int UNROLL>
-__global__ void __launch_bounds__(TW * TH, 2)
+// tab: the tables of hx = hy = 2.  With a limiter the stage result goes to X and the limiter writes the
+// stage output.
+template <int P, int FLUX, int TW, int TH>
+__global__ void __launch_bounds__(ColDims<P, 0, false, TW, TH>::NT, ColDims<P, 0, false, TW, TH>::ctas)
     batch_tile2d_kernel(const BatchCase* __restrict__ cases, const BatchMaps* __restrict__ maps,
-                        const int4* __restrict__ items, int n_items, int stage) {
+                        const int4* __restrict__ items, int n_items, int stage, int limited,
+                        const __grid_constant__ ColTab tab) {
   extern __shared__ __align__(128) unsigned char smraw[];
-  using Dm = TileDims<P, TW, TH>;
-  TileArgs* sa = reinterpret_cast<TileArgs*>(smraw + (Dm::smem_bytes + 127) / 128 * 128);
+  using Dm = ColDims<P, 0, false, TW, TH>;
+  ColArgs* sa = reinterpret_cast<ColArgs*>(smraw + (Dm::smem_bytes + 127) / 128 * 128);
   unsigned* s_flags = reinterpret_cast<unsigned*>(smraw + 16);  // head: mbarrier, ok flag, this
   if (threadIdx.x == 0) {
     mbar_init(reinterpret_cast<uint64_t*>(smraw), 1);
@@ -87,57 +89,43 @@ __global__ void __launch_bounds__(TW * TH, 2)
     if (item_flags(cases, item.x, s_flags)) continue;
     if (threadIdx.x == 0) {
       const BatchCase& c = cases[item.x];
-      TileArgs a;
+      ColArgs a;
       a.U = stage_in(c, stage);
-      a.Ubase = c.A;
-      a.out = stage_out(c, stage);
-      a.Uacc = nullptr;
+      a.base = c.A;
+      a.out = limited ? c.X : stage_out(c, stage);
+      a.base2 = nullptr;
+      a.out2 = nullptr;
       a.nbr = c.nbr;
       a.scal = c.scal;
       a.errflag = &c.scal->flags;
-      a.a = stage_a(stage);
-      a.b = stage_b(stage);
-      a.dt_override = 0.0;
-      a.invJ = c.invJ; a.cx = c.cx; a.cy = c.cy; a.sx = c.sx; a.sy = c.sy;
-      a.J = c.J; a.JFx = c.JFx; a.JFy = c.JFy;
+      a.polls = kDefaultPolls;
+      a.k0 = stage_a(stage);
+      a.k1 = a.k2 = stage_b(stage);
+      a.c2 = 0.0;
+      a.dt = 0.0;
+      a.sx = c.sx; a.sy = c.sy;
       a.nx = c.nx; a.ny = c.ny; a.ld = c.ld;
+      a.tma = 1;
       *sa = a;
     }
     __syncthreads();
-    const CUtensorMap* mu = &maps[item.x].m[stage];
-    const CUtensorMap* mb = &maps[item.x].m[0];
-    tile2d_body<P, FLUX, MODE_SSP, TW, TH, UNROLL>(*sa, mu, mb, item.y, item.z, smraw, phase);
+    cols_body<P, FLUX, 0, false, TW, TH, true>(*sa, tab, &maps[item.x].m[stage], item.y, item.z, smraw, phase);
   }
 }
 
 // ---------------------------------------------------------------------------------------------
-// 2D limiter passes (hrl: METHOD 1, m2l: METHOD 2) on the stage output, via the case's scratch X
-// x items: (case, x0 multiple of 30, row);  y items: (case, x0 multiple of 32, y0 multiple of 4, node column)
+// 2D limiter (hrl: METHOD 1, m2l: METHOD 2), X -> stage output (items: case, tile column, tile row)
 // ---------------------------------------------------------------------------------------------
 template <int P, int METHOD>
-__global__ void __launch_bounds__(32 * (P + 1)) batch_lim2d_x_kernel(const BatchCase* __restrict__ cases,
-                                                                   const int4* __restrict__ items, int n_items,
-                                                                   int stage) {
+__global__ void __launch_bounds__(LimDims<P, METHOD, 0>::NT, LimDims<P, METHOD, 0>::ctas)
+    batch_lim2d_kernel(const BatchCase* __restrict__ cases, const int4* __restrict__ items, int n_items, int stage) {
+  extern __shared__ __align__(16) double lsm[];
   __shared__ unsigned s_flags;
   for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
     const int4 item = __ldg(items + it);
     if (item_flags(cases, item.x, &s_flags)) continue;
     const BatchCase& c = cases[item.x];
-    const LimArgs la{c.ld, c.ne};
-    lim2d_xpass_body<P, METHOD>(la, c.nx, stage_out(c, stage), c.nbr, c.X, item.y, item.z);
-  }
-}
-
-template <int P, int METHOD>
-__global__ void __launch_bounds__(32 * 6) batch_lim2d_y_kernel(const BatchCase* __restrict__ cases,
-                                                             const int4* __restrict__ items, int n_items, int stage) {
-  __shared__ unsigned s_flags;
-  for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const int4 item = __ldg(items + it);
-    if (item_flags(cases, item.x, &s_flags)) continue;
-    const BatchCase& c = cases[item.x];
-    const LimArgs la{c.ld, c.ne};
-    lim2d_ypass_body<P, METHOD>(la, c.nx, c.ny, c.X, c.nbr, stage_out(c, stage), item.y, item.z, item.w);
+    lim2d_body<P, METHOD, 0>(LimArgs{c.ld, c.ne}, c.nx, c.ny, c.X, c.nbr, stage_out(c, stage), item.y, item.z, lsm);
   }
 }
 

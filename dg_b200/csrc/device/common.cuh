@@ -27,11 +27,6 @@ struct Consts {
   double Bf[MAXN][MAXN], wf[MAXN];
   // element inverse mass matrix in tensor order (Minv[t][t'])
   double Minv[MAXNS][MAXNS];
-  // 1D Lagrange -> scaled Taylor monomial transform in tensor (ascending) node order and inverse
-  double T[MAXN][MAXN], Tinv[MAXN][MAXN];
-  // limiter integrals (limiting_kernels.cu:1748-1775): imd[k][n] = int_{-1}^{1} d^k/dx^k x^n/n!,
-  // imdL[k][n] over [-3,-1], imdR[k][n] over [1,3]; ifact[k] = 1/k!
-  double imd[MAXN][MAXN], imdL[MAXN][MAXN], imdR[MAXN][MAXN], ifact[8];
   // metric of the uniform Cartesian element: J = hx*hy/4 (1D: hx/2), invJac = diag(2/hx, 2/hy)
   double J, ixx, iyy;
   // face Jacobians: x-faces (constant x) and y-faces
@@ -59,77 +54,114 @@ enum { FLAG_NONFINITE = 1u, FLAG_DT_SMALL = 2u, FLAG_TIMEOUT = 4u };
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-__device__ __forceinline__ int signum_d(double v) { return v > 0 ? 1 : (v < 0 ? -1 : 0); }
-
-// minmod of two arguments (limiting_kernels.cu:1470-1486)
+// minmod of two arguments (limiting_kernels.cu:1470-1486): the smaller in magnitude when their signs
+// agree, else 0.  Signs are compared as bits (a zero argument gives 0 either way).
 __device__ __forceinline__ double minmod2(double a, double b) {
-  const int sa = signum_d(a);
-  if (sa != signum_d(b)) return 0.0;
-  const double fa = fabs(a), fb = fabs(b);
-  return fa < fb ? sa * fa : sa * fb;
+  const double m = fabs(a) < fabs(b) ? a : b;
+  return (__double2hiint(a) ^ __double2hiint(b)) < 0 ? 0.0 : m;
 }
 
-// 1D tables of the limiter for order P (reference element, identical for every problem):
-//   T, Tinv   Lagrange (ascending nodes) <-> scaled Taylor monomial x^n/n! transforms
-//   imd[k][n] = int_{-1}^{1} d^k/dx^k x^n/n! dx, imdL over [-3,-1], imdR over [1,3]
-//             (integrate_monomial_derivative(_bounds), limiting_kernels.cu:1748-1775)
-//   ifact[k]  = 1/k!
+// ---- hierarchical reconstruction of one 1D slice -------------------------------------------------
+// Nodes are equispaced on [-1, 1]; a[n] are scaled Taylor coefficients, u(x) = sum a_n x^n / n!.  The
+// limiter (limit_monomial, limiting_kernels.cu:1534-1583) compares, for k = P-1 .. 0, the cell means of
+// the k-th derivative in the cell and its two neighbours, after taking from each the mean of the
+// already limited higher terms.  So a cell enters only through the means of its derivatives 0 .. P-1 --
+// P numbers, simple sums of its nodal values -- and the integrals over the neighbours' intervals
+// are the constants 13/6 and 5/3.  Written out per order this is a quarter of the multiplications of the
+// general form with its transform and integral tables.
+// D: the P means times fixed factors (P = 1: 2 u; P = 2: 6 u, 2 u'; P = 3: 8 u, 2 u', 8/9 u'').
 template <int P>
-struct LimTab {
-  double T[P + 1][P + 1], Tinv[P + 1][P + 1];
-  double imd[P + 1][P + 1], imdL[P + 1][P + 1], imdR[P + 1][P + 1];
-  double ifact[P + 3];
-};
-// one copy per translation unit (each .cu file is its own device module)
-static __constant__ LimTab<1> c_lim_p1;
-static __constant__ LimTab<2> c_lim_p2;
-static __constant__ LimTab<3> c_lim_p3;
-// by-name access (a reference to a __constant__ object can be materialised as a local copy)
-#define DGB_LIM(P, member) ((P) == 1 ? c_lim_p1.member : (P) == 2 ? c_lim_p2.member : c_lim_p3.member)
-
-// Hierarchical-reconstruction limiting of one 1D slice of scaled Taylor coefficients
-// (limit_monomial, limiting_kernels.cu:1534-1583).  N = polynomial order.
-template <int N>
-__device__ __forceinline__ void limit_monomial(const double* AL, const double* AC, const double* AR, double* Alim) {
-  double avgLC = 0.0;
-#pragma unroll
-  for (int m = N; m > 0; --m) {
-    double dUL = 0, dUC = 0, dUR = 0, RL = 0, RC = 0, RR = 0;
-#pragma unroll
-    for (int n = m - 1; n <= N; ++n) {
-      const double integral = DGB_LIM(N, imd[m - 1][n]);
-      dUL += AL[n] * integral;
-      dUC += AC[n] * integral;
-      dUR += AR[n] * integral;
-      if (n >= m + 1) {
-        const double al = Alim[n];
-        RL += al * DGB_LIM(N, imdL[m - 1][n]);
-        RC += al * integral;
-        RR += al * DGB_LIM(N, imdR[m - 1][n]);
-      }
-    }
-    const double avgLL = 0.5 * (dUL - RL);
-    avgLC = 0.5 * (dUC - RC);
-    const double avgLR = 0.5 * (dUR - RR);
-    const double c1 = 0.5 * (avgLC - avgLL);
-    const double c2 = 0.5 * (avgLR - avgLC);
-    Alim[m] = minmod2(c1, c2);
+__device__ __forceinline__ void hr_moments(const double* v, double* D) {
+  if constexpr (P == 1) {
+    D[0] = v[0] + v[1];
+  } else if constexpr (P == 2) {
+    D[0] = (v[0] + v[2]) + 4.0 * v[1];
+    D[1] = v[2] - v[0];
+  } else {
+    const double s0 = v[0] + v[3], s1 = v[1] + v[2];
+    D[0] = s0 + 3.0 * s1;
+    D[1] = v[3] - v[0];
+    D[2] = s0 - s1;
   }
-  Alim[0] = avgLC;
 }
-
-// average_monomial (limiting_kernels.cu:1777-1790): keep the cell average, zero the slopes
-template <int N>
-__device__ __forceinline__ void average_monomial(const double* A, double* Alim) {
-  double avg = 0;
+// the cell mean
+template <int P>
+__device__ __forceinline__ double hr_mean(const double* D) {
+  return P == 1 ? 0.5 * D[0] : P == 2 ? D[0] * (1.0 / 6.0) : 0.125 * D[0];
+}
+// the limited Taylor coefficients of the cell with moments DC between neighbours DL and DR
+template <int P>
+__device__ __forceinline__ void hr_limit(const double* DL, const double* DC, const double* DR, double* lim) {
+  if constexpr (P == 1) {
+    lim[1] = 0.25 * minmod2(DC[0] - DL[0], DR[0] - DC[0]);
+    lim[0] = 0.5 * DC[0];
+  } else if constexpr (P == 2) {
+    lim[2] = 0.25 * minmod2(DC[1] - DL[1], DR[1] - DC[1]);
+    lim[1] = minmod2((DC[0] - DL[0]) * (1.0 / 12.0) + lim[2], (DR[0] - DC[0]) * (1.0 / 12.0) - lim[2]);
+    lim[0] = (DC[0] - lim[2]) * (1.0 / 6.0);
+  } else {
+    lim[3] = 0.5625 * minmod2(DC[2] - DL[2], DR[2] - DC[2]);
+    lim[2] = minmod2(0.25 * (DC[1] - DL[1]) + lim[3], 0.25 * (DR[1] - DC[1]) - lim[3]);
+    const double t = lim[3] * (-5.0 / 6.0);
+    lim[1] = minmod2(0.0625 * (DC[0] - DL[0]) + (t + lim[2]), 0.0625 * (DR[0] - DC[0]) + (t - lim[2]));
+    lim[0] = 0.125 * DC[0] - lim[2] * (1.0 / 6.0);
+  }
+}
+// the cell mean kept, the rest zero (average_monomial, limiting_kernels.cu:1777-1790)
+template <int P>
+__device__ __forceinline__ void hr_flat(const double* DC, double* lim) {
+  lim[0] = hr_mean<P>(DC);
 #pragma unroll
-  for (int n = 0; n <= N; ++n) { avg += A[n] * DGB_LIM(N, imd[0][n]); Alim[n] = 0; }
-  Alim[0] = 0.5 * avg;
+  for (int m = 1; m <= P; ++m) lim[m] = 0.0;
 }
-
+// nodal values -> scaled Taylor coefficients, and back
 template <int P>
-__device__ __forceinline__ double lim_T(int m, int i) { return DGB_LIM(P, T[m][i]); }
+__device__ __forceinline__ void to_mono(const double* v, double* a) {
+  if constexpr (P == 1) {
+    a[0] = 0.5 * (v[0] + v[1]);
+    a[1] = 0.5 * (v[1] - v[0]);
+  } else if constexpr (P == 2) {
+    a[0] = v[1];
+    a[1] = 0.5 * (v[2] - v[0]);
+    a[2] = (v[0] + v[2]) - 2.0 * v[1];
+  } else {
+    const double s0 = v[0] + v[3], s1 = v[1] + v[2], d0 = v[3] - v[0], d1 = v[2] - v[1];
+    a[0] = 0.0625 * (9.0 * s1 - s0);
+    a[1] = 0.0625 * (27.0 * d1 - d0);
+    a[2] = 1.125 * (s0 - s1);
+    a[3] = 3.375 * (d0 - 3.0 * d1);
+  }
+}
 template <int P>
-__device__ __forceinline__ double lim_Tinv(int i, int m) { return DGB_LIM(P, Tinv[i][m]); }
+__device__ __forceinline__ void to_lag(const double* a, double* v) {
+  if constexpr (P == 1) {
+    v[0] = a[0] - a[1];
+    v[1] = a[0] + a[1];
+  } else if constexpr (P == 2) {
+    const double e = a[0] + 0.5 * a[2];
+    v[0] = e - a[1];
+    v[1] = a[0];
+    v[2] = e + a[1];
+  } else {
+    const double e1 = a[0] + 0.5 * a[2], o1 = a[1] + a[3] * (1.0 / 6.0);
+    const double e3 = a[0] + a[2] * (1.0 / 18.0), o3 = a[1] * (1.0 / 3.0) + a[3] * (1.0 / 162.0);
+    v[0] = e1 - o1;
+    v[1] = e3 - o3;
+    v[2] = e3 + o3;
+    v[3] = e1 + o1;
+  }
+}
+// E of a slice from its limited pressure and alpha and its kinetic energy: coefficients m >= 1 are those
+// of rho e + K, rho e the Leibniz product of p and alpha (internal_energy_multifluid,
+// limiting_kernels.cu:160-199), and the cell mean of E is kept (reconstruct_energy, :111-156)
+template <int P>
+__device__ __forceinline__ void hr_energy(const double* plim, const double* alim, const double* Kmono, double mean,
+                                          double* E) {
+  E[1] = (plim[1] * alim[0] + plim[0] * alim[1]) + Kmono[1];
+  if constexpr (P >= 2) E[2] = (plim[2] * alim[0] + (2.0 * plim[1] * alim[1] + plim[0] * alim[2])) + Kmono[2];
+  if constexpr (P >= 3)
+    E[3] = (plim[3] * alim[0] + (3.0 * (plim[2] * alim[1] + plim[1] * alim[2]) + plim[0] * alim[3])) + Kmono[3];
+  E[0] = P >= 2 ? mean - E[P >= 2 ? 2 : 0] * (1.0 / 6.0) : mean;
+}
 
 }  // namespace dgb

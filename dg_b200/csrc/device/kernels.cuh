@@ -167,9 +167,9 @@ __global__ void __launch_bounds__(NT) residual2d_kernel(const Consts cin, const 
       // the volume terms of the tiled kernel's point_terms: the conservative fluxes of the NFL
       // fields (mass fractions rho Y_k u, physics.cu:293-298; GAMCONS alpha flux rho u/(gamma-1),
       // physics.cu:253-281) and, under GAMNCON, the alpha source
-      const double rho = ug[0], irho = __drcp_rn(rho);
+      const double rho = ug[0], irho = phys::rcp(rho);
       const double uu = ug[1] * irho, vv = ug[2] * irho, Et = ug[3];
-      const double gm1 = GC ? rho * __drcp_rn(ug[4]) : __drcp_rn(ug[4]);
+      const double gm1 = GC ? rho * phys::rcp(ug[4]) : phys::rcp(ug[4]);
       const double p = gm1 * (Et - 0.5 * rho * (uu * uu + vv * vv));
       const double W = c.wq[g / NG1] * c.wq[g % NG1];
       const double wx = W * (c.J * c.ixx), wy = W * (c.J * c.iyy);
@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(NT) residual2d_kernel(const Consts cin, const 
       continue;
     }
     // physics.cu:248-257 with correctly rounded reciprocals in place of its divisions
-    const double rho = ug[0], ir = __drcp_rn(rho), u = ug[1] * ir, v = ug[2] * ir, Et = ug[3];
-    const double p = __drcp_rn(ug[4]) * (Et - 0.5 * rho * (u * u + v * v));
+    const double rho = ug[0], ir = phys::rcp(rho), u = ug[1] * ir, v = ug[2] * ir, Et = ug[3];
+    const double p = phys::rcp(ug[4]) * (Et - 0.5 * rho * (u * u + v * v));
     const double W = c.wq[g / NG1] * c.wq[g % NG1];
     const double cx = W * (c.ixx * c.J), cy = W * (c.iyy * c.J);
     G[(0 * NG + g) * TE + el] = cx * (rho * u);
@@ -431,72 +431,39 @@ __global__ void __launch_bounds__(128) residual1d_kernel(const Consts cin, const
 }
 
 // ------------------------------------------------------------------------------------------
-// Limiters.  Fields are limited slice by slice in the scaled Taylor basis (T, Tinv).
+// Limiters.  Fields are limited slice by slice (hr_limit, common.cuh).
 // ------------------------------------------------------------------------------------------
-template <int P>
-__device__ __forceinline__ void to_mono(const double* v, double* a) {
-#pragma unroll
-  for (int m = 0; m <= P; ++m) {
-    double s = 0;
-#pragma unroll
-    for (int i = 0; i <= P; ++i) s += lim_T<P>(m, i) * v[i];
-    a[m] = s;
-  }
-}
-template <int P>
-__device__ __forceinline__ void to_lag(const double* a, double* v) {
-#pragma unroll
-  for (int i = 0; i <= P; ++i) {
-    double s = 0;
-#pragma unroll
-    for (int m = 0; m <= P; ++m) s += lim_Tinv<P>(i, m) * a[m];
-    v[i] = s;
-  }
-}
-
 // Limit one slice given the nodal values of the centre and (when interior) both neighbours.
 // phys: 0 interior, 2/3 flatten (zero-gradient / reflective), 4 leave unchanged, 5 copy
 // (reflective wall-normal momentum under HR limiting, hrl1D limiting_kernels.cu:291-302).
 template <int P>
 __device__ __forceinline__ void limit_slice(int phys, const double* vL, const double* vC, const double* vR,
                                             double* lim) {
-  constexpr int N1 = P + 1;
-  double aC[N1];
-  to_mono<P>(vC, aC);
+  double DC[P];
   if (phys == 0) {
-    double aL[N1], aR[N1];
-    to_mono<P>(vL, aL);
-    to_mono<P>(vR, aR);
-    limit_monomial<P>(aL, aC, aR, lim);
+    double DL[P], DR[P];
+    hr_moments<P>(vC, DC);
+    hr_moments<P>(vL, DL);
+    hr_moments<P>(vR, DR);
+    hr_limit<P>(DL, DC, DR, lim);
   } else if (phys == 2 || phys == 3) {
-    average_monomial<P>(aC, lim);
+    hr_moments<P>(vC, DC);
+    hr_flat<P>(DC, lim);
   } else {
-#pragma unroll
-    for (int m = 0; m < N1; ++m) lim[m] = aC[m];
+    to_mono<P>(vC, lim);
   }
 }
 
-// rho e = Leibniz product of the monomial p and alpha (internal_energy_multifluid,
-// limiting_kernels.cu:160-199), then E (reconstruct_energy, limiting_kernels.cu:111-156)
+// E rebuilt from the limited coefficients of p and alpha, the limited kinetic energy K and the slice
+// vE of E before (nodal values, and out)
 template <int P>
-__device__ __forceinline__ void reconstruct_energy(const double* plim, const double* alim, const double* Kmono,
-                                                   const double* Emono, double* Elim) {
-  constexpr int N1 = P + 1;
-  constexpr double binom[4][4] = {{1, 0, 0, 0}, {1, 1, 0, 0}, {1, 2, 1, 0}, {1, 3, 3, 1}};
-  double rhoe[N1];
-#pragma unroll
-  for (int m = 0; m < N1; ++m) {
-    double I = 0;
-#pragma unroll
-    for (int k = 0; k <= m; ++k) I += binom[m][k] * plim[m - k] * alim[k];
-    rhoe[m] = I;
-  }
-#pragma unroll
-  for (int m = 1; m < N1; ++m) Elim[m] = rhoe[m] + Kmono[m];
-  double E0 = Emono[0];
-#pragma unroll
-  for (int k = 2; k < N1; k += 2) E0 -= DGB_LIM(P, ifact[k + 1]) * (Elim[k] - Emono[k]);
-  Elim[0] = E0;
+__device__ __forceinline__ void rebuild_energy(const double* plim, const double* alim, const double* K, const double* vE,
+                                               double* E) {
+  double Km[P + 1], D[P], El[P + 1];
+  to_mono<P>(K, Km);
+  hr_moments<P>(vE, D);
+  hr_energy<P>(plim, alim, Km, hr_mean<P>(D), El);
+  to_lag<P>(El, E);
 }
 
 __device__ __forceinline__ int boundary_code(int left, int right) {
@@ -552,8 +519,8 @@ __global__ void __launch_bounds__(128) lim2d_xpass_kernel(const LimArgs la, cons
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) {
         const double ru = v[s][1][ix], rv = v[s][2][ix], E = v[s][3][ix];
-        const double gm1 = __drcp_rn(v[s][4][ix]);
-        pr[s][ix] = gm1 * (E - 0.5 * (ru * ru + rv * rv) * __drcp_rn(v[s][0][ix]));
+        const double gm1 = phys::rcp(v[s][4][ix]);
+        pr[s][ix] = gm1 * (E - 0.5 * (ru * ru + rv * rv) * phys::rcp(v[s][0][ix]));
       }
     }
     double lr[N1], lu[N1], lv[N1], la_[N1], lp[N1];
@@ -562,18 +529,15 @@ __global__ void __launch_bounds__(128) lim2d_xpass_kernel(const LimArgs la, cons
     limit_slice<P>(phys, v[0][2], v[1][2], v[2][2], lv);
     limit_slice<P>(phys, v[0][4], v[1][4], v[2][4], la_);
     limit_slice<P>(phys, pr[0], pr[1], pr[2], lp);
-    double r_[N1], u_[N1], v_[N1], a_[N1], p_[N1], K[N1], Km[N1], Em[N1], El[N1], E_[N1];
+    double r_[N1], u_[N1], v_[N1], a_[N1], p_[N1], K[N1], E_[N1];
     to_lag<P>(lr, r_);
     to_lag<P>(lu, u_);
     to_lag<P>(lv, v_);
     to_lag<P>(la_, a_);
     to_lag<P>(lp, p_);
 #pragma unroll
-    for (int ix = 0; ix < N1; ++ix) K[ix] = 0.5 * (u_[ix] * u_[ix] + v_[ix] * v_[ix]) * __drcp_rn(r_[ix]);
-    to_mono<P>(K, Km);
-    to_mono<P>(v[1][3], Em);
-    reconstruct_energy<P>(lp, la_, Km, Em, El);
-    to_lag<P>(El, E_);
+    for (int ix = 0; ix < N1; ++ix) K[ix] = 0.5 * (u_[ix] * u_[ix] + v_[ix] * v_[ix]) * phys::rcp(r_[ix]);
+    rebuild_energy<P>(lp, la_, K, v[1][3], E_);
 #pragma unroll
     for (int ix = 0; ix < N1; ++ix) {
       const size_t o = (size_t)(ix + N1 * iy) * ld + e;
@@ -627,17 +591,14 @@ __global__ void __launch_bounds__(128) lim2d_ypass_kernel(const LimArgs la, cons
     limit_slice<P>(phys, v[0][2], v[1][2], v[2][2], lv);
     limit_slice<P>(phys, v[0][3], v[1][3], v[2][3], la_);
     limit_slice<P>(phys, v[0][4], v[1][4], v[2][4], lp);
-    double r_[N1], u_[N1], v_[N1], a_[N1], K[N1], Km[N1], Em[N1], El[N1], E_[N1];
+    double r_[N1], u_[N1], v_[N1], a_[N1], K[N1], E_[N1];
     to_lag<P>(lr, r_);
     to_lag<P>(lu, u_);
     to_lag<P>(lv, v_);
     to_lag<P>(la_, a_);
 #pragma unroll
-    for (int iy = 0; iy < N1; ++iy) K[iy] = 0.5 * (u_[iy] * u_[iy] + v_[iy] * v_[iy]) * __drcp_rn(r_[iy]);
-    to_mono<P>(K, Km);
-    to_mono<P>(v[1][5], Em);
-    reconstruct_energy<P>(lp, la_, Km, Em, El);
-    to_lag<P>(El, E_);
+    for (int iy = 0; iy < N1; ++iy) K[iy] = 0.5 * (u_[iy] * u_[iy] + v_[iy] * v_[iy]) * phys::rcp(r_[iy]);
+    rebuild_energy<P>(lp, la_, K, v[1][5], E_);
 #pragma unroll
     for (int iy = 0; iy < N1; ++iy) {
       const size_t o = (size_t)(ix + N1 * iy) * ld + e;
@@ -672,8 +633,8 @@ __device__ __forceinline__ void lim1d_limit(int phys, const double (&v)[3][4 + N
 #pragma unroll
       for (int i = 0; i < N1; ++i) {
         const double ru = v[s][1][i], E = v[s][2][i];
-        const double gm1 = __drcp_rn(v[s][3][i]);
-        pr[s][i] = gm1 * (E - 0.5 * ru * ru * __drcp_rn(v[s][0][i]));
+        const double gm1 = phys::rcp(v[s][3][i]);
+        pr[s][i] = gm1 * (E - 0.5 * ru * ru * phys::rcp(v[s][0][i]));
       }
     }
     double lr[N1], lu[N1], la_[N1], lp[N1];
@@ -681,16 +642,13 @@ __device__ __forceinline__ void lim1d_limit(int phys, const double (&v)[3][4 + N
     limit_slice<P>(phys, v[0][1], v[1][1], v[2][1], lu);
     limit_slice<P>(phys, v[0][3], v[1][3], v[2][3], la_);
     limit_slice<P>(phys, pr[0], pr[1], pr[2], lp);
-    double K[N1], Km[N1], Em[N1], El[N1];
+    double K[N1];
     to_lag<P>(lr, o[0]);
     to_lag<P>(lu, o[1]);
     to_lag<P>(la_, o[3]);
 #pragma unroll
-    for (int i = 0; i < N1; ++i) K[i] = 0.5 * o[1][i] * o[1][i] * __drcp_rn(o[0][i]);  // kinetic_energy1D
-    to_mono<P>(K, Km);
-    to_mono<P>(v[1][2], Em);
-    reconstruct_energy<P>(lp, la_, Km, Em, El);
-    to_lag<P>(El, o[2]);
+    for (int i = 0; i < N1; ++i) K[i] = 0.5 * o[1][i] * o[1][i] * phys::rcp(o[0][i]);  // kinetic_energy1D
+    rebuild_energy<P>(lp, la_, K, v[1][2], o[2]);
 #pragma unroll
     for (int k = 4; k < NF; ++k) {
       double ly[N1];

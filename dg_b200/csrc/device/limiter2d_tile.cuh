@@ -1,9 +1,11 @@
-// Tiled 2D limiter passes for structured row-major grids (HR and m2 methods).
+// 2D limiters of structured row-major grids (HR and m2 methods).
 //
-// Same arithmetic as lim2d_xpass_kernel / lim2d_ypass_kernel, but every element's monomial
-// coefficients (and, for m2, its nodal pressure) are computed once per slice and shared through
-// shared memory with the neighbours that need them, instead of being recomputed by the three
-// threads that read them.
+//   lim2d_kernel       both passes in one launch, out of place: one thread per element
+//   lim2d_*pass_*      x pass, then y pass through a global scratch: the batched ensemble, the
+//                      allocation-free limiter, primitive variables, sides with frozen data
+//
+// Either way every element's moments (hr_moments) are computed once per slice and shared with the
+// neighbours that need them.
 //   x pass: CTA = 30 consecutive elements of one element row (+ left/right neighbour slots),
 //           threads (element slot, y-slice)
 //   y pass: CTA = 32 x 4 elements (+ bottom/top neighbour rows), threads (x slot, row slot),
@@ -19,12 +21,12 @@ namespace dgb {
 // static limit (up to three mass fractions), else the arrays' size
 template <int P, int NY>
 constexpr size_t lim2d_xpass_smem_bytes() {
-  const size_t b = sizeof(double) * (5 + NY) * (P + 1) * (P + 1) * 32;
+  const size_t b = sizeof(double) * (5 + NY) * (P + 1) * P * 32;
   return b <= 48 * 1024 ? 0 : b;
 }
 template <int P, int NY>
 constexpr size_t lim2d_ypass_smem_bytes() {
-  const size_t b = sizeof(double) * (5 + NY) * (P + 1) * 6 * 32;
+  const size_t b = sizeof(double) * (5 + NY) * P * 6 * 32;
   return b <= 48 * 1024 ? 0 : b;
 }
 
@@ -37,15 +39,15 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
                                                  const int* __restrict__ nbr, double* __restrict__ X, int x0,
                                                  int ey) {
   constexpr int N1 = P + 1, NS = N1 * N1, NQ = 5 + NY, NF = 5 + NY, TWI = 30;
-  // [quantity][slice][coefficient][slot]: static shared memory, or dynamic (lim2d_xpass_smem_bytes)
+  // [quantity][slice][moment][slot]: static shared memory, or dynamic (lim2d_xpass_smem_bytes)
   // when the quantities would not fit the static limit (many mass fractions)
-  double(*A)[N1][N1][32];
+  double(*A)[N1][P][32];
   if constexpr (lim2d_xpass_smem_bytes<P, NY>() == 0) {
-    __shared__ double As[NQ][N1][N1][32];
+    __shared__ double As[NQ][N1][P][32];
     A = As;
   } else {
     extern __shared__ __align__(16) double lsm[];
-    A = reinterpret_cast<double(*)[N1][N1][32]>(lsm);
+    A = reinterpret_cast<double(*)[N1][P][32]>(lsm);
   }
   const int ld = la.ld;
   const int tx = threadIdx.x, sl = threadIdx.y;
@@ -56,14 +58,12 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
   if (interior) e = ey * nx + ex;
   else if (tx == 0) e = __ldg(nbr + (size_t)0 * ld + ey * nx + x0);
   else if (ex - 1 < nx && ex - 1 >= 0) e = __ldg(nbr + (size_t)1 * ld + ey * nx + ex - 1);
-  double v[NF][N1];
-  double Em[N1];
+  double v[NF][N1], q[NQ][N1];
   if (e >= 0) {
 #pragma unroll
     for (int f = 0; f < NF; ++f)
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) v[f][ix] = __ldg(U + (size_t)(f * NS + ix + N1 * sl) * ld + e);
-    double q[NQ][N1];
 #pragma unroll
     for (int ix = 0; ix < N1; ++ix) {
 #pragma unroll
@@ -79,17 +79,16 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
         // pressure from the unlimited state (pressure kernel, physics.cu:891-958), with correctly
         // rounded reciprocals in place of its divisions
         const double ru = v[1][ix], rv = v[2][ix];
-        q[4][ix] = __drcp_rn(v[4][ix]) * (v[3][ix] - 0.5 * (ru * ru + rv * rv) * __drcp_rn(v[0][ix]));
+        q[4][ix] = phys::rcp(v[4][ix]) * (v[3][ix] - 0.5 * (ru * ru + rv * rv) * phys::rcp(v[0][ix]));
       }
     }
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
-      double a[N1];
-      to_mono<P>(q[k], a);
+      double D[P];
+      hr_moments<P>(q[k], D);
 #pragma unroll
-      for (int m = 0; m < N1; ++m) A[k][sl][m][tx] = a[m];
+      for (int m = 0; m < P; ++m) A[k][sl][m][tx] = D[m];
     }
-    if constexpr (METHOD == 2) to_mono<P>(v[3], Em);
   }
   __syncthreads();
   if (!interior) return;
@@ -97,19 +96,18 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
   double lim[NQ][N1];
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
-    double aL[N1], aC[N1], aR[N1];
+    double DL[P], DC[P], DR[P];
 #pragma unroll
-    for (int m = 0; m < N1; ++m) aC[m] = A[k][sl][m][tx];
+    for (int m = 0; m < P; ++m) DC[m] = A[k][sl][m][tx];
     const int ph = (METHOD == 1 && phys == 3 && k == 1) ? 5 : phys;
     if (ph == 0) {
 #pragma unroll
-      for (int m = 0; m < N1; ++m) { aL[m] = A[k][sl][m][tx - 1]; aR[m] = A[k][sl][m][tx + 1]; }
-      limit_monomial<P>(aL, aC, aR, lim[k]);
+      for (int m = 0; m < P; ++m) { DL[m] = A[k][sl][m][tx - 1]; DR[m] = A[k][sl][m][tx + 1]; }
+      hr_limit<P>(DL, DC, DR, lim[k]);
     } else if (ph == 2 || ph == 3) {
-      average_monomial<P>(aC, lim[k]);
+      hr_flat<P>(DC, lim[k]);
     } else {
-#pragma unroll
-      for (int m = 0; m < N1; ++m) lim[k][m] = aC[m];
+      to_mono<P>(q[k], lim[k]);
     }
   }
   if constexpr (METHOD == 1) {
@@ -121,17 +119,15 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
       for (int ix = 0; ix < N1; ++ix) X[(size_t)(k * NS + ix + N1 * sl) * ld + e] = out[ix];
     }
   } else {
-    double r_[N1], u_[N1], v_[N1], a_[N1], p_[N1], K[N1], Km[N1], El[N1], E_[N1];
+    double r_[N1], u_[N1], v_[N1], a_[N1], p_[N1], K[N1], E_[N1];
     to_lag<P>(lim[0], r_);
     to_lag<P>(lim[1], u_);
     to_lag<P>(lim[2], v_);
     to_lag<P>(lim[3], a_);
     to_lag<P>(lim[4], p_);
 #pragma unroll
-    for (int ix = 0; ix < N1; ++ix) K[ix] = 0.5 * (u_[ix] * u_[ix] + v_[ix] * v_[ix]) * __drcp_rn(r_[ix]);
-    to_mono<P>(K, Km);
-    reconstruct_energy<P>(lim[4], lim[3], Km, Em, El);
-    to_lag<P>(El, E_);
+    for (int ix = 0; ix < N1; ++ix) K[ix] = 0.5 * (u_[ix] * u_[ix] + v_[ix] * v_[ix]) * phys::rcp(r_[ix]);
+    rebuild_energy<P>(lim[4], lim[3], K, v[3], E_);
 #pragma unroll
     for (int ix = 0; ix < N1; ++ix) {
       const size_t o = (size_t)(ix + N1 * sl) * ld + e;
@@ -173,14 +169,14 @@ __device__ __forceinline__ void lim2d_ypass_body(const LimArgs la, int nx, int n
   constexpr int N1 = P + 1, NS = N1 * N1, NQ = 5 + NY, THI = 4;
   // row of quantity k in X: HR -> field k; m2 -> [rho, rhou, rhov, alpha, p, E, rho Y_k]
   auto xrow = [](int k) { return (METHOD == 2 && k >= 5) ? k + 1 : k; };
-  // [quantity][coefficient][row slot][x slot]: static or (many mass fractions) dynamic
-  double(*B)[N1][THI + 2][32];
+  // [quantity][moment][row slot][x slot]: static or (many mass fractions) dynamic
+  double(*B)[P][THI + 2][32];
   if constexpr (lim2d_ypass_smem_bytes<P, NY>() == 0) {
-    __shared__ double Bs[NQ][N1][THI + 2][32];
+    __shared__ double Bs[NQ][P][THI + 2][32];
     B = Bs;
   } else {
     extern __shared__ __align__(16) double lsm[];
-    B = reinterpret_cast<double(*)[N1][THI + 2][32]>(lsm);
+    B = reinterpret_cast<double(*)[P][THI + 2][32]>(lsm);
   }
   const int ld = la.ld;
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -193,22 +189,20 @@ __device__ __forceinline__ void lim2d_ypass_body(const LimArgs la, int nx, int n
     else if (ty == 0) e = __ldg(nbr + (size_t)2 * ld + y0 * nx + x);
     else if (yy - 1 < ny && yy - 1 >= 0) e = __ldg(nbr + (size_t)3 * ld + (yy - 1) * nx + x);
   }
-  double Em[N1];
+  double vE[N1], col[NQ][N1];
   if (e >= 0) {
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
-      double col[N1], a[N1];
+      double D[P];
 #pragma unroll
-      for (int iy = 0; iy < N1; ++iy) col[iy] = __ldg(X + (size_t)(xrow(k) * NS + ix + N1 * iy) * ld + e);
-      to_mono<P>(col, a);
+      for (int iy = 0; iy < N1; ++iy) col[k][iy] = __ldg(X + (size_t)(xrow(k) * NS + ix + N1 * iy) * ld + e);
+      hr_moments<P>(col[k], D);
 #pragma unroll
-      for (int m = 0; m < N1; ++m) B[k][m][ty][tx] = a[m];
+      for (int m = 0; m < P; ++m) B[k][m][ty][tx] = D[m];
     }
     if constexpr (METHOD == 2) {
-      double col[N1];
 #pragma unroll
-      for (int iy = 0; iy < N1; ++iy) col[iy] = __ldg(X + (size_t)(5 * NS + ix + N1 * iy) * ld + e);
-      to_mono<P>(col, Em);
+      for (int iy = 0; iy < N1; ++iy) vE[iy] = __ldg(X + (size_t)(5 * NS + ix + N1 * iy) * ld + e);
     }
   }
   __syncthreads();
@@ -217,19 +211,18 @@ __device__ __forceinline__ void lim2d_ypass_body(const LimArgs la, int nx, int n
   double lim[NQ][N1];
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
-    double aD[N1], aC[N1], aU[N1];
+    double DD[P], DC[P], DU[P];
 #pragma unroll
-    for (int m = 0; m < N1; ++m) aC[m] = B[k][m][ty][tx];
+    for (int m = 0; m < P; ++m) DC[m] = B[k][m][ty][tx];
     const int ph = (METHOD == 1 && phys == 3 && k == 2) ? 5 : phys;
     if (ph == 0) {
 #pragma unroll
-      for (int m = 0; m < N1; ++m) { aD[m] = B[k][m][ty - 1][tx]; aU[m] = B[k][m][ty + 1][tx]; }
-      limit_monomial<P>(aD, aC, aU, lim[k]);
+      for (int m = 0; m < P; ++m) { DD[m] = B[k][m][ty - 1][tx]; DU[m] = B[k][m][ty + 1][tx]; }
+      hr_limit<P>(DD, DC, DU, lim[k]);
     } else if (ph == 2 || ph == 3) {
-      average_monomial<P>(aC, lim[k]);
+      hr_flat<P>(DC, lim[k]);
     } else {
-#pragma unroll
-      for (int m = 0; m < N1; ++m) lim[k][m] = aC[m];
+      to_mono<P>(col[k], lim[k]);
     }
   }
   if constexpr (METHOD == 1) {
@@ -241,16 +234,14 @@ __device__ __forceinline__ void lim2d_ypass_body(const LimArgs la, int nx, int n
       for (int iy = 0; iy < N1; ++iy) Uout[(size_t)(k * NS + ix + N1 * iy) * ld + e] = out[iy];
     }
   } else {
-    double r_[N1], u_[N1], v_[N1], a_[N1], K[N1], Km[N1], El[N1], E_[N1];
+    double r_[N1], u_[N1], v_[N1], a_[N1], K[N1], E_[N1];
     to_lag<P>(lim[0], r_);
     to_lag<P>(lim[1], u_);
     to_lag<P>(lim[2], v_);
     to_lag<P>(lim[3], a_);
 #pragma unroll
-    for (int iy = 0; iy < N1; ++iy) K[iy] = 0.5 * (u_[iy] * u_[iy] + v_[iy] * v_[iy]) * __drcp_rn(r_[iy]);
-    to_mono<P>(K, Km);
-    reconstruct_energy<P>(lim[4], lim[3], Km, Em, El);
-    to_lag<P>(El, E_);
+    for (int iy = 0; iy < N1; ++iy) K[iy] = 0.5 * (u_[iy] * u_[iy] + v_[iy] * v_[iy]) * phys::rcp(r_[iy]);
+    rebuild_energy<P>(lim[4], lim[3], K, vE, E_);
 #pragma unroll
     for (int iy = 0; iy < N1; ++iy) {
       const size_t o = (size_t)(ix + N1 * iy) * ld + e;
@@ -286,223 +277,165 @@ __global__ void __launch_bounds__(32 * 6) lim2d_ypass_tile_kernel(const LimArgs 
 
 namespace dgb {
 
-template <int P, int METHOD>
-constexpr size_t lim2d_fused_smem_bytes() {
-  return ((size_t)5 * (P + 1) * (P + 1) * 32 + (size_t)3 * (METHOD == 2 ? 6 : 5) * (P + 1) * (P + 1) * 32) *
-         sizeof(double);
-}
+// Both limiter passes in one launch, out of place.  A warp is one slice of one element row of the tile,
+// a lane one element: 30 elements and the neighbour on either side; ROWS rows and the row below and
+// above, P + 1 warps each.  The x pass (warp = y-slice) takes the neighbours' moments by shuffle and leaves
+// the x-limited nodes in shared memory; the y pass (warp = x-column) reads its column and those of
+// the rows above and below from there, so the x-limited state never goes to memory.  Uout must not alias U.
+// Per stage of m2l, against the two passes through a global scratch: p = 2, 512 x 256: 52 -> 33 us; p = 3,
+// 1024 x 512: 326 -> 212; p = 1, 1024 x 256: 34 -> 23.  The two passes were FP64-bound at half the memory
+// rate (2,240 FP64 instructions per p = 2 element, 1,280 now with the halo rows' second x pass) and moved
+// 35 B per value; this moves 16 plus halos (15 us at the copy rate) and waits on its loads: long
+// scoreboard 4.3 of 12 stall cycles at 36 warps per SM, FP64 pipe 37 %.
+// Rows per tile: more rows repeat less x work, fewer leave room for a second CTA.  p = 2: 2 rows 41 us,
+// 3: 35, 4 (two CTAs): 35, 6: 35, 8: 33; p = 3: 1: 436, 2: 242, 3: 224, 4: 212; p = 1: 4: 26, 6: 27, 8 (two
+// CTAs): 23, 8 (three): 33, 14: 35.  One thread per element with all slices in registers (164
+// registers, 12 warps per SM, moments through shared memory) took 39 us at p = 2 and 330 at p = 3.
+template <int P, int METHOD, int NY>
+struct LimDims {
+  static constexpr int NQ = 5 + NY, N1 = P + 1, NX = NQ + (METHOD == 2 ? 1 : 0);  // m2: E after the quantities
+  static constexpr int ROWS = P == 3 ? 4 : 8;
+  static constexpr int PITCH = 32 * (ROWS + 2), NT = PITCH * N1;
+  static constexpr size_t smem_bytes = sizeof(double) * NX * N1 * N1 * PITCH;
+  static constexpr int ctas = P == 1 ? 2 : 1;
+};
 
-// Both limiter passes in one kernel.  A CTA owns a strip of 30 element columns and H element rows
-// and walks up the strip one row at a time: the x pass of row r (threads: element slot incl. the
-// left/right neighbour slots, y-slice) writes its x-limited Lagrange values into a three-row ring
-// buffer in shared memory, then the y pass of row r-1 (threads: element slot, x-column) reads
-// rows r-2, r-1, r from the ring and writes the limited state.  The rows below and above the strip
-// are x-limited too (2/H extra x work), so the x-limited intermediate never goes to HBM.  Rows
-// beyond the domain edges come from the neighbour table (periodic wrap) or are absent (walls,
-// transmissive boundaries: the y pass then needs no neighbour).  Same arithmetic as
-// lim2d_xpass_tile_kernel followed by lim2d_ypass_tile_kernel.  Uout must not alias U.
-template <int P, int METHOD, int H>
-__global__ void __launch_bounds__(32 * (P + 1)) lim2d_fused_tile_kernel(const LimArgs la, int nx, int ny,
-                                                                       const double* __restrict__ U,
-                                                                       const int* __restrict__ nbr,
-                                                                       double* __restrict__ Uout,
-                                                                       const DevScalars* __restrict__ scal) {
-  constexpr int N1 = P + 1, NS = N1 * N1, NQ = 5, NQS = METHOD == 2 ? 6 : 5, TWI = 30;
-  extern __shared__ __align__(16) double lsm[];
-  auto A = reinterpret_cast<double(*)[N1][N1][32]>(lsm);                 // [q][slice][m][slot]
-  auto XR = reinterpret_cast<double(*)[NQS][NS][32]>(lsm + NQ * N1 * N1 * 32);  // [row % 3][q][node][slot]
-  if (scal && scal->flags) return;
-  const int ld = la.ld;
-  const int tx = threadIdx.x, sl = threadIdx.y;
-  const int x0 = blockIdx.x * TWI, y0 = blockIdx.y * H;
-  const int nrow = min(H, ny - y0);
-  const int ex = x0 - 1 + tx;
-  const bool icol = tx >= 1 && tx <= TWI && ex < nx;
-  // element of column x (0 <= x < nx) in strip row s (s = 0: the row below, s = nrow + 1: above)
-  auto row_elem = [&](int s, int x) -> int {
-    if (s >= 1 && s <= nrow) return (y0 + s - 1) * nx + x;
-    if (s == 0) return __ldg(nbr + (size_t)2 * ld + y0 * nx + x);
-    return __ldg(nbr + (size_t)3 * ld + (y0 + nrow - 1) * nx + x);
+// one tile: element columns from 30 bx, rows from ROWS by
+template <int P, int METHOD, int NY>
+__device__ __forceinline__ void lim2d_body(const LimArgs la, int nx, int ny, const double* __restrict__ U,
+                                           const int* __restrict__ nbr, double* __restrict__ Uout, int bx, int by,
+                                           double* lsm) {  // lsm: [quantity, node][row][lane], x-limited nodes
+  using Dm = LimDims<P, METHOD, NY>;
+  constexpr int N1 = Dm::N1, NS = N1 * N1, NQ = Dm::NQ, NF = 5 + NY, PITCH = Dm::PITCH;
+  const int ld = la.ld, tx = threadIdx.x, sl = threadIdx.y, row = threadIdx.z;
+  const int ex = bx * 30 - 1 + tx, y = by * Dm::ROWS - 1 + row;
+  // the element of column x in this row: beyond the bottom and top sides what the neighbour table says
+  auto row_elem = [&](int x) -> int {
+    if (y < 0) return __ldg(nbr + (size_t)2 * ld + x);
+    if (y == ny) return __ldg(nbr + (size_t)3 * ld + (size_t)(ny - 1) * nx + x);
+    return y < ny ? y * nx + x : -1;
   };
-  auto lane_elem = [&](int s) -> int {
-    if (icol) return row_elem(s, ex);
-    if (tx == 0) {
-      const int e1 = row_elem(s, x0);
-      return e1 >= 0 ? __ldg(nbr + e1) : -1;
-    }
-    if (ex - 1 < nx && ex - 1 >= 0) {
-      const int el = row_elem(s, ex - 1);
-      return el >= 0 ? __ldg(nbr + (size_t)ld + el) : -1;
-    }
-    return -1;
-  };
-  double v[5][N1];  // raw values of this lane's slice in the current row (prefetched)
-  int e = lane_elem(0);
-  if (e >= 0) {
-#pragma unroll
-    for (int f = 0; f < 5; ++f)
-#pragma unroll
-      for (int ix = 0; ix < N1; ++ix) v[f][ix] = __ldg(U + (size_t)(f * NS + ix + N1 * sl) * ld + e);
+  int e = -1;
+  if (ex < 0 || ex == nx) {
+    const int in = row_elem(ex < 0 ? 0 : nx - 1);
+    if (in >= 0) e = __ldg(nbr + (ex < 0 ? 0 : (size_t)ld) + in);
+  } else if (ex < nx) {
+    e = row_elem(ex);
   }
-  for (int s = 0; s <= nrow + 1; ++s) {
-    // ---- x pass of strip row s: monomial coefficients of every slot ----
-    double Em[N1];
-    if (e >= 0) {
-      double q[NQ][N1];
+  const bool icol = tx >= 1 && tx <= 30 && ex < nx;
+  double* B = lsm + row * 32 + tx;
+  // ---- x pass: the slice iy = sl ----
+  {
+    double v[NF][N1];
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+      for (int ix = 0; ix < N1; ++ix) v[f][ix] = e >= 0 ? __ldg(U + (size_t)(f * NS + ix + N1 * sl) * ld + e) : 1.0;
+    int phx = 0;
+    if (e >= 0 && icol && (ex == 0 || ex == nx - 1))
+      phx = boundary_code(ex == 0 ? __ldg(nbr + e) : 0, ex == nx - 1 ? __ldg(nbr + (size_t)ld + e) : 0);
+    double o[NQ][N1], lp[N1], la_[N1];
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+      double q[N1], DC[P], DL[P], DR[P], lim[N1];
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) {
-        if constexpr (METHOD == 1) {
-#pragma unroll
-          for (int f = 0; f < 5; ++f) q[f][ix] = v[f][ix];
-        } else {
-          q[0][ix] = v[0][ix];
-          q[1][ix] = v[1][ix];
-          q[2][ix] = v[2][ix];
-          q[3][ix] = v[4][ix];
-          const double ru = v[1][ix], rv = v[2][ix];
-          q[4][ix] = __drcp_rn(v[4][ix]) * (v[3][ix] - 0.5 * (ru * ru + rv * rv) * __drcp_rn(v[0][ix]));
-        }
+        if (METHOD == 1 || k >= 5) q[ix] = v[k][ix];
+        else if (k < 3) q[ix] = v[k][ix];
+        else if (k == 3) q[ix] = v[4][ix];
+        else  // pressure from the unlimited state (pressure kernel, physics.cu:891-958)
+          q[ix] = phys::rcp(v[4][ix]) *
+                  (v[3][ix] - 0.5 * (v[1][ix] * v[1][ix] + v[2][ix] * v[2][ix]) * phys::rcp(v[0][ix]));
       }
+      hr_moments<P>(q, DC);
 #pragma unroll
-      for (int k = 0; k < NQ; ++k) {
-        double am[N1];
-        to_mono<P>(q[k], am);
-#pragma unroll
-        for (int m = 0; m < N1; ++m) A[k][sl][m][tx] = am[m];
+      for (int m = 0; m < P; ++m) {
+        DL[m] = __shfl_up_sync(0xffffffffu, DC[m], 1);
+        DR[m] = __shfl_down_sync(0xffffffffu, DC[m], 1);
       }
-      if constexpr (METHOD == 2) to_mono<P>(v[3], Em);
-    }
-    __syncthreads();
-    // ---- x pass: limit the interior slots, x-limited Lagrange values into the ring ----
-    const int slot = s % 3;
-    if (icol && e >= 0) {
-      const int phys = boundary_code(__ldg(nbr + e), __ldg(nbr + (size_t)ld + e));
-      double lim[NQ][N1];
-#pragma unroll
-      for (int k = 0; k < NQ; ++k) {
-        double aL[N1], aC[N1], aR[N1];
-#pragma unroll
-        for (int m = 0; m < N1; ++m) aC[m] = A[k][sl][m][tx];
-        const int ph = (METHOD == 1 && phys == 3 && k == 1) ? 5 : phys;
-        if (ph == 0) {
-#pragma unroll
-          for (int m = 0; m < N1; ++m) { aL[m] = A[k][sl][m][tx - 1]; aR[m] = A[k][sl][m][tx + 1]; }
-          limit_monomial<P>(aL, aC, aR, lim[k]);
-        } else if (ph == 2 || ph == 3) {
-          average_monomial<P>(aC, lim[k]);
-        } else {
-#pragma unroll
-          for (int m = 0; m < N1; ++m) lim[k][m] = aC[m];
-        }
+      hr_limit<P>(DL, DC, DR, lim);
+      if (phx != 0) {
+        if (phx == 4 || (METHOD == 1 && phx == 3 && k == 1)) to_mono<P>(q, lim);
+        else hr_flat<P>(DC, lim);
       }
-      if constexpr (METHOD == 1) {
+      to_lag<P>(lim, o[k]);
 #pragma unroll
-        for (int k = 0; k < NQ; ++k) {
-          double out[N1];
-          to_lag<P>(lim[k], out);
-#pragma unroll
-          for (int ix = 0; ix < N1; ++ix) XR[slot][k][ix + N1 * sl][tx] = out[ix];
-        }
-      } else {
-        double r_[N1], u_[N1], v_[N1], a_[N1], p_[N1], K[N1], Km[N1], El[N1], E_[N1];
-        to_lag<P>(lim[0], r_);
-        to_lag<P>(lim[1], u_);
-        to_lag<P>(lim[2], v_);
-        to_lag<P>(lim[3], a_);
-        to_lag<P>(lim[4], p_);
-#pragma unroll
-        for (int ix = 0; ix < N1; ++ix) K[ix] = 0.5 * (u_[ix] * u_[ix] + v_[ix] * v_[ix]) * __drcp_rn(r_[ix]);
-        to_mono<P>(K, Km);
-        reconstruct_energy<P>(lim[4], lim[3], Km, Em, El);
-        to_lag<P>(El, E_);
-#pragma unroll
-        for (int ix = 0; ix < N1; ++ix) {
-          const int t = ix + N1 * sl;
-          XR[slot][0][t][tx] = r_[ix];
-          XR[slot][1][t][tx] = u_[ix];
-          XR[slot][2][t][tx] = v_[ix];
-          XR[slot][3][t][tx] = a_[ix];
-          XR[slot][4][t][tx] = p_[ix];
-          XR[slot][5][t][tx] = E_[ix];
-        }
+      for (int ix = 0; ix < N1; ++ix) {
+        B[(k * NS + ix + N1 * sl) * PITCH] = o[k][ix];
+        if (METHOD == 2 && k == 3) la_[ix] = lim[ix];
+        if (METHOD == 2 && k == 4) lp[ix] = lim[ix];
       }
     }
-    __syncthreads();
-    // prefetch the next row's raw values while the y pass runs
-    if (s <= nrow) {
-      e = lane_elem(s + 1);
-      if (e >= 0) {
+    if constexpr (METHOD == 2) {
+      double K[N1], E[N1];
 #pragma unroll
-        for (int f = 0; f < 5; ++f)
+      for (int ix = 0; ix < N1; ++ix)
+        K[ix] = 0.5 * (o[1][ix] * o[1][ix] + o[2][ix] * o[2][ix]) * phys::rcp(o[0][ix]);
+      rebuild_energy<P>(lp, la_, K, v[3], E);
 #pragma unroll
-          for (int ix = 0; ix < N1; ++ix) v[f][ix] = __ldg(U + (size_t)(f * NS + ix + N1 * sl) * ld + e);
-      }
-    }
-    // ---- y pass of strip row s - 1 (threads: slot, x-column ix = threadIdx.y) ----
-    if (s >= 2 && icol) {
-      const int ix = sl;
-      const int ec = (y0 + s - 2) * nx + ex;
-      const int phys = boundary_code(__ldg(nbr + (size_t)2 * ld + ec), __ldg(nbr + (size_t)3 * ld + ec));
-      const int cD = (s - 2) % 3, cC = (s - 1) % 3, cU = s % 3;
-      double lim[NQ][N1], Emy[N1];
-#pragma unroll
-      for (int k = 0; k < NQ; ++k) {
-        double col[N1], aC[N1];
-#pragma unroll
-        for (int iy = 0; iy < N1; ++iy) col[iy] = XR[cC][k][ix + N1 * iy][tx];
-        to_mono<P>(col, aC);
-        const int ph = (METHOD == 1 && phys == 3 && k == 2) ? 5 : phys;
-        if (ph == 0) {
-          double aD[N1], aU[N1];
-#pragma unroll
-          for (int iy = 0; iy < N1; ++iy) col[iy] = XR[cD][k][ix + N1 * iy][tx];
-          to_mono<P>(col, aD);
-#pragma unroll
-          for (int iy = 0; iy < N1; ++iy) col[iy] = XR[cU][k][ix + N1 * iy][tx];
-          to_mono<P>(col, aU);
-          limit_monomial<P>(aD, aC, aU, lim[k]);
-        } else if (ph == 2 || ph == 3) {
-          average_monomial<P>(aC, lim[k]);
-        } else {
-#pragma unroll
-          for (int m = 0; m < N1; ++m) lim[k][m] = aC[m];
-        }
-      }
-      if constexpr (METHOD == 1) {
-#pragma unroll
-        for (int k = 0; k < NQ; ++k) {
-          double out[N1];
-          to_lag<P>(lim[k], out);
-#pragma unroll
-          for (int iy = 0; iy < N1; ++iy) Uout[(size_t)(k * NS + ix + N1 * iy) * ld + ec] = out[iy];
-        }
-      } else {
-        double col[N1];
-#pragma unroll
-        for (int iy = 0; iy < N1; ++iy) col[iy] = XR[cC][5][ix + N1 * iy][tx];
-        to_mono<P>(col, Emy);
-        double r_[N1], u_[N1], v_[N1], a_[N1], K[N1], Km[N1], El[N1], E_[N1];
-        to_lag<P>(lim[0], r_);
-        to_lag<P>(lim[1], u_);
-        to_lag<P>(lim[2], v_);
-        to_lag<P>(lim[3], a_);
-#pragma unroll
-        for (int iy = 0; iy < N1; ++iy) K[iy] = 0.5 * (u_[iy] * u_[iy] + v_[iy] * v_[iy]) * __drcp_rn(r_[iy]);
-        to_mono<P>(K, Km);
-        reconstruct_energy<P>(lim[4], lim[3], Km, Emy, El);
-        to_lag<P>(El, E_);
-#pragma unroll
-        for (int iy = 0; iy < N1; ++iy) {
-          const size_t o = (size_t)(ix + N1 * iy) * ld + ec;
-          Uout[o + (size_t)0 * NS * ld] = r_[iy];
-          Uout[o + (size_t)1 * NS * ld] = u_[iy];
-          Uout[o + (size_t)2 * NS * ld] = v_[iy];
-          Uout[o + (size_t)3 * NS * ld] = E_[iy];
-          Uout[o + (size_t)4 * NS * ld] = a_[iy];
-        }
-      }
+      for (int ix = 0; ix < N1; ++ix) B[(NQ * NS + ix + N1 * sl) * PITCH] = E[ix];
     }
   }
+  __syncthreads();
+  // ---- y pass: the column ix = sl ----
+  if (!icol || row < 1 || row > Dm::ROWS || y >= ny) return;
+  int phy = 0;
+  if (y == 0 || y == ny - 1)
+    phy = boundary_code(y == 0 ? __ldg(nbr + (size_t)2 * ld + e) : 0, y == ny - 1 ? __ldg(nbr + (size_t)3 * ld + e) : 0);
+  double* out = Uout + (size_t)sl * ld + e;
+  double o[NQ][N1], lp[N1], la_[N1];
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) {
+    double c[N1], w[N1], DC[P], DD[P], DU[P], lim[N1];
+    const double* b = B + (k * NS + sl) * PITCH;
+#pragma unroll
+    for (int iy = 0; iy < N1; ++iy) c[iy] = b[N1 * iy * PITCH];
+    hr_moments<P>(c, DC);
+    if (phy == 0) {
+#pragma unroll
+      for (int iy = 0; iy < N1; ++iy) w[iy] = b[N1 * iy * PITCH - 32];
+      hr_moments<P>(w, DD);
+#pragma unroll
+      for (int iy = 0; iy < N1; ++iy) w[iy] = b[N1 * iy * PITCH + 32];
+      hr_moments<P>(w, DU);
+      hr_limit<P>(DD, DC, DU, lim);
+    } else if (phy == 4 || (METHOD == 1 && phy == 3 && k == 2)) {
+      to_mono<P>(c, lim);
+    } else {
+      hr_flat<P>(DC, lim);
+    }
+    to_lag<P>(lim, o[k]);
+#pragma unroll
+    for (int iy = 0; iy < N1; ++iy) {
+      const size_t t = (size_t)(N1 * iy) * ld;
+      if (METHOD == 1 || k >= 5 || k < 3) out[t + (size_t)k * NS * ld] = o[k][iy];
+      else if (k == 3) out[t + (size_t)4 * NS * ld] = o[k][iy];
+      if (METHOD == 2 && k == 3) la_[iy] = lim[iy];
+      if (METHOD == 2 && k == 4) lp[iy] = lim[iy];
+    }
+  }
+  if constexpr (METHOD == 2) {
+    double K[N1], vE[N1], E[N1];
+#pragma unroll
+    for (int iy = 0; iy < N1; ++iy) {
+      vE[iy] = B[(NQ * NS + sl + N1 * iy) * PITCH];
+      K[iy] = 0.5 * (o[1][iy] * o[1][iy] + o[2][iy] * o[2][iy]) * phys::rcp(o[0][iy]);
+    }
+    rebuild_energy<P>(lp, la_, K, vE, E);
+#pragma unroll
+    for (int iy = 0; iy < N1; ++iy) out[(size_t)(N1 * iy + 3 * NS) * ld] = E[iy];
+  }
+}
+
+template <int P, int METHOD, int NY>
+__global__ void __launch_bounds__(LimDims<P, METHOD, NY>::NT, LimDims<P, METHOD, NY>::ctas)
+    lim2d_kernel(const LimArgs la, int nx, int ny, const double* __restrict__ U, const int* __restrict__ nbr,
+                 double* __restrict__ Uout, const DevScalars* __restrict__ scal) {
+  extern __shared__ __align__(16) double lsm[];
+  pdl_wait();
+  if (scal && scal->flags) return;
+  lim2d_body<P, METHOD, NY>(la, nx, ny, U, nbr, Uout, blockIdx.x, blockIdx.y, lsm);
+  pdl_trigger();
 }
 
 }  // namespace dgb

@@ -90,16 +90,13 @@ __device__ __forceinline__ void m2i_slice(int phys, const double (&c)[D + 3][P +
     }
   }
   // total energy from the limited pressure, 1/(gamma-1) and kinetic energy
-  double K[N1], Km[N1], Em[N1], El[N1];
+  double K[N1];
 #pragma unroll
   for (int k = 0; k < N1; ++k) {
     const double kin = res[1][k] * res[1][k] + (D == 2 ? res[2][k] * res[2][k] : 0.0);
     K[k] = 0.5 * kin * __drcp_rn(res[0][k]);
   }
-  to_mono<P>(K, Km);
-  to_mono<P>(c[IE], Em);
-  reconstruct_energy<P>(mp, ma, Km, Em, El);
-  to_lag<P>(El, res[IE]);
+  rebuild_energy<P>(mp, ma, K, c[IE], res[IE]);
 }
 
 // One pass of hri / pri (METHOD 1) or m2i (METHOD 2).  PASS 0: x slices (row iy = blockIdx.y,

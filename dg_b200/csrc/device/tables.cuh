@@ -1,7 +1,6 @@
-// Reference-element tables in __constant__ memory: the limiter's monomial transforms and
-// integrals (c_lim_p*) and the tensor-product tables of the 2D tiled residual kernels (c_tab2_p*,
-// FP32 copies c_tab2f_p*), and in global memory the lane tables of the p = 2 DMMA residual
-// (g_dmma_tab2).  Those symbols are static, one copy per translation unit (each .cu file
+// Reference-element tables in __constant__ memory: the tensor-product tables of the 2D tiled residual
+// kernels (c_tab2_p*, FP32 copies c_tab2f_p*), and in global memory the lane tables of the p = 2 DMMA
+// residual (g_dmma_tab2).  Those symbols are static, one copy per translation unit (each .cu file
 // is its own device module), so every .cu file that launches kernels reading them calls
 // upload_tables from its own code; the function is static for the same reason.
 #pragma once
@@ -134,25 +133,8 @@ static DmmaTab2 make_dmma_tab2(const Tab2<2>& d) {
   return T;
 }
 
-// Tables of order p (and, in 2D, the tiled kernels' tables) from the problem constants.
+// The 2D tiled kernels' tables of order p from the problem constants.
 static int upload_tables(const Consts& cs, int D, int p) {
-  cudaError_t el = cudaSuccess;
-  auto fill = [&](auto& t, int n1) {
-    std::memset(&t, 0, sizeof(t));
-    for (int m = 0; m < n1; ++m)
-      for (int i = 0; i < n1; ++i) {
-        t.T[m][i] = cs.T[m][i];
-        t.Tinv[m][i] = cs.Tinv[m][i];
-        t.imd[m][i] = cs.imd[m][i];
-        t.imdL[m][i] = cs.imdL[m][i];
-        t.imdR[m][i] = cs.imdR[m][i];
-      }
-    for (int k = 0; k < n1 + 2; ++k) t.ifact[k] = cs.ifact[k];
-  };
-  if (p == 1) { LimTab<1> t; fill(t, 2); el = cudaMemcpyToSymbol(c_lim_p1, &t, sizeof(t)); }
-  if (p == 2) { LimTab<2> t; fill(t, 3); el = cudaMemcpyToSymbol(c_lim_p2, &t, sizeof(t)); }
-  if (p == 3) { LimTab<3> t; fill(t, 4); el = cudaMemcpyToSymbol(c_lim_p3, &t, sizeof(t)); }
-  if (el != cudaSuccess) return set_error(5, std::string("limiter tables: ") + cudaGetErrorString(el));
   if (D == 2) {
     cudaError_t et = cudaSuccess;
     if (p == 1) {

@@ -36,6 +36,7 @@ struct ColTab {
   double EX[2][MAXN], EY[2][MAXN];  // M1^-1 column of the first / last node, face metric and sign
 };
 
+// One stage of one problem
 struct ColArgs {
   const double* __restrict__ U;     // stage input
   const double* base;               // out = k0 base + k1 U + k2 du   (base not read when k0 == 0;
@@ -48,8 +49,8 @@ struct ColArgs {
   long long polls;                  // budget of the first wait on each tile copy (then drained)
   double k0, k1, k2, c2;
   double dt;                        // du = dt M^-1 (...); 0: the step in scal
+  double sx, sy;                    // SCALED: 2/hx, 2/hy (the tables are those of hx = hy = 2)
   int nx, ny, ld, tma;
-  ColTab t;
 };
 
 // Shapes.  The kernel is bound by instruction issue and latency, not by bandwidth: of some 7,300
@@ -63,12 +64,16 @@ struct ColArgs {
 //   p = 3, 1024 x 512   888 us; 16 x 2: 450, 8 x 4: 437, 16 x 4: 479, 32 x 2: 493, 8 x 8: 491   (Roe)
 // Small tiles pay more faces per element (16 x 4: 2.31, 16 x 2: 2.56) but put more CTAs on an SM, whose
 // loads, barriers and compute phases then overlap.
-template <int P, int NY, bool GC>
+template <int P>
+constexpr int col_tw() { return P == 3 ? 8 : 16; }
+template <int P>
+constexpr int col_th() { return P == 2 ? 2 : 4; }
+template <int P, int NY, bool GC, int TW_ = col_tw<P>(), int TH_ = col_th<P>()>
 struct ColDims {
   static constexpr int N1 = P + 1, NS = N1 * N1, NF = 5 + NY, NG1 = P == 1 ? 2 : P + 2;
   static constexpr int NFL = 4 + NY + (GC ? 1 : 0);       // fields with a conservative volume flux
   static constexpr int NA = (2 * NFL + (GC ? 0 : 1)) * N1;  // column sums per thread
-  static constexpr int TW = P == 3 ? 8 : 16, TH = P == 2 ? 2 : 4;
+  static constexpr int TW = TW_, TH = TH_;
   static constexpr int NE = TW * TH, NT = NE * NG1;
   static constexpr int NXF = (TW + 1) * TH, NYF = TW * (TH + 1), NFACE = NXF + NYF;
   static constexpr int NEDGE = 2 * TH + 2 * TW;           // edge slots: left, right, bottom, top
@@ -151,14 +156,17 @@ __device__ __forceinline__ void riemann_n2(const double* L, const double* R, dou
   }
 }
 
-template <int P, int FLUX, int NY, bool GC>
-__global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ctas)
-    residual2d_cols_kernel(const __grid_constant__ ColArgs a, const __grid_constant__ CUtensorMap mapU) {
+// The work of one tile (origin tx0, ty0).  The caller has initialised the mbarrier at the start of shared
+// memory; `phase` counts its completed phases (a persistent caller runs many tiles on one barrier).  Every
+// early return is taken by the whole CTA, after its last barrier.
+// SCALED: the tables carry no metric, a.sx and a.sy do (tiles of problems of many mesh widths).
+template <int P, int FLUX, int NY, bool GC, int TW, int TH, bool SCALED>
+__device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, const CUtensorMap* mapU, int tx0, int ty0,
+                                          unsigned char* smraw, uint32_t& phase) {
   static_assert(!(GC && NY > 0), "GAMCONS with mass fractions is not built");
-  using Dm = ColDims<P, NY, GC>;
+  using Dm = ColDims<P, NY, GC, TW, TH>;
   constexpr int N1 = Dm::N1, NS = Dm::NS, NF = Dm::NF, NFL = Dm::NFL, NG1 = Dm::NG1;
-  constexpr int TW = Dm::TW, TH = Dm::TH, NE = Dm::NE, NT = Dm::NT, NXF = Dm::NXF, NFACE = Dm::NFACE;
-  extern __shared__ __align__(128) unsigned char smraw[];
+  constexpr int NE = Dm::NE, NT = Dm::NT, NXF = Dm::NXF, NFACE = Dm::NFACE;
   uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);
   int* s_ok = reinterpret_cast<int*>(smraw + 8);
   int* codes = reinterpret_cast<int*>(smraw + Dm::off_code);       // [NEDGE] neighbours / boundary codes
@@ -167,11 +175,7 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
   double* FS = reinterpret_cast<double*>(smraw + Dm::off_face);    // [(NF+1)*N1][NFACE] lifted face fluxes
   double* AS = reinterpret_cast<double*>(smraw + Dm::off_sums);    // [NA][NT] column sums
   const int tid = threadIdx.x, ld = a.ld, nx = a.nx;
-  const int tx0 = blockIdx.x * TW, ty0 = blockIdx.y * TH;
   const int tw = min(TW, nx - tx0), th = min(TH, a.ny - ty0);
-
-  pdl_wait();
-  if (a.scal && a.scal->flags) return;
 
   // ---------------- the tile and the neighbours' face nodes ----------------
   // a TMA copy must land on a 128-byte shared boundary and start on a 16-byte global column;
@@ -179,10 +183,8 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
   const bool tma_ok = a.tma && (smem_u32(Us) & 127u) == 0 && ((tx0 * 8) & 15) == 0;
   if (tid == 0) {
     if (tma_ok) {
-      mbar_init(bar, 1);
-      fence_mbar_init();
       mbar_arrive_expect_tx(bar, (uint32_t)Dm::tile_bytes);
-      tma_load_3d(Us, &mapU, tx0, ty0, 0, bar);
+      tma_load_3d(Us, mapU, tx0, ty0, 0, bar);
     } else if (a.tma) {
       atomicOr(a.errflag, (unsigned)FLAG_TIMEOUT);
     }
@@ -221,13 +223,14 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
     }
   }
   if (tid == 0) {
-    bool ok = !a.tma || (tma_ok && mbar_wait(bar, 0, a.polls));
+    bool ok = !a.tma || (tma_ok && mbar_wait(bar, phase & 1, a.polls));
     if (tma_ok && !ok) {
       atomicOr(a.errflag, (unsigned)FLAG_TIMEOUT);
-      mbar_wait(bar, 0);
+      mbar_wait(bar, phase & 1);
     }
     *s_ok = ok ? 1 : 0;
   }
+  if (tma_ok) ++phase;
   __syncthreads();
   if (!*s_ok) return;
 
@@ -239,7 +242,7 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
       {
         double b[N1], d[N1];
 #pragma unroll
-        for (int ix = 0; ix < N1; ++ix) { b[ix] = a.t.B1[gx][ix]; d[ix] = a.t.Dx[gx][ix]; }
+        for (int ix = 0; ix < N1; ++ix) { b[ix] = tab.B1[gx][ix]; d[ix] = SCALED ? a.sx * tab.Dx[gx][ix] : tab.Dx[gx][ix]; }
 #pragma unroll
         for (int iy = 0; iy < N1; ++iy) {
 #pragma unroll
@@ -262,9 +265,9 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
         double ug[NF];
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
-          ug[f] = a.t.B1[gy][0] * T[f][0];
+          ug[f] = tab.B1[gy][0] * T[f][0];
 #pragma unroll
-          for (int iy = 1; iy < N1; ++iy) ug[f] += a.t.B1[gy][iy] * T[f][iy];
+          for (int iy = 1; iy < N1; ++iy) ug[f] += tab.B1[gy][iy] * T[f][iy];
         }
         // volume flux and alpha source (evaluate_sf, code/src/physics/physics.cu:248-301)
         const double rho = ug[0], ir = phys::rcp(rho), ia = phys::rcp(ug[4]);
@@ -282,21 +285,22 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
 #pragma unroll
           for (int f = 0; f < NFL; ++f) {
             if (gy == 0) {
-              Ax[f][iy] = a.t.LB[0][iy] * fx[f];
-              Ay[f][iy] = a.t.LD[0][iy] * fy[f];
+              Ax[f][iy] = tab.LB[0][iy] * fx[f];
+              Ay[f][iy] = tab.LD[0][iy] * fy[f];
             } else {
-              Ax[f][iy] += a.t.LB[gy][iy] * fx[f];
-              Ay[f][iy] += a.t.LD[gy][iy] * fy[f];
+              Ax[f][iy] += tab.LB[gy][iy] * fx[f];
+              Ay[f][iy] += tab.LD[gy][iy] * fy[f];
             }
           }
         }
         if constexpr (!GC) {
-          double dax = a.t.B1[gy][0] * dT[0], day = a.t.Dy[gy][0] * T[4][0];
+          double dax = tab.B1[gy][0] * dT[0], day = tab.Dy[gy][0] * T[4][0];
 #pragma unroll
-          for (int iy = 1; iy < N1; ++iy) { dax += a.t.B1[gy][iy] * dT[iy]; day += a.t.Dy[gy][iy] * T[4][iy]; }
+          for (int iy = 1; iy < N1; ++iy) { dax += tab.B1[gy][iy] * dT[iy]; day += tab.Dy[gy][iy] * T[4][iy]; }
+          if (SCALED) day *= a.sy;
           const double src = -(u * dax + v * day);
 #pragma unroll
-          for (int iy = 0; iy < N1; ++iy) As[iy] = gy == 0 ? a.t.LB[0][iy] * src : As[iy] + a.t.LB[gy][iy] * src;
+          for (int iy = 0; iy < N1; ++iy) As[iy] = gy == 0 ? tab.LB[0][iy] * src : As[iy] + tab.LB[gy][iy] * src;
         }
       }
 #pragma unroll
@@ -348,10 +352,10 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
       for (int j = 0; j < N1; ++j) { vl[j] = pL[ff * sfL + j * sjL]; vr[j] = pR[ff * sfR + j * sjR]; }
 #pragma unroll
       for (int g = 0; g < N1; ++g) {
-        tl[f][g] = a.t.BF[g][0] * vl[0];
-        tr[f][g] = a.t.BF[g][0] * vr[0];
+        tl[f][g] = tab.BF[g][0] * vl[0];
+        tr[f][g] = tab.BF[g][0] * vr[0];
 #pragma unroll
-        for (int j = 1; j < N1; ++j) { tl[f][g] += a.t.BF[g][j] * vl[j]; tr[f][g] += a.t.BF[g][j] * vr[j]; }
+        for (int j = 1; j < N1; ++j) { tl[f][g] += tab.BF[g][j] * vl[j]; tr[f][g] += tab.BF[g][j] * vr[j]; }
       }
     }
     if (code < 0) {
@@ -375,7 +379,7 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
 #pragma unroll
         for (int j = 0; j < N1; ++j) {
           const double v = f < NF ? F2[f < NF ? f : 0] : am;
-          Ff[f][j] = g == 0 ? a.t.LF[0][j] * v : Ff[f][j] + a.t.LF[g][j] * v;
+          Ff[f][j] = g == 0 ? tab.LF[0][j] * v : Ff[f][j] + tab.LF[g][j] * v;
         }
     }
     if (flip) {  // -F with the same nc: the two alpha records trade places
@@ -433,28 +437,30 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
         for (int gx = 0; gx < NG1; ++gx) {
           const double v = as[gx * NE];
 #pragma unroll
-          for (int ix = 0; ix < N1; ++ix) s[ix] = gx == 0 ? a.t.XS[0][ix] * v : s[ix] + a.t.XS[gx][ix] * v;
+          for (int ix = 0; ix < N1; ++ix) s[ix] = gx == 0 ? tab.XS[0][ix] * v : s[ix] + tab.XS[gx][ix] * v;
         }
       } else {
         const double* as = AS + (GC || NY == 0 || r < 4 * N1 ? r : r - N1) * NT + el;
 #pragma unroll
         for (int gx = 0; gx < NG1; ++gx) {
-          const double vx = as[gx * NE], vy = as[NFL * N1 * NT + gx * NE];
+          double vx = as[gx * NE], vy = as[NFL * N1 * NT + gx * NE];
+          if (SCALED) { vx *= a.sx; vy *= a.sy; }
 #pragma unroll
           for (int ix = 0; ix < N1; ++ix) {
-            s[ix] = gx == 0 ? a.t.XD[0][ix] * vx : s[ix] + a.t.XD[gx][ix] * vx;
-            s[ix] += a.t.XB[gx][ix] * vy;
+            s[ix] = gx == 0 ? tab.XD[0][ix] * vx : s[ix] + tab.XD[gx][ix] * vx;
+            s[ix] += tab.XB[gx][ix] * vy;
           }
         }
       }
       {
         const int far = alpha ? (NF - 4) * N1 * NFACE : 0;  // the record the element left of / below a face reads
-        const double l = fx[q * NG1 * NFACE], rr = fx[q * NG1 * NFACE + 1 + far];
+        double l = fx[q * NG1 * NFACE], rr = fx[q * NG1 * NFACE + 1 + far];
         const double* fy = FS + (r - iy) * NFACE + NXF + el;
-        const double eb = a.t.EY[0][iy], et = a.t.EY[1][iy];
+        double eb = tab.EY[0][iy], et = tab.EY[1][iy];
+        if (SCALED) { l *= a.sx; rr *= a.sx; eb *= a.sy; et *= a.sy; }
 #pragma unroll
         for (int ix = 0; ix < N1; ++ix)
-          s[ix] += a.t.EX[0][ix] * l + a.t.EX[1][ix] * rr + eb * fy[ix * NFACE] + et * fy[ix * NFACE + TW + far];
+          s[ix] += tab.EX[0][ix] * l + tab.EX[1][ix] * rr + eb * fy[ix * NFACE] + et * fy[ix * NFACE + TW + far];
       }
       const double* us = Us + N1 * r * NE + el;
 #pragma unroll
@@ -469,6 +475,24 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
       }
     }
   }
+}
+
+template <int P, int FLUX, int NY, bool GC>
+__global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ctas)
+    residual2d_cols_kernel(const __grid_constant__ ColArgs a, const __grid_constant__ ColTab tab,
+                           const __grid_constant__ CUtensorMap mapU) {
+  constexpr int TW = col_tw<P>(), TH = col_th<P>();
+  extern __shared__ __align__(128) unsigned char smraw[];
+  if (threadIdx.x == 0) {
+    mbar_init(reinterpret_cast<uint64_t*>(smraw), 1);
+    fence_mbar_init();
+  }
+  pdl_wait();
+  if (a.scal && a.scal->flags) return;
+  uint32_t phase = 0;
+  cols_body<P, FLUX, NY, GC, TW, TH, false>(a, tab, &mapU, blockIdx.x * TW, blockIdx.y * TH, smraw, phase);
+  // (at the end: with the trigger at the start the next launch's CTAs, waiting, hold the shared memory that this
+  // one's last wave could use: 240 -> 256 us per 512 x 256 step)
   pdl_trigger();
 }
 

@@ -22,7 +22,11 @@
 #include "../../include/dgb.h"
 #include "ctx.h"
 #include "device/batch.cuh"
-#include "device/tables.cuh"
+#include "device/kernels.cuh"
+
+namespace dgb {
+ColTab make_col_tab(const Consts& cs, bool raw);  // dgb_tile.cu
+}
 
 using namespace dgb;
 
@@ -35,12 +39,14 @@ using namespace dgb;
 
 namespace {
 
-// residual tile shapes of the 2D classes: width, height (elements), unrolling of the quadrature
-// column loop
+// residual tile shapes of the 2D classes: width, height (elements).  32 x 2 first: two CTAs of 256 threads
+// per SM at p = 2 (the others: one of 512), the fastest in the single-problem kernel too.  unroll is part
+// of the tuning interface; the quadrature loops are always unrolled now, so both 32 x 4 entries run
+// the same kernel.
 struct Shape2 {
   int tw, th, unroll;
 };
-constexpr Shape2 kShapes2[] = {{32, 4, 1}, {32, 2, 1}, {16, 8, 1}, {32, 4, 2}};
+constexpr Shape2 kShapes2[] = {{32, 2, 1}, {32, 4, 1}, {16, 8, 1}, {32, 4, 2}};
 constexpr int kNShapes2 = sizeof(kShapes2) / sizeof(kShapes2[0]);
 constexpr int kChunks1[] = {64, 128, 256};  // elements per CTA item of the 1D classes
 
@@ -52,10 +58,9 @@ struct Class {
   // work items
   int4* d_res = nullptr;  // 2D: tiles of the chosen shape; 1D: element chunks (also the 1D limiter's)
   int n_res = 0;
-  int4* d_x = nullptr;  // 2D limiter x pass
-  int n_x = 0;
-  int4* d_y = nullptr;  // 2D limiter y pass
-  int n_y = 0;
+  int4* d_lim = nullptr;  // 2D limiter tiles
+  int n_lim = 0;
+  ColTab tab;             // 2D: reference-element tables
   int4* d_ws = nullptr;  // wave speed: chunks of 256 elements
   int n_ws = 0;
   // tuning
@@ -128,25 +133,24 @@ int build_res_items(dgb_batch* b, Class& k) {
   return upload_vec(it, &k.d_res);
 }
 
+// element rows of the one-launch limiter's tiles
+int lim_rows(int p) { return p == 1 ? LimDims<1, 2, 0>::ROWS : LimDims<2, 2, 0>::ROWS; }
+
 int build_items(dgb_batch* b, Class& k) {
-  std::vector<int4> ws, xs, ys;
+  std::vector<int4> ws, ls;
   for (int ci : k.cases) {
     dgb_ctx* c = b->ctx[ci];
     for (int e = 0; e < c->ne; e += 256) ws.push_back(item(ci, e, 0, 0));
     if (k.D == 2 && k.limiter) {
-      for (int y = 0; y < c->ny; ++y)
-        for (int x = 0; x < c->nx; x += 30) xs.push_back(item(ci, x, y, 0));
-      for (int ix = 0; ix <= k.p; ++ix)
-        for (int y = 0; y < c->ny; y += 4)
-          for (int x = 0; x < c->nx; x += 32) ys.push_back(item(ci, x, y, ix));
+      const int rows = lim_rows(k.p);
+      for (int by = 0; by * rows < c->ny; ++by)
+        for (int bx = 0; bx * 30 < c->nx; ++bx) ls.push_back(item(ci, bx, by, 0));
     }
   }
   k.n_ws = (int)ws.size();
-  k.n_x = (int)xs.size();
-  k.n_y = (int)ys.size();
+  k.n_lim = (int)ls.size();
   if (int rc = upload_vec(ws, &k.d_ws)) return rc;
-  if (int rc = upload_vec(xs, &k.d_x)) return rc;
-  if (int rc = upload_vec(ys, &k.d_y)) return rc;
+  if (int rc = upload_vec(ls, &k.d_lim)) return rc;
   std::vector<int> ids(k.cases.begin(), k.cases.end());
   if (int rc = upload_vec(ids, &k.d_ids)) return rc;
   return build_res_items(b, k);
@@ -163,25 +167,24 @@ int persistent_grid(dgb_batch* b, K kernel, int threads, size_t smem, int n_item
 
 // ---- launchers (templated on the class's compile-time parameters) ----
 
-template <int P, int FLUX, int TW, int TH, int UNROLL>
+template <int P, int FLUX, int TW, int TH>
 int launch_tile2d_batch(dgb_batch* b, const Class& k, int stage, cudaStream_t st) {
-  auto kern = batch_tile2d_kernel<P, FLUX, TW, TH, UNROLL>;
+  auto kern = batch_tile2d_kernel<P, FLUX, TW, TH>;
   constexpr size_t smem = batch_tile2d_smem_bytes<P, TW, TH>();
+  constexpr int nt = ColDims<P, 0, false, TW, TH>::NT;
   DGB_CUDA(allow_dynamic_smem(kern, smem));
-  const int grid = persistent_grid(b, kern, TW * TH, smem, k.n_res, k.ctas_per_sm);
-  kern<<<grid, TW * TH, smem, st>>>(b->d_cases, b->d_maps, k.d_res, k.n_res, stage);
+  const int grid = persistent_grid(b, kern, nt, smem, k.n_res, k.ctas_per_sm);
+  kern<<<grid, nt, smem, st>>>(b->d_cases, b->d_maps, k.d_res, k.n_res, stage, k.limiter ? 1 : 0, k.tab);
   return 0;
 }
 
 template <int P, int FLUX>
 int tile2d_shape(dgb_batch* b, const Class& k, int stage, cudaStream_t st) {
-  switch (k.shape) {
-    case 0: return launch_tile2d_batch<P, FLUX, 32, 4, 1>(b, k, stage, st);
-    case 1: return launch_tile2d_batch<P, FLUX, 32, 2, 1>(b, k, stage, st);
-    case 2: return launch_tile2d_batch<P, FLUX, 16, 8, 1>(b, k, stage, st);
-    case 3: return launch_tile2d_batch<P, FLUX, 32, 4, 2>(b, k, stage, st);
-    default: return set_error(DGB_ERR_ARG, "batch: tile shape");
-  }
+  const Shape2& s = kShapes2[k.shape];
+  if (s.tw == 32 && s.th == 4) return launch_tile2d_batch<P, FLUX, 32, 4>(b, k, stage, st);
+  if (s.tw == 32 && s.th == 2) return launch_tile2d_batch<P, FLUX, 32, 2>(b, k, stage, st);
+  if (s.tw == 16 && s.th == 8) return launch_tile2d_batch<P, FLUX, 16, 8>(b, k, stage, st);
+  return set_error(DGB_ERR_ARG, "batch: tile shape");
 }
 
 template <int P, int FLUX, bool LIM>
@@ -220,12 +223,11 @@ int launch_residual(dgb_batch* b, const Class& k, int stage, cudaStream_t st) {
 
 template <int P, int M>
 int launch_lim2d_batch(dgb_batch* b, const Class& k, int stage, cudaStream_t st) {
-  auto kx = batch_lim2d_x_kernel<P, M>;
-  auto ky = batch_lim2d_y_kernel<P, M>;
-  const int gx = persistent_grid(b, kx, 32 * (P + 1), 0, k.n_x, 0);
-  const int gy = persistent_grid(b, ky, 32 * 6, 0, k.n_y, 0);
-  kx<<<gx, dim3(32, P + 1), 0, st>>>(b->d_cases, k.d_x, k.n_x, stage);
-  ky<<<gy, dim3(32, 6), 0, st>>>(b->d_cases, k.d_y, k.n_y, stage);
+  using Dm = LimDims<P, M, 0>;
+  auto kern = batch_lim2d_kernel<P, M>;
+  DGB_CUDA(allow_dynamic_smem(kern, Dm::smem_bytes));
+  const int grid = persistent_grid(b, kern, Dm::NT, Dm::smem_bytes, k.n_lim, 0);
+  kern<<<grid, dim3(32, Dm::N1, Dm::ROWS + 2), Dm::smem_bytes, st>>>(b->d_cases, k.d_lim, k.n_lim, stage);
   return 0;
 }
 
@@ -256,7 +258,7 @@ int launch_limiter(dgb_batch* b, const Class& k, int stage, cudaStream_t st) {
     default: return -set_error(DGB_ERR_UNSUPPORTED, "batch: no limiter for this class");
   }
   if (rc) return -rc;
-  return k.D == 2 ? 2 : 1;
+  return 1;
 }
 
 int launch_dt(dgb_batch* b, const Class& k, cudaStream_t st) {
@@ -367,8 +369,8 @@ extern "C" int dgb_batch_create(dgb_ctx* const* cases, int n, dgb_batch** out) {
       if (cases[j] == c) return fail(set_error(DGB_ERR_ARG, "batch: a context appears twice"));
     if (c->nmass != 0 || c->gamcons)
       return fail(set_error(DGB_ERR_UNSUPPORTED, "batch: GAMNCON cases without mass fractions"));
-    if (c->form != DGB_FORM_FP64 || c->ind_on || c->fused_lim)
-      return fail(set_error(DGB_ERR_UNSUPPORTED, "batch: plain FP64 form with the two-pass limiter only"));
+    if (c->form != DGB_FORM_FP64 || c->ind_on)
+      return fail(set_error(DGB_ERR_UNSUPPORTED, "batch: plain FP64 form without the learned indicator only"));
     if (c->limiter != DGB_LIM_NONE && c->limiter != DGB_LIM_HRL && c->limiter != DGB_LIM_M2L)
       return fail(set_error(DGB_ERR_UNSUPPORTED, "batch: limiter none, hrl or m2l"));
     if (c->D == 2 && (!c->tiled_full || c->p > 2))
@@ -397,14 +399,8 @@ extern "C" int dgb_batch_create(dgb_ctx* const* cases, int n, dgb_batch** out) {
     std::memset(&q, 0, sizeof(q));
     q.A = c->A; q.B = c->B; q.C = c->C; q.X = c->X; q.nbr = c->nbr; q.scal = c->scal;
     q.nx = c->nx; q.ny = c->ny; q.ld = c->ld; q.ne = c->ne;
-    q.J = c->cs.J;
-    q.invJ = 1.0 / c->cs.J;
-    q.cx = c->cs.J * c->cs.ixx;
-    q.cy = c->cs.J * c->cs.iyy;
     q.sx = c->cs.ixx;
     q.sy = c->cs.iyy;
-    q.JFx = c->cs.JFx;
-    q.JFy = c->cs.JFy;
     q.cfl_scaled = c->cs.cfl_scaled;
     hk[i] = c->cs;
   }
@@ -436,10 +432,11 @@ extern "C" int dgb_batch_create(dgb_ctx* const* cases, int n, dgb_batch** out) {
         for (int ci : k.cases) ok = ok && b->ctx[ci]->nx % kShapes2[s].tw == 0 && b->ctx[ci]->ny % kShapes2[s].th == 0;
         if (ok) k.valid_shapes.push_back(s);
       }
-      k.shape = k.valid_shapes.front();  // 32 x 4 is always valid for a tiled case
+      k.shape = k.valid_shapes.front();  // 32 x 2 is always valid for a tiled case
+      Consts cs = b->ctx[k.cases.front()]->cs;  // every case of a group has the same order
+      cs.J = cs.ixx = cs.iyy = cs.JFx = cs.JFy = 1.0;
+      k.tab = make_col_tab(cs, false);
     }
-    // this file's copies of the constant tables (every case of a group has the same order)
-    if (int rc = upload_tables(b->ctx[k.cases.front()]->cs, k.D, k.p)) return fail(rc);
     if (int rc = build_items(b, k)) return fail(rc);
   }
   if (cudaDeviceSynchronize() != cudaSuccess) return fail(set_error(DGB_ERR_CUDA, "batch: create"));
@@ -454,7 +451,7 @@ extern "C" void dgb_batch_destroy(dgb_batch* b) {
   drop_graph(b);
   for (Class& k : b->cls) {
     if (k.st) { cudaStreamSynchronize(k.st); cudaStreamDestroy(k.st); }
-    for (void* q : {(void*)k.d_ids, (void*)k.d_res, (void*)k.d_x, (void*)k.d_y, (void*)k.d_ws})
+    for (void* q : {(void*)k.d_ids, (void*)k.d_res, (void*)k.d_lim, (void*)k.d_ws})
       if (q) cudaFree(q);
   }
   for (void* q : {(void*)b->d_cases, (void*)b->d_maps, (void*)b->d_consts, (void*)b->d_prog, (void*)b->d_t0,

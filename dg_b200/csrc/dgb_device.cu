@@ -41,6 +41,8 @@ int upload_many_y_tables(const Consts& cs, int D, int p);
 // structured 2D grids, up to three mass fractions (dgb_tile.cu)
 int residual2d_cols(dgb_ctx* c, const StageArgs& a, int mode);
 void cols_setup(dgb_ctx* c);
+// hrl / m2l on structured 2D grids in one launch (dgb_lim.cu)
+int limit2d_out(dgb_ctx* c, const double* in, double* out);
 }  // namespace dgb
 #include "host/host.h"
 #include "ctx.h"
@@ -61,8 +63,6 @@ using namespace dgb;
 
 namespace {
 
-
-double fact(int n) { double f = 1; for (int i = 2; i <= n; ++i) f *= i; return f; }
 
 Consts make_consts(const Problem& P, int ld) {
   Consts c;
@@ -94,36 +94,6 @@ Consts make_consts(const Problem& P, int ld) {
   // element inverse mass matrix (element 0; uniform mesh) permuted to tensor order
   for (int t = 0; t < P.N_s; ++t)
     for (int u = 0; u < P.N_s; ++u) c.Minv[t][u] = P.Minv[(size_t)P.tensor_perm[u] * P.N_s + P.tensor_perm[t]];
-  // Lagrange -> scaled Taylor monomials: T = V^-1 phi on the (p+1) Gauss points
-  // (monovandermonde1d and Lag2Mono of main.cc:558-567, 1146-1157)
-  std::vector<double> V((size_t)n1 * n1), phi1((size_t)n1 * n1);
-  for (int g = 0; g < n1; ++g)
-    for (int j = 0; j < n1; ++j) {
-      V[g + (size_t)j * n1] = std::pow(xf[g], j) / fact(j);
-      phi1[g + (size_t)j * n1] = lagrange1d(xs, j, xf[g]);
-    }
-  invert(V, n1);
-  std::vector<double> T((size_t)n1 * n1, 0.0);
-  for (int m = 0; m < n1; ++m)
-    for (int i = 0; i < n1; ++i) {
-      double s = 0;
-      for (int g = 0; g < n1; ++g) s += V[m + (size_t)g * n1] * phi1[g + (size_t)i * n1];
-      T[m + (size_t)i * n1] = s;
-    }
-  std::vector<double> Ti = T;
-  invert(Ti, n1);
-  for (int m = 0; m < n1; ++m)
-    for (int i = 0; i < n1; ++i) { c.T[m][i] = T[m + (size_t)i * n1]; c.Tinv[i][m] = Ti[i + (size_t)m * n1]; }
-  // limiter integrals (integrate_monomial_derivative(_bounds), limiting_kernels.cu:1748-1775)
-  for (int k = 0; k < MAXN; ++k)
-    for (int n = 0; n < MAXN; ++n) {
-      const int num = n - k + 1;
-      if (num < 1) continue;
-      c.imd[k][n] = (num % 2) ? 2.0 / fact(num) : 0.0;
-      c.imdL[k][n] = (std::pow(-1.0, num) - std::pow(-3.0, num)) / fact(num);
-      c.imdR[k][n] = (std::pow(3.0, num) - std::pow(1.0, num)) / fact(num);
-    }
-  for (int k = 0; k < 8; ++k) c.ifact[k] = 1.0 / fact(k);
   const int D = P.D, NG = P.N_G;
   c.J = P.J[0];
   c.ixx = P.invJac[((size_t)0 * NG + 0) * D * D + 0];
@@ -317,27 +287,8 @@ int residual_dispatch(dgb_ctx* c, const StageArgs& a) {
   return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (dim, p, flux)");
 }
 
-constexpr int LIM_STRIP_H = 8;
-
-// fused x+y limiter on a row-major grid, out of place (in != out)
-template <int P, int METHOD>
-void launch_lim2d_fused(dgb_ctx* c, const double* in, double* out) {
-  ProfScope ps(c, KC_LIMITER);
-  const LimArgs la{c->ld, c->ne};
-  constexpr size_t smem = lim2d_fused_smem_bytes<P, METHOD>();
-  auto k = lim2d_fused_tile_kernel<P, METHOD, LIM_STRIP_H>;
-  allow_dynamic_smem(k, smem);
-  dim3 grid((c->nx + 29) / 30, (c->ny + LIM_STRIP_H - 1) / LIM_STRIP_H), block(32, P + 1);
-  k<<<grid, block, smem, c->st>>>(la, c->nx, c->ny, in, c->nbr, out, c->scal);
-}
-
 template <int P, int METHOD, int NY = 0>
 void launch_lim2d(dgb_ctx* c, double* U) {
-  if (NY == 0 && c->fused_lim) {
-    cudaMemcpyAsync(c->X, U, c->nstate * sizeof(double), cudaMemcpyDeviceToDevice, c->st);
-    launch_lim2d_fused<P, METHOD>(c, c->X, U);
-    return;
-  }
   ProfScope ps(c, KC_LIMITER);
   const LimArgs la{c->ld, c->ne};
   if (c->rowmajor) {
@@ -422,20 +373,6 @@ void launch_prl(dgb_ctx* c, double* U) {
   {
     ProfScope ps(c, KC_LIMITER);
     convert_state_kernel<D, NS, false><<<g, 256, 0, c->st>>>(la, U, c->scal);
-  }
-}
-
-// out-of-place fused limiting (row-major grids, hrl / m2l): in -> out, in != out
-int limit_to(dgb_ctx* c, const double* in, double* out) {
-  const int key = c->p * 10 + c->limiter;
-  switch (key) {
-    case 11: launch_lim2d_fused<1, 1>(c, in, out); return 0;
-    case 12: launch_lim2d_fused<1, 2>(c, in, out); return 0;
-    case 21: launch_lim2d_fused<2, 1>(c, in, out); return 0;
-    case 22: launch_lim2d_fused<2, 2>(c, in, out); return 0;
-    case 31: launch_lim2d_fused<3, 1>(c, in, out); return 0;
-    case 32: launch_lim2d_fused<3, 2>(c, in, out); return 0;
-    default: return set_error(DGB_ERR_UNSUPPORTED, "fused limiter: hrl / m2l, p = 1..3");
   }
 }
 
@@ -558,6 +495,10 @@ int limit_dispatch(dgb_ctx* c, double* U, bool rescore = true) {
       default: return set_error(DGB_ERR_UNSUPPORTED, "order outside 1..3");
     }
   }
+  if (c->lim_out) {
+    DGB_CUDA(cudaMemcpyAsync(c->X, U, c->nstate * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
+    return limit2d_out(c, c->X, U);
+  }
   const int key = c->p * 10 + c->limiter;
   switch (c->nmass) {
     case 0: break;
@@ -640,12 +581,12 @@ int ssp_stage(dgb_ctx* c, int s) {
   StageArgs a = stage_args(c);
   a.U = in[s];
   a.Ubase = c->A;
-  const bool fused = c->fused_lim && !c->ind_on;
-  a.out = fused ? c->X : out[s];  // the fused limiter then writes the stage output
+  const bool via = c->lim_out && !c->ind_on;
+  a.out = via ? c->X : out[s];  // the limiter then writes the stage output
   a.a = coef[s][0];
   a.b = coef[s][1];
   if (int rc = residual_dispatch<MODE_SSP>(c, a)) return rc;
-  if (fused) return limit_to(c, c->X, out[s]);
+  if (via) return limit2d_out(c, c->X, out[s]);
   return limit_dispatch(c, out[s], false);
 }
 
@@ -814,18 +755,39 @@ int step_ssprk3(dgb_ctx* c, bool cfl, bool score = true) {
   return 0;
 }
 
-// Stage k (0..3) of a classical RK4 step in the reference's form (rk.cc:155-209): A = U, B = Us,
-// C = Ustar.  The residual of the stage input (B for k = 0, C after) is accumulated into A; then
-// the next stage's input C = Us + beta DU is formed and limited, or after the last stage A is
-// limited.
-int rk4_stage(dgb_ctx* c, int k) {
+// The residual kernel forms the next RK4 stage input itself (rk4_stage); otherwise axpy_kernel does
+bool rk4_direct(const dgb_ctx* c) { return c->cols && c->form != DGB_FORM_MIXED && !c->tile_dmma; }
+
+// Stage k (0..3) of a classical RK4 step (rk.cc:155-209), limiter included.
+// rk4_direct: A = U^n = Us until the last stage, B the accumulator; stage k's residual writes
+// B (+)= gam DU and the next stage input Us + beta DU (the last stage: the accumulator), which the limiter
+// moves from X into C (A).  With no limiter, or one that works in place, the stage inputs alternate between
+// C and DU.  cur: the buffer that the next stage reads.
+// Otherwise A = U, B = Us (a copy), C = Ustar: the residual is accumulated into A and the next input
+// C = Us + beta DU is formed by a kernel of its own.
+int rk4_stage(dgb_ctx* c, int k, double** cur = nullptr) {
   const double beta[4] = {0.0, 0.5, 0.5, 1.0};
   const double gam[4] = {1.0 / 6.0, 2.0 / 6.0, 2.0 / 6.0, 1.0 / 6.0};
   StageArgs a = stage_args(c);
+  a.b = gam[k];
+  if (rk4_direct(c)) {
+    const bool via = c->lim_out && !c->ind_on;
+    double* in[4] = {c->A, c->C, via ? c->C : c->DU, c->C};
+    double* next = k == 3 ? c->A : in[k + 1];
+    a.U = in[k];
+    a.out = via ? c->X : next;
+    a.Us = k == 3 ? c->B : c->A;
+    a.beta_next = k == 3 ? gam[3] : beta[k + 1];
+    a.Uacc = k == 3 ? nullptr : c->B;
+    a.Ubase = k == 0 ? c->A : c->B;  // the accumulator before this stage
+    if (int rc = residual2d_cols(c, a, MODE_RK4)) return rc;
+    if (cur) *cur = next;
+    return via ? limit2d_out(c, c->X, next) : limit_dispatch(c, next, false);
+  }
+  if (cur) *cur = k < 3 ? c->C : c->A;
   a.U = k == 0 ? c->B : c->C;
   a.out = c->DU;
   a.Uacc = c->A;
-  a.b = gam[k];
   if (int rc = residual_dispatch<MODE_RK4>(c, a)) return rc;
   if (k == 3) return limit_dispatch(c, c->A, false);
   const int grid = (int)std::min<size_t>((c->nstate + 255) / 256, 148 * 16);
@@ -841,7 +803,7 @@ int step_rk4(dgb_ctx* c, bool cfl, bool score = true) {
   if (lim1d_direct(c)) return step1d_rk4(c, cfl);
   launch_dt(c, c->A, cfl);
   if (c->ind_on && score) launch_indicator(c, c->A);  // the learned indicator's band
-  cudaMemcpyAsync(c->B, c->A, c->nstate * sizeof(double), cudaMemcpyDeviceToDevice, c->st);
+  if (!rk4_direct(c)) cudaMemcpyAsync(c->B, c->A, c->nstate * sizeof(double), cudaMemcpyDeviceToDevice, c->st);
   for (int k = 0; k < 4; ++k)
     if (int rc = rk4_stage(c, k)) return rc;
   return 0;
@@ -967,9 +929,8 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
   c->tiled_full = c->tile_tma && P.nx % TILE_W == 0 && P.ny % tile_h_for(P.p, P.N_Y) == 0;
   // structured grids, up to three mass fractions: the residual of tile2d_cols.cuh on any extents
   c->cols = c->rowmajor && P.p <= 3 && P.N_Y <= 3;
-  // opt-in: measured slower than the two tiled passes on 512 x 256, p = 2 (64 vs 55 us per stage)
-  c->fused_lim = c->rowmajor && (P.limiter == DGB_LIM_HRL || P.limiter == DGB_LIM_M2L) &&
-                 std::getenv("DGB_FUSED_LIMITER") != nullptr && P.N_Y == 0;
+  // hrl / m2l: both limiter passes in one launch
+  c->lim_out = c->rowmajor && (P.limiter == DGB_LIM_HRL || P.limiter == DGB_LIM_M2L) && P.N_Y <= 3;
   c->nmass = P.N_Y;
   c->gamcons = P.gamcons;
   if (P.gamcons) {
@@ -985,7 +946,6 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
     else if (!P.thresholds.empty())
       why = "the troubled-cell sensors are built for GAMNCON";
     if (why) { delete c; return set_error(DGB_ERR_UNSUPPORTED, why); }
-    c->fused_lim = false;
   }
   if (P.N_Y > 10) { delete c; return set_error(DGB_ERR_UNSUPPORTED, "at most ten mass fractions"); }
   if (P.N_Y > 3) {
@@ -1065,7 +1025,7 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
   std::memset(&c->mapA, 0, sizeof(CUtensorMap));
   std::memset(&c->mapB, 0, sizeof(CUtensorMap));
   std::memset(&c->mapC, 0, sizeof(CUtensorMap));
-  for (CUtensorMap* m : {&c->colA, &c->colB, &c->colC}) std::memset(m, 0, sizeof(CUtensorMap));
+  for (CUtensorMap* m : {&c->colA, &c->colB, &c->colC, &c->colD}) std::memset(m, 0, sizeof(CUtensorMap));
   if (c->tile_tma) {
     // row starts must be 16-byte aligned for TMA: nx is even and ld a multiple of 64
     const int th = tile_h_for(P.p, P.N_Y);
@@ -1644,13 +1604,12 @@ extern "C" int dgb_step_stage(dgb_ctx* c, int k) {
       ProfScope ps(c, KC_DT);
       finish_dt_kernel<<<1, 1, 0, c->st>>>(c->scal, c->cs.cfl_scaled);
     }
-    if (c->slab_scheme == DGB_RK4)
+    if (c->slab_scheme == DGB_RK4 && !rk4_direct(c))
       DGB_CUDA(cudaMemcpyAsync(c->B, c->A, c->nstate * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
   }
   int rc;
   if (c->slab_scheme == DGB_RK4) {
-    rc = rk4_stage(c, k);
-    c->slab_cur = k < 3 ? c->C : c->A;
+    rc = rk4_stage(c, k, &c->slab_cur);
   } else {
     rc = ssp_stage(c, k);
     c->slab_cur = k == 0 ? c->B : (k == 1 ? c->C : c->A);

@@ -42,49 +42,7 @@ constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 void* g_scratch_dev[kMaxDevices] = {nullptr};
 
-double fact(int n) { double f = 1; for (int i = 2; i <= n; ++i) f *= i; return f; }
-
-// limiter tables of order P from the reference element alone (same construction as the context's)
-template <int P>
-LimTab<P> make_limtab() {
-  constexpr int n1 = P + 1;
-  LimTab<P> t;
-  std::memset(&t, 0, sizeof(t));
-  std::vector<double> xs(n1), xf, wf;
-  for (int i = 0; i < n1; ++i) xs[i] = -1.0 + 2.0 * i / P;
-  gauss_legendre(n1, xf, wf);
-  std::vector<double> V((size_t)n1 * n1), phi1((size_t)n1 * n1);
-  for (int g = 0; g < n1; ++g)
-    for (int j = 0; j < n1; ++j) {
-      V[g + (size_t)j * n1] = std::pow(xf[g], j) / fact(j);
-      phi1[g + (size_t)j * n1] = lagrange1d(xs, j, xf[g]);
-    }
-  invert(V, n1);
-  std::vector<double> T((size_t)n1 * n1, 0.0);
-  for (int m = 0; m < n1; ++m)
-    for (int i = 0; i < n1; ++i) {
-      double s = 0;
-      for (int g = 0; g < n1; ++g) s += V[m + (size_t)g * n1] * phi1[g + (size_t)i * n1];
-      T[m + (size_t)i * n1] = s;
-    }
-  std::vector<double> Ti = T;
-  invert(Ti, n1);
-  for (int m = 0; m < n1; ++m)
-    for (int i = 0; i < n1; ++i) { t.T[m][i] = T[m + (size_t)i * n1]; t.Tinv[i][m] = Ti[i + (size_t)m * n1]; }
-  for (int k = 0; k < n1; ++k)
-    for (int n = 0; n < n1; ++n) {
-      const int num = n - k + 1;
-      if (num < 1) continue;
-      t.imd[k][n] = (num % 2) ? 2.0 / fact(num) : 0.0;
-      t.imdL[k][n] = (std::pow(-1.0, num) - std::pow(-3.0, num)) / fact(num);
-      t.imdR[k][n] = (std::pow(3.0, num) - std::pow(1.0, num)) / fact(num);
-    }
-  for (int k = 0; k < P + 3; ++k) t.ifact[k] = 1.0 / fact(k);
-  return t;
-}
-
-// Once per device, with that device current: the device address of the scratch array and the
-// limiter tables of this translation unit's kernels.
+// Once per device, with that device current: the device address of the scratch array.
 int setup_device(int dev, void** scratch) {
   std::lock_guard<std::mutex> lock(g_setup_mutex);
   if (dev < 0 || dev >= kMaxDevices) return set_error(DGB_ERR_ARG, "device index out of range");
@@ -96,13 +54,6 @@ int setup_device(int dev, void** scratch) {
   cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
   if (e != cudaSuccess || !ptr)
     return set_error(DGB_ERR_CUDA, std::string("cudaGetSymbolAddress(scratch): ") + cudaGetErrorString(e));
-  const LimTab<1> t1 = make_limtab<1>();
-  const LimTab<2> t2 = make_limtab<2>();
-  const LimTab<3> t3 = make_limtab<3>();
-  if ((e = cudaMemcpyToSymbol(c_lim_p1, &t1, sizeof(t1))) != cudaSuccess ||
-      (e = cudaMemcpyToSymbol(c_lim_p2, &t2, sizeof(t2))) != cudaSuccess ||
-      (e = cudaMemcpyToSymbol(c_lim_p3, &t3, sizeof(t3))) != cudaSuccess)
-    return set_error(DGB_ERR_CUDA, std::string("limiter tables: ") + cudaGetErrorString(e));
   g_scratch_dev[dev] = ptr;
   *scratch = ptr;
   return DGB_OK;

@@ -64,24 +64,24 @@ ColTab make_col_tab(const Consts& cs, bool raw) {
 namespace {
 
 template <int P, int FLUX, int NY, bool GC>
-void launch_cols(dgb_ctx* c, const ColArgs& a, const CUtensorMap& map) {
+void launch_cols(dgb_ctx* c, const ColArgs& a, const ColTab& tab, const CUtensorMap& map) {
   using Dm = ColDims<P, NY, GC>;
   auto k = residual2d_cols_kernel<P, FLUX, NY, GC>;
   allow_dynamic_smem(k, Dm::smem_bytes);
   const dim3 grid((c->nx + Dm::TW - 1) / Dm::TW, (c->ny + Dm::TH - 1) / Dm::TH);
   ProfScope ps(c, KC_RESIDUAL);
-  launch_pdl(c, k, grid, dim3(Dm::NT), Dm::smem_bytes, a, map);
+  launch_pdl(c, k, grid, dim3(Dm::NT), Dm::smem_bytes, a, tab, map);
 }
 
 template <int NY, bool GC>
-int dispatch_cols(dgb_ctx* c, const ColArgs& a, const CUtensorMap& map) {
+int dispatch_cols(dgb_ctx* c, const ColArgs& a, const ColTab& tab, const CUtensorMap& map) {
   switch (c->p * 10 + c->flux) {
-    case 10: launch_cols<1, 0, NY, GC>(c, a, map); return 0;
-    case 12: launch_cols<1, 2, NY, GC>(c, a, map); return 0;
-    case 20: launch_cols<2, 0, NY, GC>(c, a, map); return 0;
-    case 22: launch_cols<2, 2, NY, GC>(c, a, map); return 0;
-    case 30: launch_cols<3, 0, NY, GC>(c, a, map); return 0;
-    case 32: launch_cols<3, 2, NY, GC>(c, a, map); return 0;
+    case 10: launch_cols<1, 0, NY, GC>(c, a, tab, map); return 0;
+    case 12: launch_cols<1, 2, NY, GC>(c, a, tab, map); return 0;
+    case 20: launch_cols<2, 0, NY, GC>(c, a, tab, map); return 0;
+    case 22: launch_cols<2, 2, NY, GC>(c, a, tab, map); return 0;
+    case 30: launch_cols<3, 0, NY, GC>(c, a, tab, map); return 0;
+    case 32: launch_cols<3, 2, NY, GC>(c, a, tab, map); return 0;
     default: return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (dim, p, flux)");
   }
 }
@@ -107,7 +107,8 @@ void cols_setup(dgb_ctx* c) {
   else if (c->p == 2) tile_of<2>(c, tw, th);
   else tile_of<3>(c, tw, th);
   c->cols_tma = c->nx % 2 == 0 && c->nx >= tw && c->ny >= th && encode_state_map(c, c->A, &c->colA, tw, th) &&
-                encode_state_map(c, c->B, &c->colB, tw, th) && encode_state_map(c, c->C, &c->colC, tw, th);
+                encode_state_map(c, c->B, &c->colB, tw, th) && encode_state_map(c, c->C, &c->colC, tw, th) &&
+                encode_state_map(c, c->DU, &c->colD, tw, th);
 }
 
 int residual2d_cols(dgb_ctx* c, const StageArgs& s, int mode) {
@@ -121,24 +122,31 @@ int residual2d_cols(dgb_ctx* c, const StageArgs& s, int mode) {
   a.polls = c->wait_polls;
   a.nx = c->nx; a.ny = c->ny; a.ld = c->ld;
   a.tma = c->cols_tma ? 1 : 0;
-  a.t = mode == MODE_RESIDUAL ? c->col_raw : c->col_step;
+  const ColTab& tab = mode == MODE_RESIDUAL ? c->col_raw : c->col_step;
   a.dt = mode == MODE_RESIDUAL ? 1.0 : s.dt_override;
   if (mode == MODE_SSP) {
     a.base = s.Ubase;
     a.k0 = s.a;
     a.k1 = a.k2 = s.b;
+  } else if (s.Us) {  // RK4 with the next stage input: out = Us + beta DU, accumulator = Ubase + b DU
+    a.base = s.Us;
+    a.k0 = 1.0;
+    a.k2 = s.beta_next;
+    a.base2 = s.Ubase;
+    a.out2 = s.Uacc;
+    a.c2 = s.b;
   } else {
     a.k2 = 1.0;
     a.base2 = a.out2 = s.Uacc;
     a.c2 = s.b;
   }
-  const CUtensorMap& map = s.U == c->B ? c->colB : s.U == c->C ? c->colC : c->colA;
-  if (c->gamcons) return dispatch_cols<0, true>(c, a, map);
+  const CUtensorMap& map = s.U == c->B ? c->colB : s.U == c->C ? c->colC : s.U == c->DU ? c->colD : c->colA;
+  if (c->gamcons) return dispatch_cols<0, true>(c, a, tab, map);
   switch (c->nmass) {
-    case 0: return dispatch_cols<0, false>(c, a, map);
-    case 1: return dispatch_cols<1, false>(c, a, map);
-    case 2: return dispatch_cols<2, false>(c, a, map);
-    case 3: return dispatch_cols<3, false>(c, a, map);
+    case 0: return dispatch_cols<0, false>(c, a, tab, map);
+    case 1: return dispatch_cols<1, false>(c, a, tab, map);
+    case 2: return dispatch_cols<2, false>(c, a, tab, map);
+    case 3: return dispatch_cols<3, false>(c, a, tab, map);
     default: return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (dim, p, flux)");
   }
 }
