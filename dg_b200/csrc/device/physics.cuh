@@ -56,20 +56,20 @@ template <int FLUX, int NY = 0, bool GC = false>
 __device__ __forceinline__ void riemann1d(double rhoL, double rhoR, double vxL, double vxR, double EtL, double EtR,
                                           double alphaL, double alphaR, double nx, double* F, double& nc,
                                           const double* YL = nullptr, const double* YR = nullptr) {
-  // the reference's divisions as correctly rounded reciprocals (shorter dependency chains; within
-  // an ulp or two of the quotients)
-  const double irL = __drcp_rn(rhoL), irR = __drcp_rn(rhoR);
+  // the reference's divisions as reciprocals (shorter dependency chains; within an ulp or two of the
+  // quotients)
+  const double irL = rcp(rhoL), irR = rcp(rhoR);
   if (GC) {
     alphaL = alphaL * irL;
     alphaR = alphaR * irR;
   }
-  const double gm1L = __drcp_rn(alphaL), gm1R = __drcp_rn(alphaR);  // gamma - 1 = 1/alpha
+  const double gm1L = rcp(alphaL), gm1R = rcp(alphaR);  // gamma - 1 = 1/alpha
   const double gammaL = 1.0 + gm1L;
   const double gammaR = 1.0 + gm1R;
   const double pL = gm1L * (EtL - 0.5 * rhoL * vxL * vxL);
   const double pR = gm1R * (EtR - 0.5 * rhoR * vxR * vxR);
-  const double aL = sqrt(gammaL * pL * irL);
-  const double aR = sqrt(gammaR * pR * irR);
+  const double aL = root(gammaL * pL * irL);
+  const double aR = root(gammaR * pR * irR);
   if (FLUX == FLUX_RUS) {
     const double maxvap = fmax(fabs(vxL) + aL, fabs(vxR) + aR);
     F[0] = 0.5 * ((rhoL * vxL + rhoR * vxR) * nx - maxvap * (rhoR - rhoL));
@@ -93,7 +93,7 @@ __device__ __forceinline__ void riemann1d(double rhoL, double rhoR, double vxL, 
     const double SR = fmax(vxL * nx + aL, vxR * nx + aR);
     const double vnc = -0.5 * (vxL * nx + vxR * nx) * (alphaL - alphaR);
     const double vncabs = -0.5 * fabs(vxL * nx + vxR * nx) * (alphaL - alphaR);
-    const double iw = __drcp_rn(fabs(SR - SL));
+    const double iw = rcp(fabs(SR - SL));
     auto fhll = [iw](double UL, double SLv, double FL, double UR, double SRv, double FR) {
       return (SRv * FL - SLv * FR + SLv * SRv * (UR - UL)) * iw;
     };
@@ -126,23 +126,23 @@ __device__ __forceinline__ void riemann1d(double rhoL, double rhoR, double vxL, 
     }
     nc = GC ? 0.0 : -0.5 * vnc;
   } else {
-    const double RT = sqrt(rhoR * irL);
+    const double RT = root(rhoR * irL);
     const double rho = RT * rhoL;
-    const double i1 = __drcp_rn(1 + RT);
+    const double i1 = rcp(1 + RT);
     const double v = (vxL + RT * vxR) * i1;
     const double HL = (EtL + pL) * irL;
     const double HR = (EtR + pR) * irR;
     const double H = (HL + RT * HR) * i1;
     const double alpha = (alphaL + RT * alphaR) * i1;
-    const double gm1 = __drcp_rn(alpha);  // gamma - 1
-    const double a = sqrt(gm1 * (H - 0.5 * v * v));
+    const double gm1 = rcp(alpha);  // gamma - 1
+    const double a = root(gm1 * (H - 0.5 * v * v));
     const double iL = pL * alphaL;
     const double iR = pR * alphaR;
-    const double sL = sqrt(rhoL), sR = sqrt(rhoR);
-    const double i = (sL * iL + sR * iR) * __drcp_rn(sL + sR);
+    const double sL = root(rhoL), sR = root(rhoR);
+    const double i = (sL * iL + sR * iR) * rcp(sL + sR);
     const double Dp = gm1 * gm1 * (alpha * (iR - iL) - i * (alphaR - alphaL));
     const double p = gm1 * i;
-    const double ia2 = __drcp_rn(a * a);
+    const double ia2 = rcp(a * a);
     const double dV0 = (Dp - rho * a * (vxR - vxL)) * (0.5 * ia2);
     const double dV1 = (rhoR - rhoL) - Dp * ia2;
     const double dV2 = (Dp + rho * a * (vxR - vxL)) * (0.5 * ia2);
@@ -313,20 +313,20 @@ template <int FLUX, int NY = 0, bool GC = false>
 __device__ __forceinline__ void riemann2d_rcp(const double* L, const double* R, double nx, double ny, double* F,
                                               double& nc) {
   const double rhoL = L[0], rhoR = R[0];
-  const double irL = __drcp_rn(rhoL), irR = __drcp_rn(rhoR);
+  const double irL = rcp(rhoL), irR = rcp(rhoR);
   const double vxL = L[1] * irL, vyL = L[2] * irL, vxR = R[1] * irR, vyR = R[2] * irR;
   const double EtL = L[3], EtR = R[3];
   // GAMCONS: divided by rho on entry; the Rusanov solver's right alpha is the left one divided
   // twice by rhoL (see riemann2d)
   const double alphaL = GC ? L[4] * irL : L[4];
   const double alphaR = GC ? (FLUX == FLUX_ROE ? R[4] * irR : alphaL * irL) : R[4];
-  const double gm1L = __drcp_rn(alphaL), gm1R = __drcp_rn(alphaR);
+  const double gm1L = rcp(alphaL), gm1R = rcp(alphaR);
   const double vnL = vxL * nx + vyL * ny;
   const double vnR = vxR * nx + vyR * ny;
   const double pL = gm1L * (EtL - 0.5 * rhoL * (vxL * vxL + vyL * vyL));
   const double pR = gm1R * (EtR - 0.5 * rhoR * (vxR * vxR + vyR * vyR));
-  const double aL = sqrt((1.0 + gm1L) * pL * irL);
-  const double aR = sqrt((1.0 + gm1R) * pR * irR);
+  const double aL = root((1.0 + gm1L) * pL * irL);
+  const double aR = root((1.0 + gm1R) * pR * irR);
   const double HL = (EtL + pL) * irL;
   const double HR = (EtR + pR) * irR;
   if (FLUX == FLUX_ROE) {
@@ -334,18 +334,18 @@ __device__ __forceinline__ void riemann2d_rcp(const double* L, const double* R, 
     const double vtL = vxL * tx + vyL * ty;
     const double vtR = vxR * tx + vyR * ty;
     const double iL = pL * alphaL, iR = pR * alphaR;
-    const double RT = sqrt(rhoR * irL);
+    const double RT = root(rhoR * irL);
     const double rho = RT * rhoL;
-    const double i1 = __drcp_rn(1 + RT);
+    const double i1 = rcp(1 + RT);
     const double vx = (vxL + RT * vxR) * i1;
     const double vy = (vyL + RT * vyR) * i1;
     const double vn = vx * nx + vy * ny;
     const double vt = vx * tx + vy * ty;
     const double H = (HL + RT * HR) * i1;
     const double alpha = (alphaL + RT * alphaR) * i1;
-    const double gm1 = __drcp_rn(alpha);
-    const double a = sqrt(gm1 * (H - 0.5 * (vx * vx + vy * vy)));
-    const double ia = __drcp_rn(a);
+    const double gm1 = rcp(alpha);
+    const double a = root(gm1 * (H - 0.5 * (vx * vx + vy * vy)));
+    const double ia = rcp(a);
     const double i = (iL + RT * iR) * i1;
     const double p = gm1 * i;
     const double drho = rhoR - rhoL;

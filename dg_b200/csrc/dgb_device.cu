@@ -637,9 +637,9 @@ void launch_res_lim1d(dgb_ctx* c, const StageArgs& a, int mode, const double* ac
   const int grid = (c->ne + RL1D_B - 1) / RL1D_B;
   ProfScope ps(c, KC_RESIDUAL);
   if (mode == MODE_SSP)
-    res_lim1d_chain_kernel<P, FLUX, MODE_SSP, METHOD><<<grid, 96, 0, c->st>>>(c->cs, a, acc_in, acc_out, last, lim_out);
+    launch_pdl(c, res_lim1d_chain_kernel<P, FLUX, MODE_SSP, METHOD>, dim3(grid), dim3(96), 0, c->cs, a, acc_in, acc_out, last, lim_out);
   else
-    res_lim1d_chain_kernel<P, FLUX, MODE_RK4, METHOD><<<grid, 96, 0, c->st>>>(c->cs, a, acc_in, acc_out, last, lim_out);
+    launch_pdl(c, res_lim1d_chain_kernel<P, FLUX, MODE_RK4, METHOD>, dim3(grid), dim3(96), 0, c->cs, a, acc_in, acc_out, last, lim_out);
 }
 
 int res_lim1d(dgb_ctx* c, const StageArgs& a, int mode, const double* acc_in, double* acc_out, int last,
