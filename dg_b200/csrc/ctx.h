@@ -76,6 +76,7 @@ struct dgb_ctx {
   dgb::Consts cs;
   double *A = nullptr, *B = nullptr, *C = nullptr, *DU = nullptr, *X = nullptr, *ref = nullptr;
   int *nbr = nullptr, *perm = nullptr;
+  unsigned long long perm_bits = 0;  // perm, 4 bits per node
   // sensor-gated limiters (hri, m2i, pri, p0i): sensor work arrays and flags
   bool gated = false, has_sensors = false;
   int sm_count = 148;           // multiprocessors of the device

@@ -809,8 +809,31 @@ int step_rk4(dgb_ctx* c, bool cfl, bool score = true) {
   return 0;
 }
 
+template <int NF, int NS>
+void launch_convert(dgb_ctx* c, bool to_int, const double* src, double* dst, int n) {
+  const int grid = (n + CONV_FE - 1) / CONV_FE;
+  if (to_int) convert_fixed_kernel<true, NF, NS><<<grid, 256, 0, c->st>>>(src, dst, c->perm_bits, n, c->ld);
+  else convert_fixed_kernel<false, NF, NS><<<grid, 256, 0, c->st>>>(src, dst, c->perm_bits, n, c->ld);
+}
+
 // layout conversions of elements [e0, e0 + n) (reference <-> internal) on the context's stream
 int convert_range(dgb_ctx* c, bool to_int, const double* src, double* dst, int e0, int n) {
+  if (n > 0 && c->nmass <= 1) {  // the field counts of nearly every problem; the general kernel takes the others
+    const size_t per = (size_t)c->nf * c->ns;
+    const double* s = src + (to_int ? e0 * per : e0);
+    double* d = dst + (to_int ? e0 : e0 * per);
+#define CV(D, NS)                                                     \
+  case D * 100 + NS:                                                  \
+    if (c->nmass) launch_convert<D + 4, NS>(c, to_int, s, d, n);      \
+    else launch_convert<D + 3, NS>(c, to_int, s, d, n);               \
+    DGB_CUDA(cudaGetLastError());                                     \
+    return 0;
+    switch (c->D * 100 + c->ns) {
+      CV(1, 2) CV(1, 3) CV(1, 4) CV(2, 4) CV(2, 9) CV(2, 16)
+      default: break;
+    }
+#undef CV
+  }
   const size_t per = (size_t)c->nf * c->ns, smem = convert_smem_bytes(c->nf, c->ns);
   const int grid = std::max(1, std::min((n + CONV_EB - 1) / CONV_EB, c->sm_count * 16));
   if (to_int)
@@ -985,6 +1008,7 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
   cudaMemcpy(c->nbr, nb.data(), nb.size() * sizeof(int), cudaMemcpyHostToDevice);
   if ((e = cudaMalloc(&c->perm, c->ns * sizeof(int))) != cudaSuccess) return fail(e, "perm");
   cudaMemcpy(c->perm, P.tensor_perm.data(), c->ns * sizeof(int), cudaMemcpyHostToDevice);
+  for (int t = 0; t < c->ns; ++t) c->perm_bits |= (unsigned long long)P.tensor_perm[t] << (4 * t);
   c->gated = P.limiter == DGB_LIM_HRI || P.limiter == DGB_LIM_M2I || P.limiter == DGB_LIM_PRI || P.limiter == DGB_LIM_P0I;
   c->has_sensors = c->gated || !P.thresholds.empty();
   if (c->has_sensors) {
