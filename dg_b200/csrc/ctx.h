@@ -61,12 +61,12 @@ struct dgb_ctx {
   bool tiled_full = false;  // ... with TMA and extents that are tile multiples (no leftover strips)
   int* left = nullptr;    // the elements outside the full tiles (generic residual kernel), nleft of them
   int nleft = 0;
-  int form = DGB_FORM_FP64;  // arithmetic of the residual: plain FP64 or mixed FP32/FP64
+  int form = DGB_FORM_FP64;  // the form asked for (both run the FP64 residual, dgb_set_form)
   long long wait_polls = 1ll << 22;  // poll budget of the residual kernels' first wait per tile copy
   bool rowmajor = false;  // structured row-major grid: tiled limiter passes
   bool chain1d = false;   // 1D elements in chain order: fused residual + limiter stages
   bool lim_out = false;   // row-major grid, hrl / m2l: both limiter passes in one launch, out of place
-  CUtensorMap mapA, mapB, mapC;  // TMA descriptors of the state buffers (mixed, DMMA and many-Y tiles)
+  CUtensorMap mapA, mapB, mapC;  // TMA descriptors of the state buffers (DMMA and many-Y tiles)
   // structured 2D grids: the residual with one thread per (element, quadrature column)
   bool cols = false, cols_tma = false;
   CUtensorMap colA, colB, colC, colD;  // its TMA descriptors
@@ -81,7 +81,6 @@ struct dgb_ctx {
   bool gated = false, has_sensors = false;
   int sm_count = 148;           // multiprocessors of the device
   bool ind_on = false;          // learned indicator gates the limiter (dgb_set_indicator)
-  bool mixed_ct = false;        // mixed form: the compressed-tile kernel (else the TMA-tile kernel)
   bool pdl = true;              // programmatic dependent launches (kernels that wait in pdl_wait)
   bool tile_dmma = false;       // p = 2 FP64 stages: the DMMA residual (else the scalar tiled kernel)
   bool ind_tc = true;           // scoring GEMMs on tcgen05 (else the mma.sync kernel)

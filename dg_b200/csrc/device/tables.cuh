@@ -1,5 +1,5 @@
 // Reference-element tables in __constant__ memory: the tensor-product tables of the 2D tiled residual
-// kernels (c_tab2_p*, FP32 copies c_tab2f_p*), and in global memory the lane tables of the p = 2 DMMA
+// kernels (c_tab2_p*), and in global memory the lane tables of the p = 2 DMMA
 // residual (g_dmma_tab2).  Those symbols are static, one copy per translation unit (each .cu file
 // is its own device module), so every .cu file that launches kernels reading them calls
 // upload_tables from its own code; the function is static for the same reason.
@@ -14,7 +14,6 @@
 #include "common.cuh"
 #include "tile2d.cuh"
 #include "tile2d_dmma.cuh"
-#include "tile2d_mixed.cuh"
 
 namespace dgb {
 
@@ -52,28 +51,6 @@ static Tab2<P> make_tab2(const Consts& c) {
   invert(M, N1);
   for (int i = 0; i < N1; ++i)
     for (int j = 0; j < N1; ++j) T.M1i[i][j] = M[i + (size_t)j * N1];
-  return T;
-}
-
-template <int P>
-static Tab2f<P> make_tab2f(const Tab2<P>& d) {
-  Tab2f<P> T;
-  std::memset(&T, 0, sizeof(T));
-  constexpr int N1 = Tab2<P>::N1, NG1 = Tab2<P>::NG1, NS = Tab2<P>::NS, NG = Tab2<P>::NG;
-  for (int g = 0; g < NG; ++g) {
-    T.W[g] = (float)d.W[g];
-    for (int t = 0; t < NS; ++t) {
-      T.dPx[g][t] = (float)d.dPx[g][t];
-      T.dPy[g][t] = (float)d.dPy[g][t];
-      T.Phi[g][t] = (float)d.Phi[g][t];
-    }
-  }
-  for (int i = 0; i < N1; ++i) {
-    T.wf[i] = (float)d.wf[i];
-    for (int j = 0; j < N1; ++j) { T.Bf[i][j] = (float)d.Bf[i][j]; T.M1i[i][j] = (float)d.M1i[i][j]; }
-  }
-  for (int g = 0; g < NG1; ++g)
-    for (int i = 0; i < N1; ++i) { T.B1[g][i] = (float)d.B1[g][i]; T.D1[g][i] = (float)d.D1[g][i]; }
   return T;
 }
 
@@ -139,15 +116,11 @@ static int upload_tables(const Consts& cs, int D, int p) {
     cudaError_t et = cudaSuccess;
     if (p == 1) {
       auto t = make_tab2<1>(cs);
-      auto tf = make_tab2f<1>(t);
       et = cudaMemcpyToSymbol(c_tab2_p1, &t, sizeof(t));
-      if (et == cudaSuccess) et = cudaMemcpyToSymbol(c_tab2f_p1, &tf, sizeof(tf));
     }
     if (p == 2) {
       auto t = make_tab2<2>(cs);
-      auto tf = make_tab2f<2>(t);
       et = cudaMemcpyToSymbol(c_tab2_p2, &t, sizeof(t));
-      if (et == cudaSuccess) et = cudaMemcpyToSymbol(c_tab2f_p2, &tf, sizeof(tf));
       if (et == cudaSuccess) {
         const DmmaTab2 td = make_dmma_tab2(t);
         et = cudaMemcpyToSymbol(g_dmma_tab2, &td, sizeof(td));
@@ -155,9 +128,7 @@ static int upload_tables(const Consts& cs, int D, int p) {
     }
     if (p == 3) {
       auto t = make_tab2<3>(cs);
-      auto tf = make_tab2f<3>(t);
       et = cudaMemcpyToSymbol(c_tab2_p3, &t, sizeof(t));
-      if (et == cudaSuccess) et = cudaMemcpyToSymbol(c_tab2f_p3, &tf, sizeof(tf));
     }
     if (et != cudaSuccess) return set_error(5, std::string("constant tables: ") + cudaGetErrorString(et));
   }

@@ -24,7 +24,6 @@
 #include "device/tile2d_dmma.cuh"
 #include "device/limiter2d_tile.cuh"
 #include "device/limiter_gated.cuh"
-#include "device/tile2d_mixed.cuh"
 #include "device/learned.cuh"
 #include "device/learned_tc.cuh"
 #include "device/tables.cuh"
@@ -146,30 +145,6 @@ void launch_res1d(dgb_ctx* c, const StageArgs& a) {
   residual1d_kernel<P, FLUX, MODE, NY, GC><<<grid, 128, 0, c->st>>>(c->cs, a);
 }
 
-template <int P, int FLUX, int MODE>
-void launch_tile2d_mixed(dgb_ctx* c, const StageArgs& s) {
-  constexpr int TH = tile_h_for(P);
-  if (c->mixed_ct) {
-    constexpr size_t smem = TileDimsMixedCT<P, TILE_W, TH>::smem_bytes;
-    auto k = residual2d_tile_mixed_ct_kernel<P, FLUX, MODE, TILE_W, TH>;
-    allow_dynamic_smem(k, smem);
-    const TileArgs a = tile_args(c, s);
-    dim3 grid(c->nx / TILE_W, c->ny / TH);
-    ProfScope ps(c, KC_RESIDUAL);
-    launch_pdl(c, k, grid, dim3(TILE_W * TH), smem, a);
-    return;
-  }
-  constexpr size_t smem = TileDimsMixed<P, TILE_W, TH>::smem_bytes;
-  auto k = residual2d_tile_mixed_kernel<P, FLUX, MODE, TILE_W, TH>;
-  allow_dynamic_smem(k, smem);
-  const TileArgs a = tile_args(c, s);
-  const CUtensorMap& mb = MODE == MODE_SSP ? map_of(c, s.Ubase)
-                          : MODE == MODE_RK4 && s.Uacc ? map_of(c, s.Uacc) : map_of(c, s.U);
-  dim3 grid(c->nx / TILE_W, c->ny / TH);
-  ProfScope ps(c, KC_RESIDUAL);
-  launch_pdl(c, k, grid, dim3(TILE_W * TH), smem, a, map_of(c, s.U), mb);
-}
-
 // p = 2 FP64 stage on the FP64 tensor cores (tile2d_dmma.cuh): same tiles and tensor map
 template <int FLUX, int MODE>
 void launch_tile2d_dmma(dgb_ctx* c, const StageArgs& s) {
@@ -222,19 +197,6 @@ int residual_ny(dgb_ctx* c, const StageArgs& a) {
 
 template <int MODE>
 int residual_dispatch(dgb_ctx* c, const StageArgs& a) {
-  if (c->tile_tma && c->form == DGB_FORM_MIXED) {
-    // mixed full tiles; the strips outside them (if any) in the plain FP64 form
-    const int key = c->p * 10 + c->flux;
-    switch (key) {
-      case 10: launch_tile2d_mixed<1, 0, MODE>(c, a); if (c->nleft) launch_res2d<1, 0, MODE>(c, a, c->left, c->nleft); return 0;
-      case 12: launch_tile2d_mixed<1, 2, MODE>(c, a); if (c->nleft) launch_res2d<1, 2, MODE>(c, a, c->left, c->nleft); return 0;
-      case 20: launch_tile2d_mixed<2, 0, MODE>(c, a); if (c->nleft) launch_res2d<2, 0, MODE>(c, a, c->left, c->nleft); return 0;
-      case 22: launch_tile2d_mixed<2, 2, MODE>(c, a); if (c->nleft) launch_res2d<2, 2, MODE>(c, a, c->left, c->nleft); return 0;
-      case 30: launch_tile2d_mixed<3, 0, MODE>(c, a); if (c->nleft) launch_res2d<3, 0, MODE>(c, a, c->left, c->nleft); return 0;
-      case 32: launch_tile2d_mixed<3, 2, MODE>(c, a); if (c->nleft) launch_res2d<3, 2, MODE>(c, a, c->left, c->nleft); return 0;
-      default: return set_error(DGB_ERR_UNSUPPORTED, "mixed form: p = 1..3 with Rusanov or Roe");
-    }
-  }
   if (c->cols) {
     if constexpr (MODE != MODE_RESIDUAL) {
       if (c->tile_tma && c->tile_dmma && c->p == 2 && c->nmass == 0 && !c->gamcons) {
@@ -756,7 +718,7 @@ int step_ssprk3(dgb_ctx* c, bool cfl, bool score = true) {
 }
 
 // The residual kernel forms the next RK4 stage input itself (rk4_stage); otherwise axpy_kernel does
-bool rk4_direct(const dgb_ctx* c) { return c->cols && c->form != DGB_FORM_MIXED && !c->tile_dmma; }
+bool rk4_direct(const dgb_ctx* c) { return c->cols && !c->tile_dmma; }
 
 // Stage k (0..3) of a classical RK4 step (rk.cc:155-209), limiter included.
 // rk4_direct: A = U^n = Us until the last stage, B the accumulator; stage k's residual writes
@@ -920,11 +882,6 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
     // programmatic dependent launches of the 2D step's kernels unless DGB_PDL=0
     const char* pk = std::getenv("DGB_PDL");
     c->pdl = !(pk && std::string(pk) == "0");
-    // mixed-form tiles: the compressed shared tile (FP64 anchors + FP32 deviations, plain loads)
-    // at p = 3, the TMA-loaded FP64 tile at p = 1, 2 (the faster of the two at each order);
-    // DGB_MIXED_TILE=ct / tma selects one for every order
-    const char* mk = std::getenv("DGB_MIXED_TILE");
-    c->mixed_ct = mk ? std::string(mk) == "ct" : P.p == 3;
     // element chunks of dgb_advance_host's copies (DGB_HOST_CHUNKS, 1 .. kHostChunks; 16 measured best)
     const char* hk = std::getenv("DGB_HOST_CHUNKS");
     c->host_chunks = hk ? std::max(1, std::min(kHostChunks, std::atoi(hk))) : kHostChunksDefault;

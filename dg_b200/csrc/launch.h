@@ -32,7 +32,7 @@ void launch_pdl(dgb_ctx* c, void (*k)(KArgs...), dim3 grid, dim3 block, size_t s
 
 constexpr int TILE_W = 32, TILE_H = 4;
 // p = 3 tiles are two element rows high: the per-element register state (80 nodal values per
-// field set) and the shared tile then leave room for two (FP64) or three (mixed) CTAs per SM
+// field set) and the shared tile then leave room for two CTAs per SM
 // (and with more than three mass fractions, whose fields would not leave room for a 32 x 4 tile)
 constexpr int tile_h_for(int p, int ny = 0) { return p == 3 || ny > 3 ? 2 : TILE_H; }
 

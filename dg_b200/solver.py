@@ -177,7 +177,7 @@ class DGSolver:
 
     def set_form(self, form: str) -> None:
         """Arithmetic of the residual: "fp64" (plain, the parity form) or "mixed" (FP32 contractions
-        and fluxes on FP64 anchors, FP64 pressure recovery and stage update)."""
+        and fluxes allowed; the FP64 kernels are the faster ones here, so both run them)."""
         F.check(F.lib().dgb_set_form(self._h, F.FORM[form]))
 
     def set_wait_limit(self, polls: int = 1 << 22) -> None:

@@ -62,9 +62,10 @@ enum dgb_limiter {
   DGB_LIM_M2I = 4, DGB_LIM_PRL = 5, DGB_LIM_PRI = 6, DGB_LIM_P0I = 7
 };
 
-/* Arithmetic of the residual kernels.  FP64: plain double precision (the parity form).  MIXED:
- * basis contractions, Rusanov flux and lift in FP32 on deviations from a per-element FP64 anchor;
- * state, pressure recovery, Roe solver and stage update in FP64 (structured 2D grids, p <= 3). */
+/* Arithmetic of the residual kernels.  FP64: plain double precision (the parity form).  MIXED: the
+ * caller allows FP32 contractions and fluxes on FP64 anchors (structured 2D grids, p <= 3).  It is a
+ * permission: on sm_100a, whose FP64 rate is half its FP32 rate, the FP64 kernels are the faster ones
+ * at every order, so both forms run them and give the same result. */
 enum dgb_form { DGB_FORM_FP64 = 0, DGB_FORM_MIXED = 1 };
 
 /* Gamma model (GAMM of the reference Makefile): GAMNCON carries alpha = 1/(gamma-1) with a
