@@ -109,7 +109,8 @@ __global__ void __launch_bounds__(ColDims<P, 0, false, TW, TH>::NT, ColDims<P, 0
       *sa = a;
     }
     __syncthreads();
-    cols_body<P, FLUX, 0, false, TW, TH, true>(*sa, tab, &maps[item.x].m[stage], item.y, item.z, smraw, phase);
+    cols_body<P, FLUX, 0, false, TW, TH, true>(*sa, tab, &maps[item.x].m[stage], &maps[item.x].m[0], item.y, item.z,
+                                              smraw, phase);
   }
 }
 

@@ -63,7 +63,10 @@ struct ColArgs {
 //   p = 2, 512 x 256     84 us; 16 x 4: 54, 16 x 2: 52, 32 x 2: 55, 8 x 4: 56, 8 x 8: 59
 //   p = 3, 1024 x 512   888 us; 16 x 2: 450, 8 x 4: 437, 16 x 4: 479, 32 x 2: 493, 8 x 8: 491   (Roe)
 // Small tiles pay more faces per element (16 x 4: 2.31, 16 x 2: 2.56) but put more CTAs on an SM, whose
-// loads, barriers and compute phases then overlap.
+// loads, barriers and compute phases then overlap.  With the step's status read beside the tile's copy instead of
+// before it, the stage base prefetched into L2 and 32-bit offsets: 50 us (p = 2), 421 us (p = 3).  There it
+// spends 10 us on the volume terms, 10 on the faces, 13 on the update and 20 on loads, in p = 2's 50 (the
+// copy rate would take 22 for stages 2 and 3); starting the CTAs of an SM staggered changes nothing.
 template <int P>
 constexpr int col_tw() { return P == 3 ? 8 : 16; }
 template <int P>
@@ -161,8 +164,9 @@ __device__ __forceinline__ void riemann_n2(const double* L, const double* R, dou
 // early return is taken by the whole CTA, after its last barrier.
 // SCALED: the tables carry no metric, a.sx and a.sy do (tiles of problems of many mesh widths).
 template <int P, int FLUX, int NY, bool GC, int TW, int TH, bool SCALED>
-__device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, const CUtensorMap* mapU, int tx0, int ty0,
-                                          unsigned char* smraw, uint32_t& phase) {
+__device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, const CUtensorMap* mapU,
+                                          const CUtensorMap* mapBase, int tx0, int ty0, unsigned char* smraw,
+                                          uint32_t& phase) {
   static_assert(!(GC && NY > 0), "GAMCONS with mass fractions is not built");
   using Dm = ColDims<P, NY, GC, TW, TH>;
   constexpr int N1 = Dm::N1, NS = Dm::NS, NF = Dm::NF, NFL = Dm::NFL, NG1 = Dm::NG1;
@@ -178,6 +182,8 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
   const int tw = min(TW, nx - tx0), th = min(TH, a.ny - ty0);
 
   // ---------------- the tile and the neighbours' face nodes ----------------
+  // (the step's status is read along with them: its latency before the copy would be every CTA's)
+  const unsigned failed = tid == 0 && a.scal ? a.scal->flags : 0u;
   // a TMA copy must land on a 128-byte shared boundary and start on a 16-byte global column;
   // otherwise record the fault and skip the copy
   const bool tma_ok = a.tma && (smem_u32(Us) & 127u) == 0 && ((tx0 * 8) & 15) == 0;
@@ -185,6 +191,7 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
     if (tma_ok) {
       mbar_arrive_expect_tx(bar, (uint32_t)Dm::tile_bytes);
       tma_load_3d(Us, mapU, tx0, ty0, 0, bar);
+      if (a.k0 != 0.0 && mapBase) tma_prefetch_3d(mapBase, tx0, ty0, 0);
     } else if (a.tma) {
       atomicOr(a.errflag, (unsigned)FLAG_TIMEOUT);
     }
@@ -195,12 +202,13 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
       Us[k] = x < tw && y < th ? __ldg(a.U + (size_t)q * ld + (size_t)(ty0 + y) * nx + tx0 + x) : 0.0;
     }
   }
-  // edge slot s of the tile (left, right, bottom, top): the neighbour across it -- the next element
-  // of the row or column, or at the domain's edges what the neighbour table says -- and its face
-  // nodes.  A thread keeps one slot and takes every NHG-th (field, node) of it, all loads in flight.
-  constexpr int NHG = NT / Dm::NEDGE, NHL = (NF * N1 + NHG - 1) / NHG;
-  if (tid < NHG * Dm::NEDGE) {
-    const int s = tid % Dm::NEDGE, r0 = tid / Dm::NEDGE;
+  // edge slot s of the tile (left, right, bottom, top): the neighbour across it -- the next element of the row or
+  // column, or at the domain's edges what the neighbour table says -- and its face nodes.  A thread takes
+  // node j of every field of one slot, all loads in flight.  (Offsets into a state are 32-bit counts of
+  // values: 2^32 of them in each of a context's seven buffers is more than the GPU's memory.)
+  const unsigned plane = ld;
+  for (int k = tid; k < N1 * Dm::NEDGE; k += NT) {
+    const int s = k % Dm::NEDGE, j = k / Dm::NEDGE;
     const bool side = s < 2 * TH;
     const int hi = side ? s / TH : (s - 2 * TH) / TW, q = side ? s % TH : (s - 2 * TH) % TW;
     if (q < (side ? th : tw)) {
@@ -209,17 +217,13 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
       const bool border = side ? (hi ? x == nx - 1 : x == 0) : (hi ? y == a.ny - 1 : y == 0);
       const int step = side ? 1 : nx;
       const int nb = border ? __ldg(a.nbr + (size_t)(side ? hi : 2 + hi) * ld + eo) : (hi ? eo + step : eo - step);
-      const int n0 = side ? (hi ? 0 : P) : (hi ? 0 : N1 * P), dj = side ? N1 : 1;
-      double v[NHL];
+      const unsigned o = ((side ? (hi ? 0 : P) : (hi ? 0 : N1 * P)) + (side ? N1 : 1) * j) * plane + (unsigned)nb;
+      double v[NF];
 #pragma unroll
-      for (int k = 0; k < NHL; ++k) {
-        const int r = r0 + k * NHG, j = r % N1, f = r / N1;
-        v[k] = r < NF * N1 && nb >= 0 ? __ldg(a.U + (size_t)(f * NS + n0 + dj * j) * ld + nb) : 0.0;
-      }
-      if (r0 == 0) codes[s] = nb;
+      for (int f = 0; f < NF; ++f) v[f] = nb >= 0 ? __ldg(a.U + (o + f * NS * plane)) : 0.0;
+      if (j == 0) codes[s] = nb;
 #pragma unroll
-      for (int k = 0; k < NHL; ++k)
-        if (r0 + k * NHG < NF * N1) HS[(r0 + k * NHG) * Dm::NEDGE + s] = v[k];
+      for (int f = 0; f < NF; ++f) HS[(f * N1 + j) * Dm::NEDGE + s] = v[f];
     }
   }
   if (tid == 0) {
@@ -228,7 +232,7 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
       atomicOr(a.errflag, (unsigned)FLAG_TIMEOUT);
       mbar_wait(bar, phase & 1);
     }
-    *s_ok = ok ? 1 : 0;
+    *s_ok = ok && !failed ? 1 : 0;
   }
   if (tma_ok) ++phase;
   __syncthreads();
@@ -408,14 +412,14 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
   constexpr int NIT = (NF * N1 + NG1 - 1) / NG1;
   const int el = tid % NE, tx = el % TW, ty = el / TW, r0 = tid / NE;
   const bool own = tx < tw && ty < th;
-  const size_t g0 = (size_t)(N1 * r0) * ld + (size_t)(ty0 + ty) * nx + tx0 + tx;
+  const unsigned g0 = N1 * r0 * plane + (unsigned)((ty0 + ty) * nx + tx0 + tx);
   double v0[NIT][N1], v2[NIT][N1];
 #pragma unroll
   for (int q = 0; q < NIT; ++q) {
     const bool on = own && r0 + q * NG1 < NF * N1;
 #pragma unroll
     for (int ix = 0; ix < N1; ++ix) {
-      const size_t gi = g0 + (size_t)(q * NG1 * N1 + ix) * ld;
+      const unsigned gi = g0 + (q * NG1 * N1 + ix) * plane;
       v0[q][ix] = on && a.k0 != 0.0 ? a.base[gi] : 0.0;
       v2[q][ix] = on && a.out2 ? a.base2[gi] : 0.0;
     }
@@ -465,7 +469,7 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
       const double* us = Us + N1 * r * NE + el;
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) {
-        const size_t gi = g0 + (size_t)(q * NG1 * N1 + ix) * ld;
+        const unsigned gi = g0 + (q * NG1 * N1 + ix) * plane;
         const double du = dt * s[ix];
         double o = a.k2 * du;
         if (a.k1 != 0.0) o = a.k1 * us[ix * NE] + o;
@@ -480,7 +484,7 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
 template <int P, int FLUX, int NY, bool GC>
 __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ctas)
     residual2d_cols_kernel(const __grid_constant__ ColArgs a, const __grid_constant__ ColTab tab,
-                           const __grid_constant__ CUtensorMap mapU) {
+                           const __grid_constant__ CUtensorMap mapU, const __grid_constant__ CUtensorMap mapBase) {
   constexpr int TW = col_tw<P>(), TH = col_th<P>();
   extern __shared__ __align__(128) unsigned char smraw[];
   if (threadIdx.x == 0) {
@@ -488,9 +492,8 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
     fence_mbar_init();
   }
   pdl_wait();
-  if (a.scal && a.scal->flags) return;
   uint32_t phase = 0;
-  cols_body<P, FLUX, NY, GC, TW, TH, false>(a, tab, &mapU, blockIdx.x * TW, blockIdx.y * TH, smraw, phase);
+  cols_body<P, FLUX, NY, GC, TW, TH, false>(a, tab, &mapU, &mapBase, blockIdx.x * TW, blockIdx.y * TH, smraw, phase);
   // (at the end: with the trigger at the start the next launch's CTAs, waiting, hold the shared memory that this
   // one's last wave could use: 240 -> 256 us per 512 x 256 step)
   pdl_trigger();

@@ -64,24 +64,24 @@ ColTab make_col_tab(const Consts& cs, bool raw) {
 namespace {
 
 template <int P, int FLUX, int NY, bool GC>
-void launch_cols(dgb_ctx* c, const ColArgs& a, const ColTab& tab, const CUtensorMap& map) {
+void launch_cols(dgb_ctx* c, const ColArgs& a, const ColTab& tab, const CUtensorMap& map, const CUtensorMap& base) {
   using Dm = ColDims<P, NY, GC>;
   auto k = residual2d_cols_kernel<P, FLUX, NY, GC>;
   allow_dynamic_smem(k, Dm::smem_bytes);
   const dim3 grid((c->nx + Dm::TW - 1) / Dm::TW, (c->ny + Dm::TH - 1) / Dm::TH);
   ProfScope ps(c, KC_RESIDUAL);
-  launch_pdl(c, k, grid, dim3(Dm::NT), Dm::smem_bytes, a, tab, map);
+  launch_pdl(c, k, grid, dim3(Dm::NT), Dm::smem_bytes, a, tab, map, base);
 }
 
 template <int NY, bool GC>
-int dispatch_cols(dgb_ctx* c, const ColArgs& a, const ColTab& tab, const CUtensorMap& map) {
+int dispatch_cols(dgb_ctx* c, const ColArgs& a, const ColTab& tab, const CUtensorMap& map, const CUtensorMap& base) {
   switch (c->p * 10 + c->flux) {
-    case 10: launch_cols<1, 0, NY, GC>(c, a, tab, map); return 0;
-    case 12: launch_cols<1, 2, NY, GC>(c, a, tab, map); return 0;
-    case 20: launch_cols<2, 0, NY, GC>(c, a, tab, map); return 0;
-    case 22: launch_cols<2, 2, NY, GC>(c, a, tab, map); return 0;
-    case 30: launch_cols<3, 0, NY, GC>(c, a, tab, map); return 0;
-    case 32: launch_cols<3, 2, NY, GC>(c, a, tab, map); return 0;
+    case 10: launch_cols<1, 0, NY, GC>(c, a, tab, map, base); return 0;
+    case 12: launch_cols<1, 2, NY, GC>(c, a, tab, map, base); return 0;
+    case 20: launch_cols<2, 0, NY, GC>(c, a, tab, map, base); return 0;
+    case 22: launch_cols<2, 2, NY, GC>(c, a, tab, map, base); return 0;
+    case 30: launch_cols<3, 0, NY, GC>(c, a, tab, map, base); return 0;
+    case 32: launch_cols<3, 2, NY, GC>(c, a, tab, map, base); return 0;
     default: return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (dim, p, flux)");
   }
 }
@@ -140,13 +140,17 @@ int residual2d_cols(dgb_ctx* c, const StageArgs& s, int mode) {
     a.base2 = a.out2 = s.Uacc;
     a.c2 = s.b;
   }
-  const CUtensorMap& map = s.U == c->B ? c->colB : s.U == c->C ? c->colC : s.U == c->DU ? c->colD : c->colA;
-  if (c->gamcons) return dispatch_cols<0, true>(c, a, tab, map);
+  auto map_of_buf = [&](const double* q) -> const CUtensorMap& {
+    return q == c->B ? c->colB : q == c->C ? c->colC : q == c->DU ? c->colD : c->colA;
+  };
+  const CUtensorMap& map = map_of_buf(s.U);
+  const CUtensorMap& base = map_of_buf(a.base);  // read only when k0 != 0
+  if (c->gamcons) return dispatch_cols<0, true>(c, a, tab, map, base);
   switch (c->nmass) {
-    case 0: return dispatch_cols<0, false>(c, a, tab, map);
-    case 1: return dispatch_cols<1, false>(c, a, tab, map);
-    case 2: return dispatch_cols<2, false>(c, a, tab, map);
-    case 3: return dispatch_cols<3, false>(c, a, tab, map);
+    case 0: return dispatch_cols<0, false>(c, a, tab, map, base);
+    case 1: return dispatch_cols<1, false>(c, a, tab, map, base);
+    case 2: return dispatch_cols<2, false>(c, a, tab, map, base);
+    case 3: return dispatch_cols<3, false>(c, a, tab, map, base);
     default: return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (dim, p, flux)");
   }
 }
