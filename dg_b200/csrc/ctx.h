@@ -40,6 +40,12 @@ inline cudaError_t allow_dynamic_smem(K* kernel, size_t bytes) {
 // element chunks of the host-resident time loop's copies (dgb_advance_host): at most, by default
 constexpr int kHostChunks = 16, kHostChunksDefault = 16;
 
+// Steps in one captured graph of a long run (dgb_advance).  Between two graphs the GPU waits some 1.8 us, within
+// one it does not: 5 steps per graph take the 1000-element tube's 25 steps from 645 to 601 us, 20 steps of a
+// 64 x 32 grid from 873 to 830 (8 per graph: the same).  Capturing it costs some 150 us, so a context does it
+// once it has run kMultiAfter steps.
+constexpr int kMultiSteps = 5, kMultiAfter = 100;
+
 enum { KC_RESIDUAL = 0, KC_LIMITER = 1, KC_DT = 2, KC_INDICATOR = 3, KC_OTHER = 4, KC_N = 5 };
 }
 
@@ -110,6 +116,9 @@ struct dgb_ctx {
   // captured steps per [scheme: SSP-RK3, RK4][CFL step][the step scores the learned indicator]
   cudaGraphExec_t graphs[2][2][2] = {};
   long long graph_launches[2][2][2] = {};
+  // kMultiSteps steps in one graph per [scheme][CFL step], for runs of many steps
+  cudaGraphExec_t multi[2][2] = {};
+  long long steps_run = 0;  // by dgb_advance
   int ind_every = 1;       // steps between scorings of the learned indicator (1: every step)
   long long ind_step = 0;  // steps taken since the last dgb_set_state / dgb_set_indicator
   // destroys the captured steps (their kernel arguments or launch sequence changed)
@@ -127,6 +136,9 @@ struct dgb_ctx {
       for (auto& b : a)
         for (auto& g : b)
           if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    for (auto& a : multi)
+      for (auto& g : a)
+        if (g) { cudaGraphExecDestroy(g); g = nullptr; }
   }
   // profiling (per kernel class)
   bool prof = false;

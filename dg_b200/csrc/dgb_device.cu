@@ -1394,6 +1394,22 @@ int ensure_step_graphs(dgb_ctx* c, int scheme, bool cfl) {
   return DGB_OK;
 }
 
+// captures kMultiSteps steps in a row (no learned indicator, whose scoring pattern varies)
+int ensure_multi_graph(dgb_ctx* c, int scheme, bool cfl) {
+  cudaGraphExec_t& x = c->multi[scheme == DGB_RK4 ? 1 : 0][cfl ? 1 : 0];
+  if (x) return DGB_OK;
+  cudaGraph_t g;
+  DGB_CUDA(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
+  int rc = 0;
+  for (int s = 0; s < kMultiSteps && !rc; ++s) rc = scheme == DGB_RK4 ? step_rk4(c, cfl) : step_ssprk3(c, cfl);
+  const cudaError_t ec = cudaStreamEndCapture(c->st, &g);
+  if (rc) { if (ec == cudaSuccess) cudaGraphDestroy(g); return rc; }
+  DGB_CUDA(ec);
+  DGB_CUDA(cudaGraphInstantiate(&x, g, 0));
+  cudaGraphDestroy(g);
+  return DGB_OK;
+}
+
 // the step's status from the device scalars (read after the step's last kernel)
 int step_status(dgb_ctx* c, double* time) {
   if (int rc = read_scalars(c)) return rc;
@@ -1436,9 +1452,20 @@ extern "C" int dgb_advance(dgb_ctx* c, int scheme, int nsteps, double dt, double
   } else {
     if (nsteps > 0)
       if (int rc = ensure_step_graphs(c, scheme, cfl)) return rc;
+    const bool many = nsteps >= 2 * kMultiSteps && !c->ind_on && (c->multi[si][mi] || c->steps_run + nsteps > kMultiAfter);
+    c->steps_run += nsteps;
+    if (many)
+      if (int rc = ensure_multi_graph(c, scheme, cfl)) return rc;
     DGB_CUDA(cudaEventRecord(c->e0, c->st));
     long long launches = 0;
     for (int s = 0; s < nsteps; ++s) {
+      if (many && nsteps - s >= kMultiSteps) {
+        DGB_CUDA(cudaGraphLaunch(c->multi[si][mi], c->st));
+        launches += kMultiSteps * c->graph_launches[si][mi][0];
+        c->ind_step += kMultiSteps;
+        s += kMultiSteps - 1;
+        continue;
+      }
       const int k = scores() ? 0 : 1;
       DGB_CUDA(cudaGraphLaunch(c->graphs[si][mi][k], c->st));
       launches += c->graph_launches[si][mi][k];
