@@ -16,6 +16,7 @@
 #include "device/limiter_gated.cuh"
 #include "device/sensor.h"
 #include "device/tile2d_cols.cuh"
+#include "device/tile2d_ordered.cuh"
 
 namespace dgb {
 // Dynamic shared memory above 48 KB is opted into per kernel, and cudaFuncSetAttribute acts on the
@@ -67,7 +68,7 @@ struct dgb_ctx {
   bool tiled_full = false;  // ... with TMA and extents that are tile multiples (no leftover strips)
   int* left = nullptr;    // the elements outside the full tiles (generic residual kernel), nleft of them
   int nleft = 0;
-  int form = DGB_FORM_FP64;  // the form asked for (both run the FP64 residual, dgb_set_form)
+  int form = DGB_FORM_FP64;  // the form asked for (both run FP64 kernels; ordered() is the difference)
   long long wait_polls = 1ll << 22;  // poll budget of the residual kernels' first wait per tile copy
   bool rowmajor = false;  // structured row-major grid: tiled limiter passes
   bool chain1d = false;   // 1D elements in chain order: fused residual + limiter stages
@@ -77,6 +78,9 @@ struct dgb_ctx {
   bool cols = false, cols_tma = false;
   CUtensorMap colA, colB, colC, colD;  // its TMA descriptors
   dgb::ColTab col_step, col_raw;   // its tables: stage update, residual
+  // cubic elements under a limiter, FP64 form: stages whose sums keep their order (tile2d_ordered.cuh)
+  dgb::OrdTab ord_tab;
+  bool ordered() const { return cols && p == 3 && limiter != DGB_LIM_NONE && form == DGB_FORM_FP64; }
   double hx = 0, hy = 0;
   size_t nstate = 0;
   dgb::Consts cs;

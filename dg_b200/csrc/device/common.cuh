@@ -9,6 +9,7 @@
 // boundary only.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 namespace dgb {
 
@@ -163,5 +164,117 @@ __device__ __forceinline__ void hr_energy(const double* plim, const double* alim
     E[3] = (plim[3] * alim[0] + (3.0 * (plim[2] * alim[1] + plim[1] * alim[2]) + plim[0] * alim[3])) + Kmono[3];
   E[0] = P >= 2 ? mean - E[P >= 2 ? 2 : 0] * (1.0 / 6.0) : mean;
 }
+
+// The same as a form that the kernels are written over.  NM moments of a slice are what its neighbours need.
+template <int P>
+struct HrSums {
+  static constexpr int NM = P;
+  static __device__ __forceinline__ void moments(const double* v, double* D) { hr_moments<P>(v, D); }
+  static __device__ __forceinline__ void limit(const double* DL, const double* DC, const double* DR, double* lim) {
+    hr_limit<P>(DL, DC, DR, lim);
+  }
+  static __device__ __forceinline__ void flat(const double* DC, double* lim) { hr_flat<P>(DC, lim); }
+  static __device__ __forceinline__ void mono(const double* v, double* a) { to_mono<P>(v, a); }
+  static __device__ __forceinline__ void lag(const double* a, double* v) { to_lag<P>(a, v); }
+  // E rebuilt from the limited coefficients of p and alpha, the limited kinetic energy K and the slice
+  // vE of E before (nodal values, and out)
+  static __device__ __forceinline__ void energy(const double* plim, const double* alim, const double* K, const double* vE,
+                                                double* E) {
+    double Km[P + 1], D[P], El[P + 1];
+    to_mono<P>(K, Km);
+    hr_moments<P>(vE, D);
+    hr_energy<P>(plim, alim, Km, hr_mean<P>(D), El);
+    to_lag<P>(El, E);
+  }
+  static __device__ __forceinline__ double rcp(double x);  // physics.cuh
+};
+
+// Cubic elements in 2D.  There the limited scheme itself multiplies a difference of rounding by 10 to 15 per
+// step, up to some 4e-8 of the state (with any flux; p <= 2, 1D and the unlimited scheme leave it at 1e-15), so
+// after five steps a run repeats an earlier one to 1e-11 only if every sum keeps its terms, their order and
+// their rounding.  This form does: a slice's Taylor coefficients are formed with a transform that carries
+// the rounding of its numerical inversion (within 1e-14 of 9/16, 27/16, 9/8, 27/8, ...),
+// reciprocals are correctly rounded, and the kernels apply the operations in the order written here.
+// (in constant memory: as literals they would be moved into registers)
+static __constant__ double c_hr3_T[4][4] = {
+    {-0x1.000000000000cp-4, 0x1.2p-1, 0x1.2p-1, -0x1.ffffffffffff6p-5},
+    {0x1.0000000000006p-4, -0x1.afffffffffffdp+0, 0x1.b000000000002p+0, -0x1.fffffffffffebp-5},
+    {0x1.2000000000001p+0, -0x1.2000000000001p+0, -0x1.2000000000003p+0, 0x1.1ffffffffffffp+0},
+    {-0x1.bp+1, 0x1.43ffffffffffep+3, -0x1.4400000000002p+3, 0x1.afffffffffffep+1}};
+static __constant__ double c_hr3_Ti[4][4] = {
+    {0x1.0000000000007p+0, -0x1.0000000000001p+0, 0x1.ffffffffffffep-2, -0x1.5555555555557p-3},
+    {0x1.0000000000003p+0, -0x1.5555555555559p-2, 0x1.c71c71c71c72p-5, -0x1.948b0fcd6ea03p-8},
+    {0x1.ffffffffffffcp-1, 0x1.5555555555553p-2, 0x1.c71c71c71c71cp-5, 0x1.948b0fcd6e9bdp-8},
+    {0x1.0000000000001p+0, 0x1.0000000000001p+0, 0x1p-1, 0x1.5555555555556p-3}};
+struct HrTab3 {
+  static constexpr int NM = 3;
+  static __device__ __forceinline__ void mono(const double* v, double* a) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      double s = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s += c_hr3_T[m][i] * v[i];
+      a[m] = s;
+    }
+  }
+  static __device__ __forceinline__ void lag(const double* a, double* v) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      double s = 0;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) s += c_hr3_Ti[i][m] * a[m];
+      v[i] = s;
+    }
+  }
+  // D: the integrals of u, u' and u'' over the cell (integrate_monomial_derivative(_bounds),
+  // limiting_kernels.cu:1748-1775), from the Taylor coefficients
+  static __device__ __forceinline__ void means(const double* a, double* D) {
+    D[0] = __fma_rn(a[2], 2.0 / 6.0, 2.0 * a[0]);
+    D[1] = __fma_rn(a[3], 2.0 / 6.0, 2.0 * a[1]);
+    D[2] = 2.0 * a[2];
+  }
+  static __device__ __forceinline__ void moments(const double* v, double* D) {
+    double a[4];
+    mono(v, a);
+    means(a, D);
+  }
+  static __device__ __forceinline__ void limit(const double* DL, const double* DC, const double* DR, double* lim) {
+    // a neighbour's mean less that of the limited higher terms over its interval, [-3, -1] or [1, 3]
+    auto side = [](double d, double r) { return 0.5 * __dsub_rn(d, r); };
+    auto pick = [](double l, double c, double r) { return minmod2(0.5 * __dsub_rn(c, l), 0.5 * __dsub_rn(r, c)); };
+    lim[3] = pick(0.5 * DL[2], 0.5 * DC[2], 0.5 * DR[2]);
+    const double r3 = __dmul_rn(lim[3], 26.0 / 6.0);
+    lim[2] = pick(side(DL[1], r3), side(DC[1], __dmul_rn(lim[3], 2.0 / 6.0)), side(DR[1], r3));
+    const double r2 = __dmul_rn(lim[2], 26.0 / 6.0);
+    lim[0] = side(DC[0], __dmul_rn(lim[2], 2.0 / 6.0));
+    lim[1] = pick(side(DL[0], __fma_rn(lim[3], -80.0 / 24.0, r2)), lim[0], side(DR[0], __fma_rn(lim[3], 80.0 / 24.0, r2)));
+  }
+  static __device__ __forceinline__ void flat(const double* DC, double* lim) {
+    lim[0] = 0.5 * DC[0];
+    lim[1] = lim[2] = lim[3] = 0.0;
+  }
+  static __device__ __forceinline__ void energy(const double* plim, const double* alim, const double* K, const double* vE,
+                                                double* E) {
+    constexpr double binom[4][4] = {{1, 0, 0, 0}, {1, 1, 0, 0}, {1, 2, 1, 0}, {1, 3, 3, 1}};
+    double Km[4], Em[4], El[4], re[4];
+    mono(K, Km);
+    mono(vE, Em);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      double s = 0;
+#pragma unroll
+      for (int k = 0; k <= m; ++k) s += binom[m][k] * plim[m - k] * alim[k];
+      re[m] = s;
+    }
+#pragma unroll
+    for (int m = 1; m < 4; ++m) El[m] = re[m] + Km[m];
+    El[0] = Em[0] - (1.0 / 6.0) * (El[2] - Em[2]);
+    lag(El, E);
+  }
+  static __device__ __forceinline__ double rcp(double x) { return __drcp_rn(x); }
+};
+// the form of the 2D limiters
+template <int P>
+using Hr2 = std::conditional_t<P == 3, HrTab3, HrSums<P>>;
 
 }  // namespace dgb

@@ -24,11 +24,12 @@ namespace dgb {
 // Modes of the residual kernels.
 enum { MODE_RESIDUAL = 0,  // out = S + F + Q                         (dg_solver)
        MODE_SSP = 1,       // out = a*Ubase + b*(U + dt*Minv*(S+F+Q))  (SSP-RK stage)
-       MODE_RK4 = 2 };     // out = dt*Minv*(S+F+Q); Uacc += b*out     (Lsolver + axpy)
+       MODE_RK4 = 2 };     // du = dt*Minv*(S+F+Q); out = du, Uacc += b*du  (Lsolver + axpy), or in 2D with
+                           // Us: out = Us + beta_next*du, Uacc = Ubase + b*du (Uacc null: not formed)
 
 struct StageArgs {
   const double* __restrict__ U;      // stage input (internal layout)
-  const double* __restrict__ Ubase;  // SSP: U^n
+  const double* __restrict__ Ubase;  // SSP: U^n; RK4 with Us: the accumulator before
   double* __restrict__ out;
   double* __restrict__ Uacc;         // RK4 accumulator (may be null)
   double* __restrict__ Unext;        // RK4 (1D): the next stage input Us + beta_next * DU, or null
@@ -167,9 +168,9 @@ __global__ void __launch_bounds__(NT) residual2d_kernel(const Consts cin, const 
       // the volume terms of the tiled kernel's point_terms: the conservative fluxes of the NFL
       // fields (mass fractions rho Y_k u, physics.cu:293-298; GAMCONS alpha flux rho u/(gamma-1),
       // physics.cu:253-281) and, under GAMNCON, the alpha source
-      const double rho = ug[0], irho = phys::rcp(rho);
+      const double rho = ug[0], irho = __drcp_rn(rho);
       const double uu = ug[1] * irho, vv = ug[2] * irho, Et = ug[3];
-      const double gm1 = GC ? rho * phys::rcp(ug[4]) : phys::rcp(ug[4]);
+      const double gm1 = GC ? rho * __drcp_rn(ug[4]) : __drcp_rn(ug[4]);
       const double p = gm1 * (Et - 0.5 * rho * (uu * uu + vv * vv));
       const double W = c.wq[g / NG1] * c.wq[g % NG1];
       const double wx = W * (c.J * c.ixx), wy = W * (c.J * c.iyy);
@@ -189,8 +190,8 @@ __global__ void __launch_bounds__(NT) residual2d_kernel(const Consts cin, const 
       continue;
     }
     // physics.cu:248-257 with correctly rounded reciprocals in place of its divisions
-    const double rho = ug[0], ir = phys::rcp(rho), u = ug[1] * ir, v = ug[2] * ir, Et = ug[3];
-    const double p = phys::rcp(ug[4]) * (Et - 0.5 * rho * (u * u + v * v));
+    const double rho = ug[0], ir = __drcp_rn(rho), u = ug[1] * ir, v = ug[2] * ir, Et = ug[3];
+    const double p = __drcp_rn(ug[4]) * (Et - 0.5 * rho * (u * u + v * v));
     const double W = c.wq[g / NG1] * c.wq[g % NG1];
     const double cx = W * (c.ixx * c.J), cy = W * (c.iyy * c.J);
     G[(0 * NG + g) * TE + el] = cx * (rho * u);
@@ -306,6 +307,10 @@ __global__ void __launch_bounds__(NT) residual2d_kernel(const Consts cin, const 
     if (MODE == MODE_SSP) {
       const double base = a.a != 0.0 ? a.a * __ldg(a.Ubase + gi) : 0.0;
       a.out[gi] = base + a.b * (Us[i] + du);
+    } else if (a.Us) {
+      const double acc = a.Uacc ? a.Ubase[gi] : 0.0;
+      a.out[gi] = a.Us[gi] + a.beta_next * du;
+      if (a.Uacc) a.Uacc[gi] = acc + a.b * du;
     } else {
       a.out[gi] = du;
       if (a.Uacc) a.Uacc[gi] += a.b * du;
@@ -456,34 +461,23 @@ __global__ void __launch_bounds__(128) residual1d_kernel(const __grid_constant__
 // Limit one slice given the nodal values of the centre and (when interior) both neighbours.
 // phys: 0 interior, 2/3 flatten (zero-gradient / reflective), 4 leave unchanged, 5 copy
 // (reflective wall-normal momentum under HR limiting, hrl1D limiting_kernels.cu:291-302).
-template <int P>
+// HR: the form of the reconstruction (HrSums, Hr2).
+template <class HR, int P>
 __device__ __forceinline__ void limit_slice(int phys, const double* vL, const double* vC, const double* vR,
                                             double* lim) {
-  double DC[P];
+  double DC[HR::NM];
   if (phys == 0) {
-    double DL[P], DR[P];
-    hr_moments<P>(vC, DC);
-    hr_moments<P>(vL, DL);
-    hr_moments<P>(vR, DR);
-    hr_limit<P>(DL, DC, DR, lim);
+    double DL[HR::NM], DR[HR::NM];
+    HR::moments(vC, DC);
+    HR::moments(vL, DL);
+    HR::moments(vR, DR);
+    HR::limit(DL, DC, DR, lim);
   } else if (phys == 2 || phys == 3) {
-    hr_moments<P>(vC, DC);
-    hr_flat<P>(DC, lim);
+    HR::moments(vC, DC);
+    HR::flat(DC, lim);
   } else {
-    to_mono<P>(vC, lim);
+    HR::mono(vC, lim);
   }
-}
-
-// E rebuilt from the limited coefficients of p and alpha, the limited kinetic energy K and the slice
-// vE of E before (nodal values, and out)
-template <int P>
-__device__ __forceinline__ void rebuild_energy(const double* plim, const double* alim, const double* K, const double* vE,
-                                               double* E) {
-  double Km[P + 1], D[P], El[P + 1];
-  to_mono<P>(K, Km);
-  hr_moments<P>(vE, D);
-  hr_energy<P>(plim, alim, Km, hr_mean<P>(D), El);
-  to_lag<P>(El, E);
 }
 
 __device__ __forceinline__ int boundary_code(int left, int right) {
@@ -505,6 +499,7 @@ __global__ void __launch_bounds__(128) lim2d_xpass_kernel(const LimArgs la, cons
                                                           const int* __restrict__ nbr, double* __restrict__ X,
                                                           const DevScalars* __restrict__ scal) {
   constexpr int N1 = P + 1, NS = N1 * N1;
+  using HR = Hr2<P>;
   if (scal && scal->flags) return;
   const int ld = la.ld, e = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y;
   if (e >= la.n_elem) return;
@@ -525,8 +520,8 @@ __global__ void __launch_bounds__(128) lim2d_xpass_kernel(const LimArgs la, cons
     for (int f = 0; f < 5; ++f) {
       double lim[N1], out[N1];
       const int ph = (phys == 3 && f == 1) ? 5 : phys;
-      limit_slice<P>(ph, v[0][f], v[1][f], v[2][f], lim);
-      to_lag<P>(lim, out);
+      limit_slice<HR, P>(ph, v[0][f], v[1][f], v[2][f], lim);
+      HR::lag(lim, out);
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) X[(size_t)(f * NS + ix + N1 * iy) * ld + e] = out[ix];
     }
@@ -539,25 +534,25 @@ __global__ void __launch_bounds__(128) lim2d_xpass_kernel(const LimArgs la, cons
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) {
         const double ru = v[s][1][ix], rv = v[s][2][ix], E = v[s][3][ix];
-        const double gm1 = phys::rcp(v[s][4][ix]);
-        pr[s][ix] = gm1 * (E - 0.5 * (ru * ru + rv * rv) * phys::rcp(v[s][0][ix]));
+        const double gm1 = HR::rcp(v[s][4][ix]);
+        pr[s][ix] = gm1 * (E - 0.5 * (ru * ru + rv * rv) * HR::rcp(v[s][0][ix]));
       }
     }
     double lr[N1], lu[N1], lv[N1], la_[N1], lp[N1];
-    limit_slice<P>(phys, v[0][0], v[1][0], v[2][0], lr);
-    limit_slice<P>(phys, v[0][1], v[1][1], v[2][1], lu);
-    limit_slice<P>(phys, v[0][2], v[1][2], v[2][2], lv);
-    limit_slice<P>(phys, v[0][4], v[1][4], v[2][4], la_);
-    limit_slice<P>(phys, pr[0], pr[1], pr[2], lp);
+    limit_slice<HR, P>(phys, v[0][0], v[1][0], v[2][0], lr);
+    limit_slice<HR, P>(phys, v[0][1], v[1][1], v[2][1], lu);
+    limit_slice<HR, P>(phys, v[0][2], v[1][2], v[2][2], lv);
+    limit_slice<HR, P>(phys, v[0][4], v[1][4], v[2][4], la_);
+    limit_slice<HR, P>(phys, pr[0], pr[1], pr[2], lp);
     double r_[N1], u_[N1], v_[N1], a_[N1], p_[N1], K[N1], E_[N1];
-    to_lag<P>(lr, r_);
-    to_lag<P>(lu, u_);
-    to_lag<P>(lv, v_);
-    to_lag<P>(la_, a_);
-    to_lag<P>(lp, p_);
+    HR::lag(lr, r_);
+    HR::lag(lu, u_);
+    HR::lag(lv, v_);
+    HR::lag(la_, a_);
+    HR::lag(lp, p_);
 #pragma unroll
-    for (int ix = 0; ix < N1; ++ix) K[ix] = 0.5 * (u_[ix] * u_[ix] + v_[ix] * v_[ix]) * phys::rcp(r_[ix]);
-    rebuild_energy<P>(lp, la_, K, v[1][3], E_);
+    for (int ix = 0; ix < N1; ++ix) K[ix] = 0.5 * (u_[ix] * u_[ix] + v_[ix] * v_[ix]) * HR::rcp(r_[ix]);
+    HR::energy(lp, la_, K, v[1][3], E_);
 #pragma unroll
     for (int ix = 0; ix < N1; ++ix) {
       const size_t o = (size_t)(ix + N1 * iy) * ld + e;
@@ -578,6 +573,7 @@ __global__ void __launch_bounds__(128) lim2d_ypass_kernel(const LimArgs la, cons
                                                           const int* __restrict__ nbr, double* __restrict__ Uout,
                                                           const DevScalars* __restrict__ scal) {
   constexpr int N1 = P + 1, NS = N1 * N1;
+  using HR = Hr2<P>;
   constexpr int NQ = METHOD == 1 ? 5 : 6;
   if (scal && scal->flags) return;
   const int ld = la.ld, e = blockIdx.x * blockDim.x + threadIdx.x, ix = blockIdx.y;
@@ -599,26 +595,26 @@ __global__ void __launch_bounds__(128) lim2d_ypass_kernel(const LimArgs la, cons
     for (int f = 0; f < 5; ++f) {
       double lim[N1], out[N1];
       const int ph = (phys == 3 && f == 2) ? 5 : phys;
-      limit_slice<P>(ph, v[0][f], v[1][f], v[2][f], lim);
-      to_lag<P>(lim, out);
+      limit_slice<HR, P>(ph, v[0][f], v[1][f], v[2][f], lim);
+      HR::lag(lim, out);
 #pragma unroll
       for (int iy = 0; iy < N1; ++iy) Uout[(size_t)(f * NS + ix + N1 * iy) * ld + e] = out[iy];
     }
   } else {
     double lr[N1], lu[N1], lv[N1], la_[N1], lp[N1];
-    limit_slice<P>(phys, v[0][0], v[1][0], v[2][0], lr);
-    limit_slice<P>(phys, v[0][1], v[1][1], v[2][1], lu);
-    limit_slice<P>(phys, v[0][2], v[1][2], v[2][2], lv);
-    limit_slice<P>(phys, v[0][3], v[1][3], v[2][3], la_);
-    limit_slice<P>(phys, v[0][4], v[1][4], v[2][4], lp);
+    limit_slice<HR, P>(phys, v[0][0], v[1][0], v[2][0], lr);
+    limit_slice<HR, P>(phys, v[0][1], v[1][1], v[2][1], lu);
+    limit_slice<HR, P>(phys, v[0][2], v[1][2], v[2][2], lv);
+    limit_slice<HR, P>(phys, v[0][3], v[1][3], v[2][3], la_);
+    limit_slice<HR, P>(phys, v[0][4], v[1][4], v[2][4], lp);
     double r_[N1], u_[N1], v_[N1], a_[N1], K[N1], E_[N1];
-    to_lag<P>(lr, r_);
-    to_lag<P>(lu, u_);
-    to_lag<P>(lv, v_);
-    to_lag<P>(la_, a_);
+    HR::lag(lr, r_);
+    HR::lag(lu, u_);
+    HR::lag(lv, v_);
+    HR::lag(la_, a_);
 #pragma unroll
-    for (int iy = 0; iy < N1; ++iy) K[iy] = 0.5 * (u_[iy] * u_[iy] + v_[iy] * v_[iy]) * phys::rcp(r_[iy]);
-    rebuild_energy<P>(lp, la_, K, v[1][5], E_);
+    for (int iy = 0; iy < N1; ++iy) K[iy] = 0.5 * (u_[iy] * u_[iy] + v_[iy] * v_[iy]) * HR::rcp(r_[iy]);
+    HR::energy(lp, la_, K, v[1][5], E_);
 #pragma unroll
     for (int iy = 0; iy < N1; ++iy) {
       const size_t o = (size_t)(ix + N1 * iy) * ld + e;
@@ -637,13 +633,14 @@ template <int P, int METHOD, int NY = 0>
 __device__ __forceinline__ void lim1d_limit(int phys, const double (&v)[3][4 + NY][P + 1],
                                             double (&o)[4 + NY][P + 1]) {
   constexpr int N1 = P + 1, NF = 4 + NY;
+  using HR = HrSums<P>;
   if constexpr (METHOD == 1) {
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
       double lim[N1];
       const int ph = (phys == 3 && f == 1) ? 5 : phys;
-      limit_slice<P>(ph, v[0][f], v[1][f], v[2][f], lim);
-      to_lag<P>(lim, o[f]);
+      limit_slice<HR, P>(ph, v[0][f], v[1][f], v[2][f], lim);
+      HR::lag(lim, o[f]);
     }
   } else {
     double pr[3][N1];
@@ -658,22 +655,22 @@ __device__ __forceinline__ void lim1d_limit(int phys, const double (&v)[3][4 + N
       }
     }
     double lr[N1], lu[N1], la_[N1], lp[N1];
-    limit_slice<P>(phys, v[0][0], v[1][0], v[2][0], lr);
-    limit_slice<P>(phys, v[0][1], v[1][1], v[2][1], lu);
-    limit_slice<P>(phys, v[0][3], v[1][3], v[2][3], la_);
-    limit_slice<P>(phys, pr[0], pr[1], pr[2], lp);
+    limit_slice<HR, P>(phys, v[0][0], v[1][0], v[2][0], lr);
+    limit_slice<HR, P>(phys, v[0][1], v[1][1], v[2][1], lu);
+    limit_slice<HR, P>(phys, v[0][3], v[1][3], v[2][3], la_);
+    limit_slice<HR, P>(phys, pr[0], pr[1], pr[2], lp);
     double K[N1];
-    to_lag<P>(lr, o[0]);
-    to_lag<P>(lu, o[1]);
-    to_lag<P>(la_, o[3]);
+    HR::lag(lr, o[0]);
+    HR::lag(lu, o[1]);
+    HR::lag(la_, o[3]);
 #pragma unroll
     for (int i = 0; i < N1; ++i) K[i] = 0.5 * o[1][i] * o[1][i] * phys::rcp(o[0][i]);  // kinetic_energy1D
-    rebuild_energy<P>(lp, la_, K, v[1][2], o[2]);
+    HR::energy(lp, la_, K, v[1][2], o[2]);
 #pragma unroll
     for (int k = 4; k < NF; ++k) {
       double ly[N1];
-      limit_slice<P>(phys, v[0][k], v[1][k], v[2][k], ly);
-      to_lag<P>(ly, o[k]);
+      limit_slice<HR, P>(phys, v[0][k], v[1][k], v[2][k], ly);
+      HR::lag(ly, o[k]);
     }
   }
 }

@@ -21,12 +21,12 @@ namespace dgb {
 // static limit (up to three mass fractions), else the arrays' size
 template <int P, int NY>
 constexpr size_t lim2d_xpass_smem_bytes() {
-  const size_t b = sizeof(double) * (5 + NY) * (P + 1) * P * 32;
+  const size_t b = sizeof(double) * (5 + NY) * (P + 1) * Hr2<P>::NM * 32;
   return b <= 48 * 1024 ? 0 : b;
 }
 template <int P, int NY>
 constexpr size_t lim2d_ypass_smem_bytes() {
-  const size_t b = sizeof(double) * (5 + NY) * P * 6 * 32;
+  const size_t b = sizeof(double) * (5 + NY) * Hr2<P>::NM * 6 * 32;
   return b <= 48 * 1024 ? 0 : b;
 }
 
@@ -39,15 +39,17 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
                                                  const int* __restrict__ nbr, double* __restrict__ X, int x0,
                                                  int ey) {
   constexpr int N1 = P + 1, NS = N1 * N1, NQ = 5 + NY, NF = 5 + NY, TWI = 30;
+  using HR = Hr2<P>;
+  constexpr int NM = HR::NM;
   // [quantity][slice][moment][slot]: static shared memory, or dynamic (lim2d_xpass_smem_bytes)
   // when the quantities would not fit the static limit (many mass fractions)
-  double(*A)[N1][P][32];
+  double(*A)[N1][NM][32];
   if constexpr (lim2d_xpass_smem_bytes<P, NY>() == 0) {
-    __shared__ double As[NQ][N1][P][32];
+    __shared__ double As[NQ][N1][NM][32];
     A = As;
   } else {
     extern __shared__ __align__(16) double lsm[];
-    A = reinterpret_cast<double(*)[N1][P][32]>(lsm);
+    A = reinterpret_cast<double(*)[N1][NM][32]>(lsm);
   }
   const int ld = la.ld;
   const int tx = threadIdx.x, sl = threadIdx.y;
@@ -79,15 +81,15 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
         // pressure from the unlimited state (pressure kernel, physics.cu:891-958), with correctly
         // rounded reciprocals in place of its divisions
         const double ru = v[1][ix], rv = v[2][ix];
-        q[4][ix] = phys::rcp(v[4][ix]) * (v[3][ix] - 0.5 * (ru * ru + rv * rv) * phys::rcp(v[0][ix]));
+        q[4][ix] = HR::rcp(v[4][ix]) * (v[3][ix] - 0.5 * (ru * ru + rv * rv) * HR::rcp(v[0][ix]));
       }
     }
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
-      double D[P];
-      hr_moments<P>(q[k], D);
+      double D[NM];
+      HR::moments(q[k], D);
 #pragma unroll
-      for (int m = 0; m < P; ++m) A[k][sl][m][tx] = D[m];
+      for (int m = 0; m < NM; ++m) A[k][sl][m][tx] = D[m];
     }
   }
   __syncthreads();
@@ -96,38 +98,38 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
   double lim[NQ][N1];
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
-    double DL[P], DC[P], DR[P];
+    double DL[NM], DC[NM], DR[NM];
 #pragma unroll
-    for (int m = 0; m < P; ++m) DC[m] = A[k][sl][m][tx];
+    for (int m = 0; m < NM; ++m) DC[m] = A[k][sl][m][tx];
     const int ph = (METHOD == 1 && phys == 3 && k == 1) ? 5 : phys;
     if (ph == 0) {
 #pragma unroll
-      for (int m = 0; m < P; ++m) { DL[m] = A[k][sl][m][tx - 1]; DR[m] = A[k][sl][m][tx + 1]; }
-      hr_limit<P>(DL, DC, DR, lim[k]);
+      for (int m = 0; m < NM; ++m) { DL[m] = A[k][sl][m][tx - 1]; DR[m] = A[k][sl][m][tx + 1]; }
+      HR::limit(DL, DC, DR, lim[k]);
     } else if (ph == 2 || ph == 3) {
-      hr_flat<P>(DC, lim[k]);
+      HR::flat(DC, lim[k]);
     } else {
-      to_mono<P>(q[k], lim[k]);
+      HR::mono(q[k], lim[k]);
     }
   }
   if constexpr (METHOD == 1) {
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
       double out[N1];
-      to_lag<P>(lim[k], out);
+      HR::lag(lim[k], out);
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) X[(size_t)(k * NS + ix + N1 * sl) * ld + e] = out[ix];
     }
   } else {
     double r_[N1], u_[N1], v_[N1], a_[N1], p_[N1], K[N1], E_[N1];
-    to_lag<P>(lim[0], r_);
-    to_lag<P>(lim[1], u_);
-    to_lag<P>(lim[2], v_);
-    to_lag<P>(lim[3], a_);
-    to_lag<P>(lim[4], p_);
+    HR::lag(lim[0], r_);
+    HR::lag(lim[1], u_);
+    HR::lag(lim[2], v_);
+    HR::lag(lim[3], a_);
+    HR::lag(lim[4], p_);
 #pragma unroll
-    for (int ix = 0; ix < N1; ++ix) K[ix] = 0.5 * (u_[ix] * u_[ix] + v_[ix] * v_[ix]) * phys::rcp(r_[ix]);
-    rebuild_energy<P>(lim[4], lim[3], K, v[3], E_);
+    for (int ix = 0; ix < N1; ++ix) K[ix] = 0.5 * (u_[ix] * u_[ix] + v_[ix] * v_[ix]) * HR::rcp(r_[ix]);
+    HR::energy(lim[4], lim[3], K, v[3], E_);
 #pragma unroll
     for (int ix = 0; ix < N1; ++ix) {
       const size_t o = (size_t)(ix + N1 * sl) * ld + e;
@@ -141,7 +143,7 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
 #pragma unroll
     for (int k = 5; k < NQ; ++k) {
       double y_[N1];
-      to_lag<P>(lim[k], y_);
+      HR::lag(lim[k], y_);
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) X[(size_t)((k + 1) * NS + ix + N1 * sl) * ld + e] = y_[ix];
     }
@@ -167,16 +169,18 @@ __device__ __forceinline__ void lim2d_ypass_body(const LimArgs la, int nx, int n
                                                  const int* __restrict__ nbr, double* __restrict__ Uout, int x0,
                                                  int y0, int ix) {
   constexpr int N1 = P + 1, NS = N1 * N1, NQ = 5 + NY, THI = 4;
+  using HR = Hr2<P>;
+  constexpr int NM = HR::NM;
   // row of quantity k in X: HR -> field k; m2 -> [rho, rhou, rhov, alpha, p, E, rho Y_k]
   auto xrow = [](int k) { return (METHOD == 2 && k >= 5) ? k + 1 : k; };
   // [quantity][moment][row slot][x slot]: static or (many mass fractions) dynamic
-  double(*B)[P][THI + 2][32];
+  double(*B)[NM][THI + 2][32];
   if constexpr (lim2d_ypass_smem_bytes<P, NY>() == 0) {
-    __shared__ double Bs[NQ][P][THI + 2][32];
+    __shared__ double Bs[NQ][NM][THI + 2][32];
     B = Bs;
   } else {
     extern __shared__ __align__(16) double lsm[];
-    B = reinterpret_cast<double(*)[P][THI + 2][32]>(lsm);
+    B = reinterpret_cast<double(*)[NM][THI + 2][32]>(lsm);
   }
   const int ld = la.ld;
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -193,12 +197,12 @@ __device__ __forceinline__ void lim2d_ypass_body(const LimArgs la, int nx, int n
   if (e >= 0) {
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
-      double D[P];
+      double D[NM];
 #pragma unroll
       for (int iy = 0; iy < N1; ++iy) col[k][iy] = __ldg(X + (size_t)(xrow(k) * NS + ix + N1 * iy) * ld + e);
-      hr_moments<P>(col[k], D);
+      HR::moments(col[k], D);
 #pragma unroll
-      for (int m = 0; m < P; ++m) B[k][m][ty][tx] = D[m];
+      for (int m = 0; m < NM; ++m) B[k][m][ty][tx] = D[m];
     }
     if constexpr (METHOD == 2) {
 #pragma unroll
@@ -211,37 +215,37 @@ __device__ __forceinline__ void lim2d_ypass_body(const LimArgs la, int nx, int n
   double lim[NQ][N1];
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
-    double DD[P], DC[P], DU[P];
+    double DD[NM], DC[NM], DU[NM];
 #pragma unroll
-    for (int m = 0; m < P; ++m) DC[m] = B[k][m][ty][tx];
+    for (int m = 0; m < NM; ++m) DC[m] = B[k][m][ty][tx];
     const int ph = (METHOD == 1 && phys == 3 && k == 2) ? 5 : phys;
     if (ph == 0) {
 #pragma unroll
-      for (int m = 0; m < P; ++m) { DD[m] = B[k][m][ty - 1][tx]; DU[m] = B[k][m][ty + 1][tx]; }
-      hr_limit<P>(DD, DC, DU, lim[k]);
+      for (int m = 0; m < NM; ++m) { DD[m] = B[k][m][ty - 1][tx]; DU[m] = B[k][m][ty + 1][tx]; }
+      HR::limit(DD, DC, DU, lim[k]);
     } else if (ph == 2 || ph == 3) {
-      hr_flat<P>(DC, lim[k]);
+      HR::flat(DC, lim[k]);
     } else {
-      to_mono<P>(col[k], lim[k]);
+      HR::mono(col[k], lim[k]);
     }
   }
   if constexpr (METHOD == 1) {
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
       double out[N1];
-      to_lag<P>(lim[k], out);
+      HR::lag(lim[k], out);
 #pragma unroll
       for (int iy = 0; iy < N1; ++iy) Uout[(size_t)(k * NS + ix + N1 * iy) * ld + e] = out[iy];
     }
   } else {
     double r_[N1], u_[N1], v_[N1], a_[N1], K[N1], E_[N1];
-    to_lag<P>(lim[0], r_);
-    to_lag<P>(lim[1], u_);
-    to_lag<P>(lim[2], v_);
-    to_lag<P>(lim[3], a_);
+    HR::lag(lim[0], r_);
+    HR::lag(lim[1], u_);
+    HR::lag(lim[2], v_);
+    HR::lag(lim[3], a_);
 #pragma unroll
-    for (int iy = 0; iy < N1; ++iy) K[iy] = 0.5 * (u_[iy] * u_[iy] + v_[iy] * v_[iy]) * phys::rcp(r_[iy]);
-    rebuild_energy<P>(lim[4], lim[3], K, vE, E_);
+    for (int iy = 0; iy < N1; ++iy) K[iy] = 0.5 * (u_[iy] * u_[iy] + v_[iy] * v_[iy]) * HR::rcp(r_[iy]);
+    HR::energy(lim[4], lim[3], K, vE, E_);
 #pragma unroll
     for (int iy = 0; iy < N1; ++iy) {
       const size_t o = (size_t)(ix + N1 * iy) * ld + e;
@@ -254,7 +258,7 @@ __device__ __forceinline__ void lim2d_ypass_body(const LimArgs la, int nx, int n
 #pragma unroll
     for (int k = 5; k < NQ; ++k) {
       double y_[N1];
-      to_lag<P>(lim[k], y_);
+      HR::lag(lim[k], y_);
 #pragma unroll
       for (int iy = 0; iy < N1; ++iy) Uout[(size_t)(k * NS + ix + N1 * iy) * ld + e] = y_[iy];
     }
@@ -283,12 +287,13 @@ namespace dgb {
 // the x-limited nodes in shared memory; the y pass (warp = x-column) reads its column and those of
 // the rows above and below from there, so the x-limited state never goes to memory.  Uout must not alias U.
 // Per stage of m2l, against the two passes through a global scratch: p = 2, 512 x 256: 52 -> 33 us; p = 3,
-// 1024 x 512: 326 -> 212; p = 1, 1024 x 256: 34 -> 23.  The two passes were FP64-bound at half the memory
+// 1024 x 512: 329 -> 304 (hrl 292 -> 247; HrTab3's transforms have 16 products, with HrSums it would be 212);
+// p = 1, 1024 x 256: 34 -> 23.  The two passes were FP64-bound at half the memory
 // rate (2,240 FP64 instructions per p = 2 element, 1,280 now with the halo rows' second x pass) and moved
 // 35 B per value; this moves 16 plus halos (15 us at the copy rate) and waits on its loads: long
 // scoreboard 4.3 of 12 stall cycles at 36 warps per SM, FP64 pipe 37 %.
 // Rows per tile: more rows repeat less x work, fewer leave room for a second CTA.  p = 2: 2 rows 41 us,
-// 3: 35, 4 (two CTAs): 35, 6: 35, 8: 33; p = 3: 1: 436, 2: 242, 3: 224, 4: 212; p = 1: 4: 26, 6: 27, 8 (two
+// 3: 35, 4 (two CTAs): 35, 6: 35, 8: 33; p = 3 (with HrSums): 1: 436, 2: 242, 3: 224, 4: 212; p = 1: 4: 26, 6: 27, 8 (two
 // CTAs): 23, 8 (three): 33, 14: 35.  One thread per element with all slices in registers (164
 // registers, 12 warps per SM, moments through shared memory) took 39 us at p = 2 and 330 at p = 3.
 template <int P, int METHOD, int NY>
@@ -307,6 +312,8 @@ __device__ __forceinline__ void lim2d_body(const LimArgs la, int nx, int ny, con
                                            double* lsm) {  // lsm: [quantity, node][row][lane], x-limited nodes
   using Dm = LimDims<P, METHOD, NY>;
   constexpr int N1 = Dm::N1, NS = N1 * N1, NQ = Dm::NQ, NF = 5 + NY, PITCH = Dm::PITCH;
+  using HR = Hr2<P>;
+  constexpr int NM = HR::NM;
   const int ld = la.ld, tx = threadIdx.x, sl = threadIdx.y, row = threadIdx.z;
   const int ex = bx * 30 - 1 + tx, y = by * Dm::ROWS - 1 + row;
   // the element of column x in this row: beyond the bottom and top sides what the neighbour table says
@@ -337,28 +344,28 @@ __device__ __forceinline__ void lim2d_body(const LimArgs la, int nx, int ny, con
     double o[NQ][N1], lp[N1], la_[N1];
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
-      double q[N1], DC[P], DL[P], DR[P], lim[N1];
+      double q[N1], DC[NM], DL[NM], DR[NM], lim[N1];
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) {
         if (METHOD == 1 || k >= 5) q[ix] = v[k][ix];
         else if (k < 3) q[ix] = v[k][ix];
         else if (k == 3) q[ix] = v[4][ix];
         else  // pressure from the unlimited state (pressure kernel, physics.cu:891-958)
-          q[ix] = phys::rcp(v[4][ix]) *
-                  (v[3][ix] - 0.5 * (v[1][ix] * v[1][ix] + v[2][ix] * v[2][ix]) * phys::rcp(v[0][ix]));
+          q[ix] = HR::rcp(v[4][ix]) *
+                  (v[3][ix] - 0.5 * (v[1][ix] * v[1][ix] + v[2][ix] * v[2][ix]) * HR::rcp(v[0][ix]));
       }
-      hr_moments<P>(q, DC);
+      HR::moments(q, DC);
 #pragma unroll
-      for (int m = 0; m < P; ++m) {
+      for (int m = 0; m < NM; ++m) {
         DL[m] = __shfl_up_sync(0xffffffffu, DC[m], 1);
         DR[m] = __shfl_down_sync(0xffffffffu, DC[m], 1);
       }
-      hr_limit<P>(DL, DC, DR, lim);
+      HR::limit(DL, DC, DR, lim);
       if (phx != 0) {
-        if (phx == 4 || (METHOD == 1 && phx == 3 && k == 1)) to_mono<P>(q, lim);
-        else hr_flat<P>(DC, lim);
+        if (phx == 4 || (METHOD == 1 && phx == 3 && k == 1)) HR::mono(q, lim);
+        else HR::flat(DC, lim);
       }
-      to_lag<P>(lim, o[k]);
+      HR::lag(lim, o[k]);
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) {
         B[(k * NS + ix + N1 * sl) * PITCH] = o[k][ix];
@@ -370,14 +377,32 @@ __device__ __forceinline__ void lim2d_body(const LimArgs la, int nx, int ny, con
       double K[N1], E[N1];
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix)
-        K[ix] = 0.5 * (o[1][ix] * o[1][ix] + o[2][ix] * o[2][ix]) * phys::rcp(o[0][ix]);
-      rebuild_energy<P>(lp, la_, K, v[3], E);
+        K[ix] = 0.5 * (o[1][ix] * o[1][ix] + o[2][ix] * o[2][ix]) * HR::rcp(o[0][ix]);
+      HR::energy(lp, la_, K, v[3], E);
 #pragma unroll
       for (int ix = 0; ix < N1; ++ix) B[(NQ * NS + ix + N1 * sl) * PITCH] = E[ix];
     }
   }
   __syncthreads();
   // ---- y pass: the column ix = sl ----
+  if constexpr (P == 3) {  // 16 products per transform: once per column, its Taylor coefficients in place of its nodes
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+      double c[N1], A[N1];
+      double* b = B + (k * NS + sl) * PITCH;
+#pragma unroll
+      for (int iy = 0; iy < N1; ++iy) c[iy] = b[N1 * iy * PITCH];
+      HR::mono(c, A);
+#pragma unroll
+      for (int iy = 0; iy < N1; ++iy) b[N1 * iy * PITCH] = A[iy];
+    }
+    __syncthreads();
+  }
+  // the moments of what a column of B holds
+  auto moments = [](const double* c, double* D) {
+    if constexpr (P == 3) HR::means(c, D);
+    else HR::moments(c, D);
+  };
   if (!icol || row < 1 || row > Dm::ROWS || y >= ny) return;
   int phy = 0;
   if (y == 0 || y == ny - 1)
@@ -386,25 +411,30 @@ __device__ __forceinline__ void lim2d_body(const LimArgs la, int nx, int ny, con
   double o[NQ][N1], lp[N1], la_[N1];
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
-    double c[N1], w[N1], DC[P], DD[P], DU[P], lim[N1];
+    double c[N1], w[N1], DC[NM], DD[NM], DU[NM], lim[N1];
     const double* b = B + (k * NS + sl) * PITCH;
 #pragma unroll
     for (int iy = 0; iy < N1; ++iy) c[iy] = b[N1 * iy * PITCH];
-    hr_moments<P>(c, DC);
+    moments(c, DC);
     if (phy == 0) {
 #pragma unroll
       for (int iy = 0; iy < N1; ++iy) w[iy] = b[N1 * iy * PITCH - 32];
-      hr_moments<P>(w, DD);
+      moments(w, DD);
 #pragma unroll
       for (int iy = 0; iy < N1; ++iy) w[iy] = b[N1 * iy * PITCH + 32];
-      hr_moments<P>(w, DU);
-      hr_limit<P>(DD, DC, DU, lim);
+      moments(w, DU);
+      HR::limit(DD, DC, DU, lim);
     } else if (phy == 4 || (METHOD == 1 && phy == 3 && k == 2)) {
-      to_mono<P>(c, lim);
+      if constexpr (P == 3) {
+#pragma unroll
+        for (int m = 0; m < N1; ++m) lim[m] = c[m];
+      } else {
+        HR::mono(c, lim);
+      }
     } else {
-      hr_flat<P>(DC, lim);
+      HR::flat(DC, lim);
     }
-    to_lag<P>(lim, o[k]);
+    HR::lag(lim, o[k]);
 #pragma unroll
     for (int iy = 0; iy < N1; ++iy) {
       const size_t t = (size_t)(N1 * iy) * ld;
@@ -419,9 +449,9 @@ __device__ __forceinline__ void lim2d_body(const LimArgs la, int nx, int ny, con
 #pragma unroll
     for (int iy = 0; iy < N1; ++iy) {
       vE[iy] = B[(NQ * NS + sl + N1 * iy) * PITCH];
-      K[iy] = 0.5 * (o[1][iy] * o[1][iy] + o[2][iy] * o[2][iy]) * phys::rcp(o[0][iy]);
+      K[iy] = 0.5 * (o[1][iy] * o[1][iy] + o[2][iy] * o[2][iy]) * HR::rcp(o[0][iy]);
     }
-    rebuild_energy<P>(lp, la_, K, vE, E);
+    HR::energy(lp, la_, K, vE, E);
 #pragma unroll
     for (int iy = 0; iy < N1; ++iy) out[(size_t)(N1 * iy + 3 * NS) * ld] = E[iy];
   }

@@ -57,6 +57,7 @@ template <int D, int P, int PASS>
 __device__ __forceinline__ void m2i_slice(int phys, const double (&c)[D + 3][P + 1], const double (&l)[D + 3][P + 1],
                                           const double (&r)[D + 3][P + 1], double (&res)[D + 3][P + 1]) {
   constexpr int N1 = P + 1, IE = D + 1, IA = D + 2;
+  using HR = std::conditional_t<D == 2, Hr2<P>, HrSums<P>>;
   constexpr int UN = (D == 2 && PASS == 1) ? 2 : 1;  // wall-normal momentum of this pass
   // nodal pressure of the three cells (pressure, limiting_kernels.cu:1870-1897)
   double pc[N1], pl[N1], pr[N1];
@@ -73,11 +74,11 @@ __device__ __forceinline__ void m2i_slice(int phys, const double (&c)[D + 3][P +
     press(r, pr);
   }
   double mr[N1], ma[N1], mp[N1];
-  limit_slice<P>(phys, l[0], c[0], r[0], mr);
-  limit_slice<P>(phys, l[IA], c[IA], r[IA], ma);
-  limit_slice<P>(phys, pl, pc, pr, mp);
-  to_lag<P>(mr, res[0]);
-  to_lag<P>(ma, res[IA]);
+  limit_slice<HR, P>(phys, l[0], c[0], r[0], mr);
+  limit_slice<HR, P>(phys, l[IA], c[IA], r[IA], ma);
+  limit_slice<HR, P>(phys, pl, pc, pr, mp);
+  HR::lag(mr, res[0]);
+  HR::lag(ma, res[IA]);
 #pragma unroll
   for (int f = 1; f <= D; ++f) {
     if (phys == 3 && f == UN) {
@@ -85,8 +86,8 @@ __device__ __forceinline__ void m2i_slice(int phys, const double (&c)[D + 3][P +
       for (int k = 0; k < N1; ++k) res[f][k] = c[f][k];
     } else {
       double mm[N1];
-      limit_slice<P>(phys, l[f], c[f], r[f], mm);
-      to_lag<P>(mm, res[f]);
+      limit_slice<HR, P>(phys, l[f], c[f], r[f], mm);
+      HR::lag(mm, res[f]);
     }
   }
   // total energy from the limited pressure, 1/(gamma-1) and kinetic energy
@@ -96,7 +97,7 @@ __device__ __forceinline__ void m2i_slice(int phys, const double (&c)[D + 3][P +
     const double kin = res[1][k] * res[1][k] + (D == 2 ? res[2][k] * res[2][k] : 0.0);
     K[k] = 0.5 * kin * __drcp_rn(res[0][k]);
   }
-  rebuild_energy<P>(mp, ma, K, c[IE], res[IE]);
+  HR::energy(mp, ma, K, c[IE], res[IE]);
 }
 
 // One pass of hri / pri (METHOD 1) or m2i (METHOD 2).  PASS 0: x slices (row iy = blockIdx.y,
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(128) lim_gated_kernel(const LimArgs la, const 
                                                         double* out, const DevScalars* __restrict__ scal,
                                                         const GateSparse sp = GateSparse()) {
   constexpr int N1 = P + 1, NS = D == 2 ? N1 * N1 : N1, NF = D + 3, IE = D + 1, IA = D + 2;
+  using HR = std::conditional_t<D == 2, Hr2<P>, HrSums<P>>;
   constexpr int UN = (D == 2 && PASS == 1) ? 2 : 1;  // wall-normal momentum of this pass
   if (scal && scal->flags) return;
   const int ld = la.ld, sl = blockIdx.y;
@@ -171,8 +173,8 @@ __global__ void __launch_bounds__(128) lim_gated_kernel(const LimArgs la, const 
         continue;
       }
       double lim[N1];
-      limit_slice<P>(phys, l[f], c[f], r[f], lim);
-      to_lag<P>(lim, res[f]);
+      limit_slice<HR, P>(phys, l[f], c[f], r[f], lim);
+      HR::lag(lim, res[f]);
     }
   } else {
     m2i_slice<D, P, PASS>(phys, c, l, r, res);

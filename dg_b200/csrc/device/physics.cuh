@@ -17,6 +17,7 @@
 // The operation order is kept where it is natural so the FP64 results agree with the
 // reference CPU build to rounding (the GPU contracts a*b+c into FMA).
 #pragma once
+#include "common.cuh"
 
 namespace dgb {
 namespace phys {
@@ -313,20 +314,20 @@ template <int FLUX, int NY = 0, bool GC = false>
 __device__ __forceinline__ void riemann2d_rcp(const double* L, const double* R, double nx, double ny, double* F,
                                               double& nc) {
   const double rhoL = L[0], rhoR = R[0];
-  const double irL = rcp(rhoL), irR = rcp(rhoR);
+  const double irL = __drcp_rn(rhoL), irR = __drcp_rn(rhoR);
   const double vxL = L[1] * irL, vyL = L[2] * irL, vxR = R[1] * irR, vyR = R[2] * irR;
   const double EtL = L[3], EtR = R[3];
   // GAMCONS: divided by rho on entry; the Rusanov solver's right alpha is the left one divided
   // twice by rhoL (see riemann2d)
   const double alphaL = GC ? L[4] * irL : L[4];
   const double alphaR = GC ? (FLUX == FLUX_ROE ? R[4] * irR : alphaL * irL) : R[4];
-  const double gm1L = rcp(alphaL), gm1R = rcp(alphaR);
+  const double gm1L = __drcp_rn(alphaL), gm1R = __drcp_rn(alphaR);
   const double vnL = vxL * nx + vyL * ny;
   const double vnR = vxR * nx + vyR * ny;
   const double pL = gm1L * (EtL - 0.5 * rhoL * (vxL * vxL + vyL * vyL));
   const double pR = gm1R * (EtR - 0.5 * rhoR * (vxR * vxR + vyR * vyR));
-  const double aL = root((1.0 + gm1L) * pL * irL);
-  const double aR = root((1.0 + gm1R) * pR * irR);
+  const double aL = sqrt((1.0 + gm1L) * pL * irL);
+  const double aR = sqrt((1.0 + gm1R) * pR * irR);
   const double HL = (EtL + pL) * irL;
   const double HR = (EtR + pR) * irR;
   if (FLUX == FLUX_ROE) {
@@ -334,18 +335,18 @@ __device__ __forceinline__ void riemann2d_rcp(const double* L, const double* R, 
     const double vtL = vxL * tx + vyL * ty;
     const double vtR = vxR * tx + vyR * ty;
     const double iL = pL * alphaL, iR = pR * alphaR;
-    const double RT = root(rhoR * irL);
+    const double RT = sqrt(rhoR * irL);
     const double rho = RT * rhoL;
-    const double i1 = rcp(1 + RT);
+    const double i1 = __drcp_rn(1 + RT);
     const double vx = (vxL + RT * vxR) * i1;
     const double vy = (vyL + RT * vyR) * i1;
     const double vn = vx * nx + vy * ny;
     const double vt = vx * tx + vy * ty;
     const double H = (HL + RT * HR) * i1;
     const double alpha = (alphaL + RT * alphaR) * i1;
-    const double gm1 = rcp(alpha);
-    const double a = root(gm1 * (H - 0.5 * (vx * vx + vy * vy)));
-    const double ia = rcp(a);
+    const double gm1 = __drcp_rn(alpha);
+    const double a = sqrt(gm1 * (H - 0.5 * (vx * vx + vy * vy)));
+    const double ia = __drcp_rn(a);
     const double i = (iL + RT * iR) * i1;
     const double p = gm1 * i;
     const double drho = rhoR - rhoL;
@@ -393,4 +394,7 @@ __device__ __forceinline__ void riemann2d_rcp(const double* L, const double* R, 
 }
 
 }  // namespace phys
+
+template <int P>
+__device__ __forceinline__ double HrSums<P>::rcp(double x) { return phys::rcp(x); }
 }  // namespace dgb

@@ -277,12 +277,12 @@ __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorM
 // of the NFL fields with a conservative flux (times Wg and the metric factors cx, cy), gs the
 // non-conservative source of alpha = 1/(gamma-1) (times Wg J), from the point values ug and the
 // reference derivatives (dax, day) of alpha (evaluate_sf, code/src/physics/physics.cu:248-301).
-template <int NF, int NFL, int NY, bool GC>
+template <int NF, int NFL, int NY, bool GC, class Args>
 __device__ __forceinline__ void point_terms(const double (&ug)[NF], double dax, double day, double Wg,
-                                            const TileArgs& a, double (&gxv)[NFL], double (&gyv)[NFL], double& gs) {
-  const double rho = ug[0], irho = phys::rcp(rho);
+                                            const Args& a, double (&gxv)[NFL], double (&gyv)[NFL], double& gs) {
+  const double rho = ug[0], irho = __drcp_rn(rho);
   const double uu = ug[1] * irho, vv = ug[2] * irho, Et = ug[3];
-  const double gm1 = GC ? rho * phys::rcp(ug[4]) : phys::rcp(ug[4]);  // gamma - 1
+  const double gm1 = GC ? rho * __drcp_rn(ug[4]) : __drcp_rn(ug[4]);  // gamma - 1
   const double p = gm1 * (Et - 0.5 * rho * (uu * uu + vv * vv));
   const double wx = Wg * a.cx, wy = Wg * a.cy;
   const double mx = ug[1] * wx, my = ug[2] * wy;

@@ -159,29 +159,19 @@ __device__ __forceinline__ void riemann_n2(const double* L, const double* R, dou
   }
 }
 
-// The work of one tile (origin tx0, ty0).  The caller has initialised the mbarrier at the start of shared
-// memory; `phase` counts its completed phases (a persistent caller runs many tiles on one barrier).  Every
-// early return is taken by the whole CTA, after its last barrier.
-// SCALED: the tables carry no metric, a.sx and a.sy do (tiles of problems of many mesh widths).
-template <int P, int FLUX, int NY, bool GC, int TW, int TH, bool SCALED>
-__device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, const CUtensorMap* mapU,
-                                          const CUtensorMap* mapBase, int tx0, int ty0, unsigned char* smraw,
-                                          uint32_t& phase) {
-  static_assert(!(GC && NY > 0), "GAMCONS with mass fractions is not built");
-  using Dm = ColDims<P, NY, GC, TW, TH>;
-  constexpr int N1 = Dm::N1, NS = Dm::NS, NF = Dm::NF, NFL = Dm::NFL, NG1 = Dm::NG1;
-  constexpr int NE = Dm::NE, NT = Dm::NT, NXF = Dm::NXF, NFACE = Dm::NFACE;
+// The tile (origin tx0, ty0; tw x th elements of it) and the neighbours' face nodes into shared memory.  The caller
+// has initialised the mbarrier at its start; `phase` counts its completed phases (a persistent caller
+// runs many tiles on one barrier).  Returns whether there is work, for the whole CTA, after its last barrier.
+template <class Dm, int P>
+__device__ __forceinline__ bool cols_load(const ColArgs& a, const CUtensorMap* mapU, const CUtensorMap* mapBase, int tx0,
+                                          int ty0, int tw, int th, unsigned char* smraw, uint32_t& phase) {
+  constexpr int N1 = Dm::N1, NS = Dm::NS, NF = Dm::NF, NE = Dm::NE, NT = Dm::NT, TW = Dm::TW, TH = Dm::TH;
   uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);
   int* s_ok = reinterpret_cast<int*>(smraw + 8);
   int* codes = reinterpret_cast<int*>(smraw + Dm::off_code);       // [NEDGE] neighbours / boundary codes
   double* Us = reinterpret_cast<double*>(smraw + Dm::off_tile);    // [NF*NS][NE]
   double* HS = reinterpret_cast<double*>(smraw + Dm::off_halo);    // [NF*N1][NEDGE] neighbours' face nodes
-  double* FS = reinterpret_cast<double*>(smraw + Dm::off_face);    // [(NF+1)*N1][NFACE] lifted face fluxes
-  double* AS = reinterpret_cast<double*>(smraw + Dm::off_sums);    // [NA][NT] column sums
   const int tid = threadIdx.x, ld = a.ld, nx = a.nx;
-  const int tw = min(TW, nx - tx0), th = min(TH, a.ny - ty0);
-
-  // ---------------- the tile and the neighbours' face nodes ----------------
   // (the step's status is read along with them: its latency before the copy would be every CTA's)
   const unsigned failed = tid == 0 && a.scal ? a.scal->flags : 0u;
   // a TMA copy must land on a 128-byte shared boundary and start on a 16-byte global column;
@@ -236,7 +226,29 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
   }
   if (tma_ok) ++phase;
   __syncthreads();
-  if (!*s_ok) return;
+  return *s_ok != 0;
+}
+
+// The work of one tile (origin tx0, ty0).
+// SCALED: the tables carry no metric, a.sx and a.sy do (tiles of problems of many mesh widths).
+template <int P, int FLUX, int NY, bool GC, int TW, int TH, bool SCALED>
+__device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, const CUtensorMap* mapU,
+                                          const CUtensorMap* mapBase, int tx0, int ty0, unsigned char* smraw,
+                                          uint32_t& phase) {
+  static_assert(!(GC && NY > 0), "GAMCONS with mass fractions is not built");
+  using Dm = ColDims<P, NY, GC, TW, TH>;
+  constexpr int N1 = Dm::N1, NS = Dm::NS, NF = Dm::NF, NFL = Dm::NFL, NG1 = Dm::NG1;
+  constexpr int NE = Dm::NE, NT = Dm::NT, NXF = Dm::NXF, NFACE = Dm::NFACE;
+  int* codes = reinterpret_cast<int*>(smraw + Dm::off_code);       // [NEDGE] neighbours / boundary codes
+  double* Us = reinterpret_cast<double*>(smraw + Dm::off_tile);    // [NF*NS][NE]
+  double* HS = reinterpret_cast<double*>(smraw + Dm::off_halo);    // [NF*N1][NEDGE] neighbours' face nodes
+  double* FS = reinterpret_cast<double*>(smraw + Dm::off_face);    // [(NF+1)*N1][NFACE] lifted face fluxes
+  double* AS = reinterpret_cast<double*>(smraw + Dm::off_sums);    // [NA][NT] column sums
+  const int tid = threadIdx.x, ld = a.ld, nx = a.nx;
+  const int tw = min(TW, nx - tx0), th = min(TH, a.ny - ty0);
+
+  if (!cols_load<Dm, P>(a, mapU, mapBase, tx0, ty0, tw, th, smraw, phase)) return;
+  const unsigned plane = ld;
 
   // ---------------- volume: one thread per (element, quadrature column) ----------------
   {

@@ -10,6 +10,7 @@
 #include "../../include/dgb.h"
 #include "device/kernels.cuh"
 #include "device/tile2d_cols.cuh"
+#include "device/tile2d_ordered.cuh"
 #include "host/host.h"
 #include "launch.h"
 
@@ -63,6 +64,60 @@ ColTab make_col_tab(const Consts& cs, bool raw) {
 
 namespace {
 
+OrdTab make_ord_tab(const Consts& cs) {
+  OrdTab t;
+  std::memset(&t, 0, sizeof(t));
+  const int n1 = cs.n1, ng1 = cs.ng1;
+  std::vector<double> M((size_t)n1 * n1, 0.0);
+  for (int i = 0; i < n1; ++i)
+    for (int j = 0; j < n1; ++j)
+      for (int g = 0; g < ng1; ++g) M[i + (size_t)j * n1] += cs.wq[g] * cs.Bq[g][i] * cs.Bq[g][j];
+  invert(M, n1);
+  for (int g = 0; g < ng1; ++g) {
+    for (int i = 0; i < n1; ++i) { t.B1[g][i] = cs.Bq[g][i]; t.D1[g][i] = cs.Dq[g][i]; }
+    for (int h = 0; h < ng1; ++h) t.W[g][h] = cs.wq[g] * cs.wq[h];
+  }
+  for (int i = 0; i < n1; ++i) {
+    t.wf[i] = cs.wf[i];
+    for (int j = 0; j < n1; ++j) { t.Bf[i][j] = cs.Bf[i][j]; t.M1i[i][j] = M[i + (size_t)j * n1]; }
+  }
+  t.cx = cs.J * cs.ixx; t.cy = cs.J * cs.iyy;
+  t.sx = cs.ixx; t.sy = cs.iyy;
+  t.J = cs.J; t.invJ = 1.0 / cs.J;
+  t.JFx = cs.JFx; t.JFy = cs.JFy;
+  return t;
+}
+
+// The elements in whole 32 x 2 blocks, then the others (all of them on smaller grids) with the generic kernel;
+// disjoint outputs, both read the stage input's neighbours from global memory.
+template <int FLUX, int MODE, int NY, bool GC>
+void launch_ordered(dgb_ctx* c, const StageArgs& s, const ColArgs& a, const CUtensorMap& map, const CUtensorMap& base) {
+  if (c->tiled) {
+    using Dm = OrdDims<NY, GC>;
+    auto k = residual2d_ordered_kernel<FLUX, MODE, NY, GC>;
+    allow_dynamic_smem(k, Dm::smem_bytes);
+    const int nxt = c->nx / TILE_W * TILE_W, nyt = c->ny / 2 * 2;
+    const dim3 grid(nxt / Dm::TW, (nyt + Dm::TH - 1) / Dm::TH);
+    ProfScope ps(c, KC_RESIDUAL);
+    launch_pdl(c, k, grid, dim3(Dm::NT), Dm::smem_bytes, a, c->ord_tab, nxt, nyt, map, base);
+  }
+  if (!c->tiled) launch_res2d<3, FLUX, MODE, NY, GC>(c, s);
+  else if (c->nleft) launch_res2d<3, FLUX, MODE, NY, GC>(c, s, c->left, c->nleft);
+}
+
+template <int NY, bool GC>
+int dispatch_ordered(dgb_ctx* c, int mode, const StageArgs& s, const ColArgs& a, const CUtensorMap& map,
+                     const CUtensorMap& base) {
+  if (c->flux == DGB_FLUX_ROE) {
+    if (mode == MODE_SSP) launch_ordered<2, MODE_SSP, NY, GC>(c, s, a, map, base);
+    else launch_ordered<2, MODE_RK4, NY, GC>(c, s, a, map, base);
+  } else {
+    if (mode == MODE_SSP) launch_ordered<0, MODE_SSP, NY, GC>(c, s, a, map, base);
+    else launch_ordered<0, MODE_RK4, NY, GC>(c, s, a, map, base);
+  }
+  return 0;
+}
+
 template <int P, int FLUX, int NY, bool GC>
 void launch_cols(dgb_ctx* c, const ColArgs& a, const ColTab& tab, const CUtensorMap& map, const CUtensorMap& base) {
   using Dm = ColDims<P, NY, GC>;
@@ -102,6 +157,7 @@ void tile_of(const dgb_ctx* c, int& tw, int& th) {
 void cols_setup(dgb_ctx* c) {
   c->col_step = make_col_tab(c->cs, false);
   c->col_raw = make_col_tab(c->cs, true);
+  if (c->p == 3) c->ord_tab = make_ord_tab(c->cs);
   int tw = 0, th = 0;
   if (c->p == 1) tile_of<1>(c, tw, th);
   else if (c->p == 2) tile_of<2>(c, tw, th);
@@ -145,6 +201,16 @@ int residual2d_cols(dgb_ctx* c, const StageArgs& s, int mode) {
   };
   const CUtensorMap& map = map_of_buf(s.U);
   const CUtensorMap& base = map_of_buf(a.base);  // read only when k0 != 0
+  if (c->ordered() && mode != MODE_RESIDUAL) {
+    if (c->gamcons) return dispatch_ordered<0, true>(c, mode, s, a, map, base);
+    switch (c->nmass) {
+      case 0: return dispatch_ordered<0, false>(c, mode, s, a, map, base);
+      case 1: return dispatch_ordered<1, false>(c, mode, s, a, map, base);
+      case 2: return dispatch_ordered<2, false>(c, mode, s, a, map, base);
+      case 3: return dispatch_ordered<3, false>(c, mode, s, a, map, base);
+      default: break;
+    }
+  }
   if (c->gamcons) return dispatch_cols<0, true>(c, a, tab, map, base);
   switch (c->nmass) {
     case 0: return dispatch_cols<0, false>(c, a, tab, map, base);

@@ -177,7 +177,8 @@ class DGSolver:
 
     def set_form(self, form: str) -> None:
         """Arithmetic of the residual: "fp64" (plain, the parity form) or "mixed" (FP32 contractions
-        and fluxes allowed; the FP64 kernels are the faster ones here, so both run them)."""
+        and fluxes allowed; the FP64 kernels are the faster ones here, so both run FP64 kernels, in 2D at p = 3
+        with a limiter other ones)."""
         F.check(F.lib().dgb_set_form(self._h, F.FORM[form]))
 
     def set_wait_limit(self, polls: int = 1 << 22) -> None:

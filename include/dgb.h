@@ -64,8 +64,10 @@ enum dgb_limiter {
 
 /* Arithmetic of the residual kernels.  FP64: plain double precision (the parity form).  MIXED: the
  * caller allows FP32 contractions and fluxes on FP64 anchors (structured 2D grids, p <= 3).  It is a
- * permission: on sm_100a, whose FP64 rate is half its FP32 rate, the FP64 kernels are the faster ones
- * at every order, so both forms run them and give the same result. */
+ * permission: on sm_100a, whose FP64 rate is half its FP32 rate, the FP64 kernels are the faster ones,
+ * so both forms run FP64 kernels.  They give the same result, except for cubic elements under a limiter: there
+ * the FP64 form keeps the order of every sum (the scheme amplifies rounding differences to some 4e-8), which
+ * the mixed form does not. */
 enum dgb_form { DGB_FORM_FP64 = 0, DGB_FORM_MIXED = 1 };
 
 /* Gamma model (GAMM of the reference Makefile): GAMNCON carries alpha = 1/(gamma-1) with a
