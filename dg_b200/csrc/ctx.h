@@ -18,7 +18,32 @@
 #include "device/tile2d_cols.cuh"
 #include "device/tile2d_ordered.cuh"
 
+#define DGB_CUDA(call)                                                                          \
+  do {                                                                                          \
+    cudaError_t err_ = (call);                                                                  \
+    if (err_ != cudaSuccess)                                                                    \
+      return set_error(DGB_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(err_));     \
+  } while (0)
+
 namespace dgb {
+int set_error(int code, const std::string& msg);
+
+// What `body` enqueues on st, as an executable graph.  A launch that fails on its own arguments leaves the
+// capture valid, but without that kernel, so the launches' errors are looked at too.
+template <class F>
+int capture_graph(cudaStream_t st, cudaGraphExec_t* exec, F&& body) {
+  const cudaError_t before = cudaPeekAtLastError();
+  cudaGraph_t g = nullptr;
+  DGB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+  int rc = body();
+  cudaError_t e = cudaStreamEndCapture(st, &g);
+  if (e == cudaSuccess && cudaPeekAtLastError() != before) e = cudaGetLastError();
+  if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(exec, g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (!rc && e != cudaSuccess) rc = set_error(DGB_ERR_CUDA, std::string("captured step: ") + cudaGetErrorString(e));
+  return rc;
+}
+
 // Dynamic shared memory above 48 KB is opted into per kernel, and cudaFuncSetAttribute acts on the
 // current device only: done once per (kernel, device), under a lock
 inline cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes) {

@@ -55,6 +55,9 @@ enum { FLAG_NONFINITE = 1u, FLAG_DT_SMALL = 2u, FLAG_TIMEOUT = 4u };
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// the row of tiles of a CTA (tile_grid, launch.h)
+__device__ __forceinline__ int tile_row() { return blockIdx.z * gridDim.y + blockIdx.y; }
+
 // minmod of two arguments (limiting_kernels.cu:1470-1486): the smaller in magnitude when their signs
 // agree, else 0.  Signs are compared as bits (a zero argument gives 0 either way).
 __device__ __forceinline__ double minmod2(double a, double b) {

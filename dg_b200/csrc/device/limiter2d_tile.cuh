@@ -464,7 +464,8 @@ __global__ void __launch_bounds__(LimDims<P, METHOD, NY>::NT, LimDims<P, METHOD,
   extern __shared__ __align__(16) double lsm[];
   pdl_wait();
   if (scal && scal->flags) return;
-  lim2d_body<P, METHOD, NY>(la, nx, ny, U, nbr, Uout, blockIdx.x, blockIdx.y, lsm);
+  if (tile_row() * LimDims<P, METHOD, NY>::ROWS >= ny) return;
+  lim2d_body<P, METHOD, NY>(la, nx, ny, U, nbr, Uout, blockIdx.x, tile_row(), lsm);
   pdl_trigger();
 }
 

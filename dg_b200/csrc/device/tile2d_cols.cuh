@@ -504,8 +504,10 @@ __global__ void __launch_bounds__(ColDims<P, NY, GC>::NT, ColDims<P, NY, GC>::ct
     fence_mbar_init();
   }
   pdl_wait();
+  const int ty0 = tile_row() * TH;
+  if (ty0 >= a.ny) return;
   uint32_t phase = 0;
-  cols_body<P, FLUX, NY, GC, TW, TH, false>(a, tab, &mapU, &mapBase, blockIdx.x * TW, blockIdx.y * TH, smraw, phase);
+  cols_body<P, FLUX, NY, GC, TW, TH, false>(a, tab, &mapU, &mapBase, blockIdx.x * TW, ty0, smraw, phase);
   // (at the end: with the trigger at the start the next launch's CTAs, waiting, hold the shared memory that this
   // one's last wave could use: 240 -> 256 us per 512 x 256 step)
   pdl_trigger();

@@ -65,7 +65,8 @@ __global__ void __launch_bounds__(OrdDims<NY, GC>::NT, OrdDims<NY, GC>::ctas)
   }
   pdl_wait();
   uint32_t phase = 0;
-  const int tid = threadIdx.x, tx0 = blockIdx.x * TW, ty0 = blockIdx.y * TH;
+  const int tid = threadIdx.x, tx0 = blockIdx.x * TW, ty0 = tile_row() * TH;
+  if (ty0 >= nyt) return;
   const int tw = min(TW, nxt - tx0), th = min(TH, nyt - ty0);
   if (!cols_load<Dm, P>(a, &mapU, &mapBase, tx0, ty0, tw, th, smraw, phase)) return;
 

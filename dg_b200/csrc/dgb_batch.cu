@@ -30,13 +30,6 @@ ColTab make_col_tab(const Consts& cs, bool raw);  // dgb_tile.cu
 
 using namespace dgb;
 
-#define DGB_CUDA(call)                                                                          \
-  do {                                                                                          \
-    cudaError_t err_ = (call);                                                                  \
-    if (err_ != cudaSuccess)                                                                    \
-      return set_error(DGB_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(err_));     \
-  } while (0)
-
 namespace {
 
 // residual tile shapes of the 2D classes: width, height (elements).  32 x 2 first: two CTAs of 256 threads
@@ -566,19 +559,8 @@ extern "C" int dgb_batch_advance(dgb_batch* b, int nsteps, double t_end, int* st
   if (!b) return set_error(DGB_ERR_ARG, "batch: null");
   if (nsteps < 0) return set_error(DGB_ERR_ARG, "batch: nsteps < 0");
   DGB_CUDA(cudaSetDevice(b->device));
-  if (!b->graph) {
-    cudaGraph_t g;
-    DGB_CUDA(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
-    const int rc = enqueue_step(b);
-    const cudaError_t ec = cudaStreamEndCapture(b->st, &g);
-    if (rc) {
-      if (ec == cudaSuccess) cudaGraphDestroy(g);
-      return rc;
-    }
-    DGB_CUDA(ec);
-    DGB_CUDA(cudaGraphInstantiate(&b->graph, g, 0));
-    cudaGraphDestroy(g);
-  }
+  if (!b->graph)
+    if (int rc = capture_graph(b->st, &b->graph, [&] { return enqueue_step(b); })) return rc;
   if (int rc = reset_cases(b)) return rc;
   const double te = t_end > 0 ? t_end : 0.0;
   DGB_CUDA(cudaMemcpyAsync(b->d_tend, &te, sizeof(double), cudaMemcpyHostToDevice, b->st));

@@ -53,13 +53,6 @@ const dgb::Problem& dgb_problem_ref(const dgb_problem* p);
 
 using namespace dgb;
 
-#define DGB_CUDA(call)                                                                          \
-  do {                                                                                          \
-    cudaError_t err_ = (call);                                                                  \
-    if (err_ != cudaSuccess)                                                                    \
-      return set_error(DGB_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(err_));     \
-  } while (0)
-
 namespace {
 
 
@@ -1380,15 +1373,10 @@ int ensure_step_graphs(dgb_ctx* c, int scheme, bool cfl) {
   for (int k = 0; k < 2; ++k) {
     const bool sc = k == 0;
     if (c->graphs[si][mi][k] || (!sc && (!c->ind_on || c->ind_every <= 1))) continue;
-    cudaGraph_t g;
-    DGB_CUDA(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
     c->counter = 0;
-    int rc = scheme == DGB_RK4 ? step_rk4(c, cfl, sc) : step_ssprk3(c, cfl, sc);
-    cudaError_t ec = cudaStreamEndCapture(c->st, &g);
-    if (rc) { if (ec == cudaSuccess) cudaGraphDestroy(g); return rc; }
-    DGB_CUDA(ec);
-    DGB_CUDA(cudaGraphInstantiate(&c->graphs[si][mi][k], g, 0));
-    cudaGraphDestroy(g);
+    if (int rc = capture_graph(c->st, &c->graphs[si][mi][k],
+                               [&] { return scheme == DGB_RK4 ? step_rk4(c, cfl, sc) : step_ssprk3(c, cfl, sc); }))
+      return rc;
     c->graph_launches[si][mi][k] = c->counter;
   }
   return DGB_OK;
@@ -1398,16 +1386,11 @@ int ensure_step_graphs(dgb_ctx* c, int scheme, bool cfl) {
 int ensure_multi_graph(dgb_ctx* c, int scheme, bool cfl) {
   cudaGraphExec_t& x = c->multi[scheme == DGB_RK4 ? 1 : 0][cfl ? 1 : 0];
   if (x) return DGB_OK;
-  cudaGraph_t g;
-  DGB_CUDA(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-  int rc = 0;
-  for (int s = 0; s < kMultiSteps && !rc; ++s) rc = scheme == DGB_RK4 ? step_rk4(c, cfl) : step_ssprk3(c, cfl);
-  const cudaError_t ec = cudaStreamEndCapture(c->st, &g);
-  if (rc) { if (ec == cudaSuccess) cudaGraphDestroy(g); return rc; }
-  DGB_CUDA(ec);
-  DGB_CUDA(cudaGraphInstantiate(&x, g, 0));
-  cudaGraphDestroy(g);
-  return DGB_OK;
+  return capture_graph(c->st, &x, [&] {
+    int rc = 0;
+    for (int s = 0; s < kMultiSteps && !rc; ++s) rc = scheme == DGB_RK4 ? step_rk4(c, cfl) : step_ssprk3(c, cfl);
+    return rc;
+  });
 }
 
 // the step's status from the device scalars (read after the step's last kernel)

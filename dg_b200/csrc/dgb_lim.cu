@@ -14,11 +14,11 @@ template <int P, int METHOD, int NY>
 int launch_lim(dgb_ctx* c, const double* in, double* out) {
   using Dm = LimDims<P, METHOD, NY>;
   auto k = lim2d_kernel<P, METHOD, NY>;
-  allow_dynamic_smem(k, Dm::smem_bytes);
-  const dim3 grid((c->nx + 29) / 30, (c->ny + Dm::ROWS - 1) / Dm::ROWS), block(32, Dm::N1, Dm::ROWS + 2);
+  DGB_CUDA(allow_dynamic_smem(k, Dm::smem_bytes));
+  const dim3 grid = tile_grid((c->nx + 29) / 30, (c->ny + Dm::ROWS - 1) / Dm::ROWS), block(32, Dm::N1, Dm::ROWS + 2);
   ProfScope ps(c, KC_LIMITER);
-  launch_pdl(c, k, grid, block, Dm::smem_bytes, LimArgs{c->ld, c->ne}, c->nx, c->ny, in, (const int*)c->nbr, out,
-             (const DevScalars*)c->scal);
+  DGB_CUDA(launch_pdl(c, k, grid, block, Dm::smem_bytes, LimArgs{c->ld, c->ne}, c->nx, c->ny, in, (const int*)c->nbr, out,
+                      (const DevScalars*)c->scal));
   return 0;
 }
 

@@ -91,52 +91,52 @@ OrdTab make_ord_tab(const Consts& cs) {
 // The elements in whole 32 x 2 blocks, then the others (all of them on smaller grids) with the generic kernel;
 // disjoint outputs, both read the stage input's neighbours from global memory.
 template <int FLUX, int MODE, int NY, bool GC>
-void launch_ordered(dgb_ctx* c, const StageArgs& s, const ColArgs& a, const CUtensorMap& map, const CUtensorMap& base) {
+int launch_ordered(dgb_ctx* c, const StageArgs& s, const ColArgs& a, const CUtensorMap& map, const CUtensorMap& base) {
   if (c->tiled) {
     using Dm = OrdDims<NY, GC>;
     auto k = residual2d_ordered_kernel<FLUX, MODE, NY, GC>;
-    allow_dynamic_smem(k, Dm::smem_bytes);
+    DGB_CUDA(allow_dynamic_smem(k, Dm::smem_bytes));
     const int nxt = c->nx / TILE_W * TILE_W, nyt = c->ny / 2 * 2;
-    const dim3 grid(nxt / Dm::TW, (nyt + Dm::TH - 1) / Dm::TH);
+    const dim3 grid = tile_grid(nxt / Dm::TW, (nyt + Dm::TH - 1) / Dm::TH);
     ProfScope ps(c, KC_RESIDUAL);
-    launch_pdl(c, k, grid, dim3(Dm::NT), Dm::smem_bytes, a, c->ord_tab, nxt, nyt, map, base);
+    DGB_CUDA(launch_pdl(c, k, grid, dim3(Dm::NT), Dm::smem_bytes, a, c->ord_tab, nxt, nyt, map, base));
   }
   if (!c->tiled) launch_res2d<3, FLUX, MODE, NY, GC>(c, s);
   else if (c->nleft) launch_res2d<3, FLUX, MODE, NY, GC>(c, s, c->left, c->nleft);
+  return 0;
 }
 
 template <int NY, bool GC>
 int dispatch_ordered(dgb_ctx* c, int mode, const StageArgs& s, const ColArgs& a, const CUtensorMap& map,
                      const CUtensorMap& base) {
   if (c->flux == DGB_FLUX_ROE) {
-    if (mode == MODE_SSP) launch_ordered<2, MODE_SSP, NY, GC>(c, s, a, map, base);
-    else launch_ordered<2, MODE_RK4, NY, GC>(c, s, a, map, base);
-  } else {
-    if (mode == MODE_SSP) launch_ordered<0, MODE_SSP, NY, GC>(c, s, a, map, base);
-    else launch_ordered<0, MODE_RK4, NY, GC>(c, s, a, map, base);
+    return mode == MODE_SSP ? launch_ordered<2, MODE_SSP, NY, GC>(c, s, a, map, base)
+                            : launch_ordered<2, MODE_RK4, NY, GC>(c, s, a, map, base);
   }
-  return 0;
+  return mode == MODE_SSP ? launch_ordered<0, MODE_SSP, NY, GC>(c, s, a, map, base)
+                          : launch_ordered<0, MODE_RK4, NY, GC>(c, s, a, map, base);
 }
 
 template <int P, int FLUX, int NY, bool GC>
-void launch_cols(dgb_ctx* c, const ColArgs& a, const ColTab& tab, const CUtensorMap& map, const CUtensorMap& base) {
+int launch_cols(dgb_ctx* c, const ColArgs& a, const ColTab& tab, const CUtensorMap& map, const CUtensorMap& base) {
   using Dm = ColDims<P, NY, GC>;
   auto k = residual2d_cols_kernel<P, FLUX, NY, GC>;
-  allow_dynamic_smem(k, Dm::smem_bytes);
-  const dim3 grid((c->nx + Dm::TW - 1) / Dm::TW, (c->ny + Dm::TH - 1) / Dm::TH);
+  DGB_CUDA(allow_dynamic_smem(k, Dm::smem_bytes));
+  const dim3 grid = tile_grid((c->nx + Dm::TW - 1) / Dm::TW, (c->ny + Dm::TH - 1) / Dm::TH);
   ProfScope ps(c, KC_RESIDUAL);
-  launch_pdl(c, k, grid, dim3(Dm::NT), Dm::smem_bytes, a, tab, map, base);
+  DGB_CUDA(launch_pdl(c, k, grid, dim3(Dm::NT), Dm::smem_bytes, a, tab, map, base));
+  return 0;
 }
 
 template <int NY, bool GC>
 int dispatch_cols(dgb_ctx* c, const ColArgs& a, const ColTab& tab, const CUtensorMap& map, const CUtensorMap& base) {
   switch (c->p * 10 + c->flux) {
-    case 10: launch_cols<1, 0, NY, GC>(c, a, tab, map, base); return 0;
-    case 12: launch_cols<1, 2, NY, GC>(c, a, tab, map, base); return 0;
-    case 20: launch_cols<2, 0, NY, GC>(c, a, tab, map, base); return 0;
-    case 22: launch_cols<2, 2, NY, GC>(c, a, tab, map, base); return 0;
-    case 30: launch_cols<3, 0, NY, GC>(c, a, tab, map, base); return 0;
-    case 32: launch_cols<3, 2, NY, GC>(c, a, tab, map, base); return 0;
+    case 10: return launch_cols<1, 0, NY, GC>(c, a, tab, map, base);
+    case 12: return launch_cols<1, 2, NY, GC>(c, a, tab, map, base);
+    case 20: return launch_cols<2, 0, NY, GC>(c, a, tab, map, base);
+    case 22: return launch_cols<2, 2, NY, GC>(c, a, tab, map, base);
+    case 30: return launch_cols<3, 0, NY, GC>(c, a, tab, map, base);
+    case 32: return launch_cols<3, 2, NY, GC>(c, a, tab, map, base);
     default: return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (dim, p, flux)");
   }
 }

@@ -14,9 +14,9 @@ namespace dgb {
 
 // A launch on the context's stream, programmatic (the kernel may be scheduled while its predecessor
 // finishes; it waits in pdl_wait) when the context allows it.  Only kernels that call pdl_wait
-// before touching global data are launched this way.
+// before touching global data are launched this way.  Returns the launch's own error.
 template <typename... KArgs, typename... Args>
-void launch_pdl(dgb_ctx* c, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
+cudaError_t launch_pdl(dgb_ctx* c, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -27,7 +27,15 @@ void launch_pdl(dgb_ctx* c, void (*k)(KArgs...), dim3 grid, dim3 block, size_t s
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = c->pdl ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+  return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+}
+
+// Grid of tx x ty tiles: ty in grid.y up to the device's 65,535, beyond it split evenly over grid.z (tile_row
+// gives a CTA its row; rows past the last one have no work).  Grids that narrow and tall are rare, and this way the
+// others pay neither a division nor another order of the tiles.
+inline dim3 tile_grid(int tx, int ty) {
+  const int gz = (ty + 65534) / 65535;
+  return dim3(tx, (ty + gz - 1) / gz, gz);
 }
 
 constexpr int TILE_W = 32, TILE_H = 4;
