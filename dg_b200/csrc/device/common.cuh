@@ -54,6 +54,31 @@ enum { FLAG_NONFINITE = 1u, FLAG_DT_SMALL = 2u, FLAG_TIMEOUT = 4u };
 // next kernel's CTAs be scheduled as this one's finish.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// What an earlier launch wrote, read in a kernel that waits for it.  Not with __ldg (which const __restrict__ pointers
+// can become too): ld.global.nc is for data that nobody writes while the kernel lives, and a kernel that
+// waits lives beside the one that writes.  ld_dep is a plain load that stays behind the wait, and in order with
+// the other such loads.  ld_after is one that may be scheduled freely (1 us per 512 x 256 step), through a pointer
+// that after_wait has made a result of the wait, so that it cannot move above it either.
+__device__ __forceinline__ double ld_dep(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ unsigned ld_dep(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+template <class T>
+__device__ __forceinline__ T* after_wait(T* p) {
+  asm volatile("" : "+l"(p));
+  return p;
+}
+__device__ __forceinline__ double ld_after(const double* p) {
+  double v;
+  asm("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
 
 // the row of tiles of a CTA (tile_grid, launch.h)
 __device__ __forceinline__ int tile_row() { return blockIdx.z * gridDim.y + blockIdx.y; }

@@ -330,9 +330,9 @@ __device__ __forceinline__ void res1d_load(const double* __restrict__ U, int ld,
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
 #pragma unroll
-    for (int t = 0; t < N1; ++t) u[f][t] = __ldg(U + (size_t)(f * N1 + t) * ld + e);
-    if (nL >= 0) uL[f] = __ldg(U + (size_t)(f * N1 + P) * ld + nL);
-    if (nR >= 0) uR[f] = __ldg(U + (size_t)(f * N1) * ld + nR);
+    for (int t = 0; t < N1; ++t) u[f][t] = ld_dep(U + (size_t)(f * N1 + t) * ld + e);
+    if (nL >= 0) uL[f] = ld_dep(U + (size_t)(f * N1 + P) * ld + nL);
+    if (nR >= 0) uR[f] = ld_dep(U + (size_t)(f * N1) * ld + nR);
   }
   // reflective wall: mirror the momentum (rflctive, code/src/bc/boundaries.cu:20-67)
 #pragma unroll
@@ -724,7 +724,7 @@ __global__ void __launch_bounds__(128) lim1d_kernel(const LimArgs la, const doub
 // FP64 operations: the constants are read as constant-bank operands (copied to shared memory before the
 // first use they cost a barrier and a round of loads), the neighbours are known without the table, the
 // step's status and size are read together with the state, and the launch is programmatic, so that the next
-// stage's CTAs are resident when this one ends.  1,000 elements, p = 2, Roe, RK4: 38.8 -> 23.0 us per step
+// stage's CTAs are resident when this one ends.  1,000 elements, p = 2, Roe, RK4: 38.8 -> 22.8 us per step
 // (five launches); 19,997 elements, p = 3, HLL, SSP-RK3: 41 -> 28 us.
 constexpr int RL1D_B = 64;
 template <int P, int FLUX, int MODE, int METHOD>
@@ -747,17 +747,21 @@ __global__ void __launch_bounds__(96) res_lim1d_chain_kernel(const __grid_consta
   const int nL = e > 0 ? e - 1 : e == 0 ? __ldg(a.nbr) : 0;
   const int nR = e >= 0 && e < ne - 1 ? e + 1 : e >= 0 ? __ldg(a.nbr + (size_t)ld + ne - 1) : 0;
   pdl_wait();
-  const unsigned failed = a.scal->flags;
+  const unsigned failed = ld_dep(&a.scal->flags);
   if (e >= 0) {
-    const double dt = a.dt_override > 0 ? a.dt_override : a.scal->dt;
-    double u[NF][N1], uL[NF], uR[NF], r[NF][N1], b0[NF][N1];
+    const double dt = a.dt_override > 0 ? a.dt_override : ld_dep(&a.scal->dt);
+    double u[NF][N1], uL[NF], uR[NF], r[NF][N1], b0[NF][N1], acc[NF][N1];
     res1d_load<P, 0>(a.U, ld, e, nL, nR, u, uL, uR);
     const bool need = MODE == MODE_SSP ? a.a != 0.0 : true;
     const double* base = MODE == MODE_SSP ? a.Ubase : last ? acc_in : a.Us;
 #pragma unroll
     for (int f = 0; f < NF; ++f)
 #pragma unroll
-      for (int t = 0; t < N1; ++t) b0[f][t] = need ? __ldg(base + (size_t)(f * N1 + t) * ld + e) : 0.0;
+      for (int t = 0; t < N1; ++t) {
+        const size_t gi = (size_t)(f * N1 + t) * ld + e;
+        b0[f][t] = need ? ld_dep(base + gi) : 0.0;
+        if constexpr (MODE == MODE_RK4) acc[f][t] = own && !last ? ld_dep(acc_in + gi) : 0.0;
+      }
     res1d_compute<P, FLUX>(c, u, uL, uR, nL, nR, r);
 #pragma unroll
     for (int f = 0; f < NF; ++f)
@@ -772,7 +776,7 @@ __global__ void __launch_bounds__(96) res_lim1d_chain_kernel(const __grid_consta
           w = ssp_update(a.a, a.b, b0[f][t], u[f][t], dt, sm);
         } else {
           const size_t gi = (size_t)(f * N1 + t) * ld + e;
-          if (own && !last && !failed) acc_out[gi] = __ldg(acc_in + gi) + a.b * du;
+          if (own && !last && !failed) acc_out[gi] = acc[f][t] + a.b * du;
           w = b0[f][t] + (last ? a.b : a.beta_next) * du;  // rk.cc:164-170
         }
         V[f * N1 + t][s] = w;
@@ -837,7 +841,7 @@ __global__ void __launch_bounds__(256) wavespeed_kernel(const double* __restrict
   constexpr int NV = DIM == 1 ? 4 : 5;  // fields the wave speed reads
   pdl_trigger();
   pdl_wait();
-  if (scal->flags) return;
+  if (ld_dep(&scal->flags)) return;
   double m = 0.0;
   bool bad = false;
   const int t = blockIdx.y, stride = gridDim.x * blockDim.x;
@@ -848,7 +852,7 @@ __global__ void __launch_bounds__(256) wavespeed_kernel(const double* __restrict
       const int e = e0 + r * stride;
       if (e < n_elem)
 #pragma unroll
-        for (int f = 0; f < NV; ++f) v[r][f] = __ldg(U + (size_t)(f * NS + t) * ld + e);
+        for (int f = 0; f < NV; ++f) v[r][f] = ld_dep(U + (size_t)(f * NS + t) * ld + e);
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -862,7 +866,7 @@ __global__ void __launch_bounds__(256) wavespeed_kernel(const double* __restrict
       if (!(w == w)) bad = true;
       else m = fmax(m, fabs(w));
       if (copy_to)
-        for (int f = 0; f < nf; ++f) copy_to[(size_t)(f * NS + t) * ld + e] = __ldg(U + (size_t)(f * NS + t) * ld + e);
+        for (int f = 0; f < nf; ++f) copy_to[(size_t)(f * NS + t) * ld + e] = ld_dep(U + (size_t)(f * NS + t) * ld + e);
     }
   }
 #pragma unroll

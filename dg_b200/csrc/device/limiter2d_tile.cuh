@@ -65,7 +65,7 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
 #pragma unroll
     for (int f = 0; f < NF; ++f)
 #pragma unroll
-      for (int ix = 0; ix < N1; ++ix) v[f][ix] = __ldg(U + (size_t)(f * NS + ix + N1 * sl) * ld + e);
+      for (int ix = 0; ix < N1; ++ix) v[f][ix] = ld_after(U + (size_t)(f * NS + ix + N1 * sl) * ld + e);
 #pragma unroll
     for (int ix = 0; ix < N1; ++ix) {
 #pragma unroll
@@ -157,8 +157,8 @@ __global__ void __launch_bounds__(32 * (P + 1)) lim2d_xpass_tile_kernel(const Li
                                                                       double* __restrict__ X,
                                                                       const DevScalars* __restrict__ scal) {
   pdl_wait();
-  if (scal && scal->flags) return;
-  lim2d_xpass_body<P, METHOD, NY>(la, nx, U, nbr, X, blockIdx.x * 30, blockIdx.y);
+  if (scal && ld_dep(&scal->flags)) return;
+  lim2d_xpass_body<P, METHOD, NY>(la, nx, after_wait(U), nbr, X, blockIdx.x * 30, blockIdx.y);
   pdl_trigger();
 }
 
@@ -199,14 +199,14 @@ __device__ __forceinline__ void lim2d_ypass_body(const LimArgs la, int nx, int n
     for (int k = 0; k < NQ; ++k) {
       double D[NM];
 #pragma unroll
-      for (int iy = 0; iy < N1; ++iy) col[k][iy] = __ldg(X + (size_t)(xrow(k) * NS + ix + N1 * iy) * ld + e);
+      for (int iy = 0; iy < N1; ++iy) col[k][iy] = ld_after(X + (size_t)(xrow(k) * NS + ix + N1 * iy) * ld + e);
       HR::moments(col[k], D);
 #pragma unroll
       for (int m = 0; m < NM; ++m) B[k][m][ty][tx] = D[m];
     }
     if constexpr (METHOD == 2) {
 #pragma unroll
-      for (int iy = 0; iy < N1; ++iy) vE[iy] = __ldg(X + (size_t)(5 * NS + ix + N1 * iy) * ld + e);
+      for (int iy = 0; iy < N1; ++iy) vE[iy] = ld_after(X + (size_t)(5 * NS + ix + N1 * iy) * ld + e);
     }
   }
   __syncthreads();
@@ -272,8 +272,8 @@ __global__ void __launch_bounds__(32 * 6) lim2d_ypass_tile_kernel(const LimArgs 
                                                                   double* __restrict__ Uout,
                                                                   const DevScalars* __restrict__ scal) {
   pdl_wait();
-  if (scal && scal->flags) return;
-  lim2d_ypass_body<P, METHOD, NY>(la, nx, ny, X, nbr, Uout, blockIdx.x * 32, blockIdx.y * 4, blockIdx.z);
+  if (scal && ld_dep(&scal->flags)) return;
+  lim2d_ypass_body<P, METHOD, NY>(la, nx, ny, after_wait(X), nbr, Uout, blockIdx.x * 32, blockIdx.y * 4, blockIdx.z);
   pdl_trigger();
 }
 
@@ -337,7 +337,7 @@ __device__ __forceinline__ void lim2d_body(const LimArgs la, int nx, int ny, con
 #pragma unroll
     for (int f = 0; f < NF; ++f)
 #pragma unroll
-      for (int ix = 0; ix < N1; ++ix) v[f][ix] = e >= 0 ? __ldg(U + (size_t)(f * NS + ix + N1 * sl) * ld + e) : 1.0;
+      for (int ix = 0; ix < N1; ++ix) v[f][ix] = e >= 0 ? ld_after(U + (size_t)(f * NS + ix + N1 * sl) * ld + e) : 1.0;
     int phx = 0;
     if (e >= 0 && icol && (ex == 0 || ex == nx - 1))
       phx = boundary_code(ex == 0 ? __ldg(nbr + e) : 0, ex == nx - 1 ? __ldg(nbr + (size_t)ld + e) : 0);
@@ -463,9 +463,9 @@ __global__ void __launch_bounds__(LimDims<P, METHOD, NY>::NT, LimDims<P, METHOD,
                  double* __restrict__ Uout, const DevScalars* __restrict__ scal) {
   extern __shared__ __align__(16) double lsm[];
   pdl_wait();
-  if (scal && scal->flags) return;
+  if (scal && ld_dep(&scal->flags)) return;
   if (tile_row() * LimDims<P, METHOD, NY>::ROWS >= ny) return;
-  lim2d_body<P, METHOD, NY>(la, nx, ny, U, nbr, Uout, blockIdx.x, tile_row(), lsm);
+  lim2d_body<P, METHOD, NY>(la, nx, ny, after_wait(U), nbr, Uout, blockIdx.x, tile_row(), lsm);
   pdl_trigger();
 }
 

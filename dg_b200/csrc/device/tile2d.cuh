@@ -231,7 +231,7 @@ __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorM
   if constexpr (!TMA) {
     for (int k = tid; k < NF * NS * NT; k += nthr) {  // [plane][row][column], as the tensor map lands it
       const int q = k / NT, el = k % NT;
-      Us[k] = __ldg(a.U + (size_t)q * ld + (size_t)(ty0 + el / TW) * nx + tx0 + el % TW);
+      Us[k] = ld_dep(a.U + (size_t)q * ld + (size_t)(ty0 + el / TW) * nx + tx0 + el % TW);
     }
   }
   if (TMA && tid == 0) {
@@ -248,7 +248,7 @@ __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorM
     const int ty = r / (NF * N1), f = (r / N1) % NF, j = r % N1;
     const int nb = codes[side * TH + ty];
     double v = 0.0;
-    if (nb >= 0) v = __ldg(a.U + (size_t)(f * NS + (side == 0 ? P + N1 * j : N1 * j)) * ld + nb);
+    if (nb >= 0) v = ld_dep(a.U + (size_t)(f * NS + (side == 0 ? P + N1 * j : N1 * j)) * ld + nb);
     (side == 0 ? HL : HR)[r] = v;
   }
   for (int k = tid; k < 2 * TW * NF * N1; k += nthr) {
@@ -257,7 +257,7 @@ __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorM
     const int tx = r / (NF * N1), f = (r / N1) % NF, j = r % N1;
     const int nb = codes[2 * TH + side * TW + tx];
     double v = 0.0;
-    if (nb >= 0) v = __ldg(a.U + (size_t)(f * NS + (side == 0 ? j + N1 * P : j)) * ld + nb);
+    if (nb >= 0) v = ld_dep(a.U + (size_t)(f * NS + (side == 0 ? j + N1 * P : j)) * ld + nb);
     (side == 0 ? HD : HU)[r] = v;
   }
   if (tid == 0) {
@@ -391,7 +391,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
       const double* base = MODE == MODE_SSP ? a.Ubase : a.Uacc;
       for (int k = tid; k < NF * NS * NT; k += NT) {
         const int q = k / NT, el = k % NT;
-        Ub[k] = __ldg(base + (size_t)q * ld + (size_t)(ty0 + el / TW) * nx + tx0 + el % TW);
+        Ub[k] = ld_dep(base + (size_t)q * ld + (size_t)(ty0 + el / TW) * nx + tx0 + el % TW);
       }
     }
   }
@@ -489,7 +489,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
     __syncthreads();
     if (!*s_ok) return;
   }
-  const double dt = a.dt_override > 0 ? a.dt_override : a.scal->dt;
+  const double dt = a.dt_override > 0 ? a.dt_override : ld_dep(&a.scal->dt);
   const double sc = dt * a.invJ;
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
@@ -515,7 +515,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
         const int t = ix + N1 * iy;
         const size_t gi = (size_t)(f * NS + t) * ld + e;
         if (MODE == MODE_SSP) {
-          const double ub = kPrefetch ? Ub[(f * NS + t) * NT + tid] : (a.a != 0.0 ? __ldg(a.Ubase + gi) : 0.0);
+          const double ub = kPrefetch ? Ub[(f * NS + t) * NT + tid] : (a.a != 0.0 ? ld_dep(a.Ubase + gi) : 0.0);
           const double base = a.a != 0.0 ? a.a * ub : 0.0;
           a.out[gi] = base + a.b * (us[(f * NS + t) * NT] + du);
         } else {
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(TW * TH, 2)
                            const __grid_constant__ CUtensorMap mapB) {
   extern __shared__ __align__(128) unsigned char smraw[];
   pdl_wait();
-  if (a.scal && a.scal->flags) return;
+  if (a.scal && ld_dep(&a.scal->flags)) return;
   if (threadIdx.x == 0) {
     mbar_init(reinterpret_cast<uint64_t*>(smraw), 1);
     fence_mbar_init();

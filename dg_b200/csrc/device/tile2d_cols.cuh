@@ -172,8 +172,9 @@ __device__ __forceinline__ bool cols_load(const ColArgs& a, const CUtensorMap* m
   double* Us = reinterpret_cast<double*>(smraw + Dm::off_tile);    // [NF*NS][NE]
   double* HS = reinterpret_cast<double*>(smraw + Dm::off_halo);    // [NF*N1][NEDGE] neighbours' face nodes
   const int tid = threadIdx.x, ld = a.ld, nx = a.nx;
+  const double* U = after_wait(a.U);
   // (the step's status is read along with them: its latency before the copy would be every CTA's)
-  const unsigned failed = tid == 0 && a.scal ? a.scal->flags : 0u;
+  const unsigned failed = tid == 0 && a.scal ? ld_dep(&a.scal->flags) : 0u;
   // a TMA copy must land on a 128-byte shared boundary and start on a 16-byte global column;
   // otherwise record the fault and skip the copy
   const bool tma_ok = a.tma && (smem_u32(Us) & 127u) == 0 && ((tx0 * 8) & 15) == 0;
@@ -189,7 +190,7 @@ __device__ __forceinline__ bool cols_load(const ColArgs& a, const CUtensorMap* m
   if (!a.tma) {
     for (int k = tid; k < NF * NS * NE; k += NT) {
       const int q = k / NE, el = k % NE, x = el % TW, y = el / TW;
-      Us[k] = x < tw && y < th ? __ldg(a.U + (size_t)q * ld + (size_t)(ty0 + y) * nx + tx0 + x) : 0.0;
+      Us[k] = x < tw && y < th ? ld_after(U + (size_t)q * ld + (size_t)(ty0 + y) * nx + tx0 + x) : 0.0;
     }
   }
   // edge slot s of the tile (left, right, bottom, top): the neighbour across it -- the next element of the row or
@@ -210,7 +211,7 @@ __device__ __forceinline__ bool cols_load(const ColArgs& a, const CUtensorMap* m
       const unsigned o = ((side ? (hi ? 0 : P) : (hi ? 0 : N1 * P)) + (side ? N1 : 1) * j) * plane + (unsigned)nb;
       double v[NF];
 #pragma unroll
-      for (int f = 0; f < NF; ++f) v[f] = nb >= 0 ? __ldg(a.U + (o + f * NS * plane)) : 0.0;
+      for (int f = 0; f < NF; ++f) v[f] = nb >= 0 ? ld_after(U + (o + f * NS * plane)) : 0.0;
       if (j == 0) codes[s] = nb;
 #pragma unroll
       for (int f = 0; f < NF; ++f) HS[(f * N1 + j) * Dm::NEDGE + s] = v[f];
@@ -425,6 +426,7 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
   const int el = tid % NE, tx = el % TW, ty = el / TW, r0 = tid / NE;
   const bool own = tx < tw && ty < th;
   const unsigned g0 = N1 * r0 * plane + (unsigned)((ty0 + ty) * nx + tx0 + tx);
+  const double *base = after_wait(a.base), *base2 = after_wait(a.base2);
   double v0[NIT][N1], v2[NIT][N1];
 #pragma unroll
   for (int q = 0; q < NIT; ++q) {
@@ -432,11 +434,11 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
 #pragma unroll
     for (int ix = 0; ix < N1; ++ix) {
       const unsigned gi = g0 + (q * NG1 * N1 + ix) * plane;
-      v0[q][ix] = on && a.k0 != 0.0 ? a.base[gi] : 0.0;
-      v2[q][ix] = on && a.out2 ? a.base2[gi] : 0.0;
+      v0[q][ix] = on && a.k0 != 0.0 ? ld_after(base + gi) : 0.0;
+      v2[q][ix] = on && a.out2 ? ld_after(base2 + gi) : 0.0;
     }
   }
-  const double dt = a.dt > 0 ? a.dt : a.scal->dt;
+  const double dt = a.dt > 0 ? a.dt : ld_dep(&a.scal->dt);
   __syncthreads();
   if (own) {
     const double* fx = FS + r0 * NFACE + ty * (TW + 1) + tx;

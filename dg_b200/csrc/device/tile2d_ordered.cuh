@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(OrdDims<NY, GC>::NT, OrdDims<NY, GC>::ctas)
   const bool own = ty < th;
   const unsigned g0 = N1 * r0 * plane + (unsigned)((ty0 + ty) * a.nx + tx0 + tx);
   const bool two = MODE == MODE_RK4 && a.out2;
+  const double *base = after_wait(a.base), *base2 = after_wait(a.base2);
   double v0[NIT][N1], v2[NIT][N1];
 #pragma unroll
   for (int q = 0; q < NIT; ++q) {
@@ -188,11 +189,11 @@ __global__ void __launch_bounds__(OrdDims<NY, GC>::NT, OrdDims<NY, GC>::ctas)
 #pragma unroll
     for (int ix = 0; ix < N1; ++ix) {
       const unsigned gi = g0 + (q * NG1 * N1 + ix) * plane;
-      v0[q][ix] = on && a.k0 != 0.0 ? a.base[gi] : 0.0;
-      v2[q][ix] = on && two ? a.base2[gi] : 0.0;
+      v0[q][ix] = on && a.k0 != 0.0 ? ld_after(base + gi) : 0.0;
+      v2[q][ix] = on && two ? ld_after(base2 + gi) : 0.0;
     }
   }
-  const double dt = a.dt > 0 ? a.dt : a.scal->dt;
+  const double dt = a.dt > 0 ? a.dt : ld_dep(&a.scal->dt);
   const double sc = dt * tab.invJ;
   __syncthreads();
 #pragma unroll
