@@ -89,6 +89,23 @@ __device__ __forceinline__ double minmod2(double a, double b) {
   const double m = fabs(a) < fabs(b) ? a : b;
   return (__double2hiint(a) ^ __double2hiint(b)) < 0 ? 0.0 : m;
 }
+// The same where an argument may be a NaN, which has no sign: against another number it gives 0, so that an element
+// beside one with a NaN keeps its mean; 0 or NaN against a NaN gives NaN.
+__device__ __forceinline__ double minmod2_nan(double a, double b) {
+  if (!(fabs(a) < fabs(b)) && !(fabs(a) >= fabs(b))) return b != b && !(fabs(a) > 0.0) ? b : 0.0;
+  return minmod2(a, b);
+}
+// Whether one of two values is infinite or a NaN, on the integer pipe.  The limiters test the cell sums of the two
+// neighbours, which no infinity or NaN among their nodes leaves finite, once per slice and take minmod2_nan
+// then.  p = 2, 512 x 256: 33.2 us per stage, 33.6 with the test in every minmod, 32.7 without; p = 3, 1024 x 512:
+// 315, 329 and 305.
+__device__ __forceinline__ bool nonfinite2(double a, double b) {
+  return max((unsigned)__double2hiint(a) << 1, (unsigned)__double2hiint(b) << 1) >= 0xffe00000u;
+}
+template <bool NANS>
+__device__ __forceinline__ double minmod2_of(double a, double b) {
+  return NANS ? minmod2_nan(a, b) : minmod2(a, b);
+}
 
 // ---- hierarchical reconstruction of one 1D slice -------------------------------------------------
 // Nodes are equispaced on [-1, 1]; a[n] are scaled Taylor coefficients, u(x) = sum a_n x^n / n!.  The
@@ -119,22 +136,27 @@ __device__ __forceinline__ double hr_mean(const double* D) {
   return P == 1 ? 0.5 * D[0] : P == 2 ? D[0] * (1.0 / 6.0) : 0.125 * D[0];
 }
 // the limited Taylor coefficients of the cell with moments DC between neighbours DL and DR
-template <int P>
-__device__ __forceinline__ void hr_limit(const double* DL, const double* DC, const double* DR, double* lim) {
+template <int P, bool NANS>
+__device__ __forceinline__ void hr_limit_of(const double* DL, const double* DC, const double* DR, double* lim) {
   if constexpr (P == 1) {
-    lim[1] = 0.25 * minmod2(DC[0] - DL[0], DR[0] - DC[0]);
+    lim[1] = 0.25 * minmod2_of<NANS>(DC[0] - DL[0], DR[0] - DC[0]);
     lim[0] = 0.5 * DC[0];
   } else if constexpr (P == 2) {
-    lim[2] = 0.25 * minmod2(DC[1] - DL[1], DR[1] - DC[1]);
-    lim[1] = minmod2((DC[0] - DL[0]) * (1.0 / 12.0) + lim[2], (DR[0] - DC[0]) * (1.0 / 12.0) - lim[2]);
+    lim[2] = 0.25 * minmod2_of<NANS>(DC[1] - DL[1], DR[1] - DC[1]);
+    lim[1] = minmod2_of<NANS>((DC[0] - DL[0]) * (1.0 / 12.0) + lim[2], (DR[0] - DC[0]) * (1.0 / 12.0) - lim[2]);
     lim[0] = (DC[0] - lim[2]) * (1.0 / 6.0);
   } else {
-    lim[3] = 0.5625 * minmod2(DC[2] - DL[2], DR[2] - DC[2]);
-    lim[2] = minmod2(0.25 * (DC[1] - DL[1]) + lim[3], 0.25 * (DR[1] - DC[1]) - lim[3]);
+    lim[3] = 0.5625 * minmod2_of<NANS>(DC[2] - DL[2], DR[2] - DC[2]);
+    lim[2] = minmod2_of<NANS>(0.25 * (DC[1] - DL[1]) + lim[3], 0.25 * (DR[1] - DC[1]) - lim[3]);
     const double t = lim[3] * (-5.0 / 6.0);
-    lim[1] = minmod2(0.0625 * (DC[0] - DL[0]) + (t + lim[2]), 0.0625 * (DR[0] - DC[0]) + (t - lim[2]));
+    lim[1] = minmod2_of<NANS>(0.0625 * (DC[0] - DL[0]) + (t + lim[2]), 0.0625 * (DR[0] - DC[0]) + (t - lim[2]));
     lim[0] = 0.125 * DC[0] - lim[2] * (1.0 / 6.0);
   }
+}
+template <int P>
+__device__ __forceinline__ void hr_limit(const double* DL, const double* DC, const double* DR, double* lim) {
+  if (nonfinite2(DL[0], DR[0])) hr_limit_of<P, true>(DL, DC, DR, lim);
+  else hr_limit_of<P, false>(DL, DC, DR, lim);
 }
 // the cell mean kept, the rest zero (average_monomial, limiting_kernels.cu:1777-1790)
 template <int P>
@@ -266,16 +288,21 @@ struct HrTab3 {
     mono(v, a);
     means(a, D);
   }
-  static __device__ __forceinline__ void limit(const double* DL, const double* DC, const double* DR, double* lim) {
+  template <bool NANS>
+  static __device__ __forceinline__ void limit_of(const double* DL, const double* DC, const double* DR, double* lim) {
     // a neighbour's mean less that of the limited higher terms over its interval, [-3, -1] or [1, 3]
     auto side = [](double d, double r) { return 0.5 * __dsub_rn(d, r); };
-    auto pick = [](double l, double c, double r) { return minmod2(0.5 * __dsub_rn(c, l), 0.5 * __dsub_rn(r, c)); };
+    auto pick = [](double l, double c, double r) { return minmod2_of<NANS>(0.5 * __dsub_rn(c, l), 0.5 * __dsub_rn(r, c)); };
     lim[3] = pick(0.5 * DL[2], 0.5 * DC[2], 0.5 * DR[2]);
     const double r3 = __dmul_rn(lim[3], 26.0 / 6.0);
     lim[2] = pick(side(DL[1], r3), side(DC[1], __dmul_rn(lim[3], 2.0 / 6.0)), side(DR[1], r3));
     const double r2 = __dmul_rn(lim[2], 26.0 / 6.0);
     lim[0] = side(DC[0], __dmul_rn(lim[2], 2.0 / 6.0));
     lim[1] = pick(side(DL[0], __fma_rn(lim[3], -80.0 / 24.0, r2)), lim[0], side(DR[0], __fma_rn(lim[3], 80.0 / 24.0, r2)));
+  }
+  static __device__ __forceinline__ void limit(const double* DL, const double* DC, const double* DR, double* lim) {
+    if (nonfinite2(DL[0], DR[0])) limit_of<true>(DL, DC, DR, lim);
+    else limit_of<false>(DL, DC, DR, lim);
   }
   static __device__ __forceinline__ void flat(const double* DC, double* lim) {
     lim[0] = 0.5 * DC[0];
