@@ -168,9 +168,9 @@ __global__ void __launch_bounds__(NT) residual2d_kernel(const Consts cin, const 
       // the volume terms of the tiled kernel's point_terms: the conservative fluxes of the NFL
       // fields (mass fractions rho Y_k u, physics.cu:293-298; GAMCONS alpha flux rho u/(gamma-1),
       // physics.cu:253-281) and, under GAMNCON, the alpha source
-      const double rho = ug[0], irho = __drcp_rn(rho);
+      const double rho = ug[0], irho = phys::rcp_of<P == 3>(rho);
       const double uu = ug[1] * irho, vv = ug[2] * irho, Et = ug[3];
-      const double gm1 = GC ? rho * __drcp_rn(ug[4]) : __drcp_rn(ug[4]);
+      const double gm1 = GC ? rho * phys::rcp_of<P == 3>(ug[4]) : phys::rcp_of<P == 3>(ug[4]);
       const double p = gm1 * (Et - 0.5 * rho * (uu * uu + vv * vv));
       const double W = c.wq[g / NG1] * c.wq[g % NG1];
       const double wx = W * (c.J * c.ixx), wy = W * (c.J * c.iyy);
@@ -189,9 +189,9 @@ __global__ void __launch_bounds__(NT) residual2d_kernel(const Consts cin, const 
       if constexpr (!GC) G[(2 * NFL * NG + g) * TE + el] = (W * c.J) * (-uu * dax * c.ixx - vv * day * c.iyy);
       continue;
     }
-    // physics.cu:248-257 with correctly rounded reciprocals in place of its divisions
-    const double rho = ug[0], ir = __drcp_rn(rho), u = ug[1] * ir, v = ug[2] * ir, Et = ug[3];
-    const double p = __drcp_rn(ug[4]) * (Et - 0.5 * rho * (u * u + v * v));
+    // physics.cu:248-257 with reciprocals in place of its divisions
+    const double rho = ug[0], ir = phys::rcp_of<P == 3>(rho), u = ug[1] * ir, v = ug[2] * ir, Et = ug[3];
+    const double p = phys::rcp_of<P == 3>(ug[4]) * (Et - 0.5 * rho * (u * u + v * v));
     const double W = c.wq[g / NG1] * c.wq[g % NG1];
     const double cx = W * (c.ixx * c.J), cy = W * (c.iyy * c.J);
     G[(0 * NG + g) * TE + el] = cx * (rho * u);
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(NT) residual2d_kernel(const Consts cin, const 
 #pragma unroll
     for (int f = 0; f < NF; ++f) { L[f] = swapLR ? un[f] : uo[f]; R[f] = swapLR ? uo[f] : un[f]; }
     double F[NF], nc;
-    phys::riemann2d_rcp<FLUX, NY, GC>(L, R, nx, ny, F, nc);  // the tiled kernel's flux (reciprocals for divisions)
+    phys::riemann2d_rcp<FLUX, NY, GC, P == 3>(L, R, nx, ny, F, nc);  // the tiled kernel's flux (reciprocals for divisions)
     const double jw = (xface ? c.JFx : c.JFy) * c.wf[g];
 #pragma unroll
     for (int f = 0; f < NF; ++f) {

@@ -49,6 +49,12 @@ __device__ __forceinline__ double root(double x) {
   return (unsigned)__double2hiint(x) << 1 < 0x00200000u ? 0.0 : g;
 }
 
+// 1/x and sqrt(x) in a kernel of cubic elements in 2D (EXACT: correctly rounded, see HrTab3) or any other
+template <bool EXACT>
+__device__ __forceinline__ double rcp_of(double x) { return EXACT ? __drcp_rn(x) : rcp(x); }
+template <bool EXACT>
+__device__ __forceinline__ double root_of(double x) { return EXACT ? sqrt(x) : root(x); }
+
 // ---------------------------------------------------------------- 1D -------------------------
 // Interface flux F[4] and ncterm for the alpha equation (F[3] holds the alpha dissipation).
 // Caller forms q_L = -F + nc (element on side L) and q_R = F + nc (physics.cu:800-804).
@@ -309,24 +315,24 @@ namespace phys {
 // The same 2D interface fluxes evaluated with one reciprocal per state instead of repeated
 // divisions (x/rho -> x * (1/rho), gamma-1 = 1/alpha).  Agrees with riemann2d to a few ulp,
 // far inside the 1e-12 parity bound; used by the tiled kernel.
-template <int FLUX, int NY = 0, bool GC = false>
+template <int FLUX, int NY, bool GC, bool EXACT>
 __device__ __forceinline__ void riemann2d_rcp(const double* L, const double* R, double nx, double ny, double* F,
                                               double& nc) {
   const double rhoL = L[0], rhoR = R[0];
-  const double irL = __drcp_rn(rhoL), irR = __drcp_rn(rhoR);
+  const double irL = rcp_of<EXACT>(rhoL), irR = rcp_of<EXACT>(rhoR);
   const double vxL = L[1] * irL, vyL = L[2] * irL, vxR = R[1] * irR, vyR = R[2] * irR;
   const double EtL = L[3], EtR = R[3];
   // GAMCONS: divided by rho on entry; the Rusanov solver's right alpha is the left one divided
   // twice by rhoL (see riemann2d)
   const double alphaL = GC ? L[4] * irL : L[4];
   const double alphaR = GC ? (FLUX == FLUX_ROE ? R[4] * irR : alphaL * irL) : R[4];
-  const double gm1L = __drcp_rn(alphaL), gm1R = __drcp_rn(alphaR);
+  const double gm1L = rcp_of<EXACT>(alphaL), gm1R = rcp_of<EXACT>(alphaR);
   const double vnL = vxL * nx + vyL * ny;
   const double vnR = vxR * nx + vyR * ny;
   const double pL = gm1L * (EtL - 0.5 * rhoL * (vxL * vxL + vyL * vyL));
   const double pR = gm1R * (EtR - 0.5 * rhoR * (vxR * vxR + vyR * vyR));
-  const double aL = sqrt((1.0 + gm1L) * pL * irL);
-  const double aR = sqrt((1.0 + gm1R) * pR * irR);
+  const double aL = root_of<EXACT>((1.0 + gm1L) * pL * irL);
+  const double aR = root_of<EXACT>((1.0 + gm1R) * pR * irR);
   const double HL = (EtL + pL) * irL;
   const double HR = (EtR + pR) * irR;
   if (FLUX == FLUX_ROE) {
@@ -334,18 +340,18 @@ __device__ __forceinline__ void riemann2d_rcp(const double* L, const double* R, 
     const double vtL = vxL * tx + vyL * ty;
     const double vtR = vxR * tx + vyR * ty;
     const double iL = pL * alphaL, iR = pR * alphaR;
-    const double RT = sqrt(rhoR * irL);
+    const double RT = root_of<EXACT>(rhoR * irL);
     const double rho = RT * rhoL;
-    const double i1 = __drcp_rn(1 + RT);
+    const double i1 = rcp_of<EXACT>(1 + RT);
     const double vx = (vxL + RT * vxR) * i1;
     const double vy = (vyL + RT * vyR) * i1;
     const double vn = vx * nx + vy * ny;
     const double vt = vx * tx + vy * ty;
     const double H = (HL + RT * HR) * i1;
     const double alpha = (alphaL + RT * alphaR) * i1;
-    const double gm1 = __drcp_rn(alpha);
-    const double a = sqrt(gm1 * (H - 0.5 * (vx * vx + vy * vy)));
-    const double ia = __drcp_rn(a);
+    const double gm1 = rcp_of<EXACT>(alpha);
+    const double a = root_of<EXACT>(gm1 * (H - 0.5 * (vx * vx + vy * vy)));
+    const double ia = rcp_of<EXACT>(a);
     const double i = (iL + RT * iR) * i1;
     const double p = gm1 * i;
     const double drho = rhoR - rhoL;

@@ -187,7 +187,7 @@ __device__ __forceinline__ void tile_face_fluxes(const double* Us, const double*
       R[f] = sr;
     }
     double F[NF], nc;
-    phys::riemann2d_rcp<FLUX, NY, GC>(L, R, nxv, nyv, F, nc);
+    phys::riemann2d_rcp<FLUX, NY, GC, P == 3>(L, R, nxv, nyv, F, nc);
     // boundary faces seen from the right/top element store -F so that every consumer forms
     // (+F + nc) on its left/bottom face and (-F + nc) on its right/top face
 #pragma unroll
@@ -231,7 +231,7 @@ __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorM
   if constexpr (!TMA) {
     for (int k = tid; k < NF * NS * NT; k += nthr) {  // [plane][row][column], as the tensor map lands it
       const int q = k / NT, el = k % NT;
-      Us[k] = ld_dep(a.U + (size_t)q * ld + (size_t)(ty0 + el / TW) * nx + tx0 + el % TW);
+      Us[k] = __ldg(a.U + (size_t)q * ld + (size_t)(ty0 + el / TW) * nx + tx0 + el % TW);
     }
   }
   if (TMA && tid == 0) {
@@ -248,7 +248,7 @@ __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorM
     const int ty = r / (NF * N1), f = (r / N1) % NF, j = r % N1;
     const int nb = codes[side * TH + ty];
     double v = 0.0;
-    if (nb >= 0) v = ld_dep(a.U + (size_t)(f * NS + (side == 0 ? P + N1 * j : N1 * j)) * ld + nb);
+    if (nb >= 0) v = __ldg(a.U + (size_t)(f * NS + (side == 0 ? P + N1 * j : N1 * j)) * ld + nb);
     (side == 0 ? HL : HR)[r] = v;
   }
   for (int k = tid; k < 2 * TW * NF * N1; k += nthr) {
@@ -257,7 +257,7 @@ __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorM
     const int tx = r / (NF * N1), f = (r / N1) % NF, j = r % N1;
     const int nb = codes[2 * TH + side * TW + tx];
     double v = 0.0;
-    if (nb >= 0) v = ld_dep(a.U + (size_t)(f * NS + (side == 0 ? j + N1 * P : j)) * ld + nb);
+    if (nb >= 0) v = __ldg(a.U + (size_t)(f * NS + (side == 0 ? j + N1 * P : j)) * ld + nb);
     (side == 0 ? HD : HU)[r] = v;
   }
   if (tid == 0) {
@@ -277,12 +277,12 @@ __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorM
 // of the NFL fields with a conservative flux (times Wg and the metric factors cx, cy), gs the
 // non-conservative source of alpha = 1/(gamma-1) (times Wg J), from the point values ug and the
 // reference derivatives (dax, day) of alpha (evaluate_sf, code/src/physics/physics.cu:248-301).
-template <int NF, int NFL, int NY, bool GC, class Args>
+template <int NF, int NFL, int NY, bool GC, bool EXACT, class Args>
 __device__ __forceinline__ void point_terms(const double (&ug)[NF], double dax, double day, double Wg,
                                             const Args& a, double (&gxv)[NFL], double (&gyv)[NFL], double& gs) {
-  const double rho = ug[0], irho = __drcp_rn(rho);
+  const double rho = ug[0], irho = phys::rcp_of<EXACT>(rho);
   const double uu = ug[1] * irho, vv = ug[2] * irho, Et = ug[3];
-  const double gm1 = GC ? rho * __drcp_rn(ug[4]) : __drcp_rn(ug[4]);  // gamma - 1
+  const double gm1 = GC ? rho * phys::rcp_of<EXACT>(ug[4]) : phys::rcp_of<EXACT>(ug[4]);  // gamma - 1
   const double p = gm1 * (Et - 0.5 * rho * (uu * uu + vv * vv));
   const double wx = Wg * a.cx, wy = Wg * a.cy;
   const double mx = ug[1] * wx, my = ug[2] * wy;
@@ -391,7 +391,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
       const double* base = MODE == MODE_SSP ? a.Ubase : a.Uacc;
       for (int k = tid; k < NF * NS * NT; k += NT) {
         const int q = k / NT, el = k % NT;
-        Ub[k] = ld_dep(base + (size_t)q * ld + (size_t)(ty0 + el / TW) * nx + tx0 + el % TW);
+        Ub[k] = __ldg(base + (size_t)q * ld + (size_t)(ty0 + el / TW) * nx + tx0 + el % TW);
       }
     }
   }
@@ -437,7 +437,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
 #pragma unroll
       for (int iy = 0; iy < N1; ++iy) { dax += DGB_TAB2(P, B1[gy][iy]) * dT[iy]; day += DGB_TAB2(P, D1[gy][iy]) * Tc[4][iy]; }
       double gxv[NFL], gyv[NFL], gs;
-      point_terms<NF, NFL, NY, GC>(ug, dax, day, DGB_TAB2(P, W[g]), a, gxv, gyv, gs);
+      point_terms<NF, NFL, NY, GC, P == 3>(ug, dax, day, DGB_TAB2(P, W[g]), a, gxv, gyv, gs);
       if constexpr (kSfLift) {
 #pragma unroll
         for (int iy = 0; iy < N1; ++iy) {
@@ -489,7 +489,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
     __syncthreads();
     if (!*s_ok) return;
   }
-  const double dt = a.dt_override > 0 ? a.dt_override : ld_dep(&a.scal->dt);
+  const double dt = a.dt_override > 0 ? a.dt_override : a.scal->dt;
   const double sc = dt * a.invJ;
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
@@ -515,7 +515,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
         const int t = ix + N1 * iy;
         const size_t gi = (size_t)(f * NS + t) * ld + e;
         if (MODE == MODE_SSP) {
-          const double ub = kPrefetch ? Ub[(f * NS + t) * NT + tid] : (a.a != 0.0 ? ld_dep(a.Ubase + gi) : 0.0);
+          const double ub = kPrefetch ? Ub[(f * NS + t) * NT + tid] : (a.a != 0.0 ? __ldg(a.Ubase + gi) : 0.0);
           const double base = a.a != 0.0 ? a.a * ub : 0.0;
           a.out[gi] = base + a.b * (us[(f * NS + t) * NT] + du);
         } else {
@@ -531,8 +531,7 @@ __global__ void __launch_bounds__(TW * TH, 2)
     residual2d_tile_kernel(const TileArgs a, const __grid_constant__ CUtensorMap mapU,
                            const __grid_constant__ CUtensorMap mapB) {
   extern __shared__ __align__(128) unsigned char smraw[];
-  pdl_wait();
-  if (a.scal && ld_dep(&a.scal->flags)) return;
+  if (a.scal && a.scal->flags) return;
   if (threadIdx.x == 0) {
     mbar_init(reinterpret_cast<uint64_t*>(smraw), 1);
     fence_mbar_init();

@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(DMMA_THREADS, 2)
       for (int i = 0; i < 2; ++i) {
         const int q = 2 * nb + i;
         double gxv[4], gyv[4], gs;
-        point_terms<NF, 4, 0, false>(ug[i], dax[i], day[i], T->wq[q][c], a, gxv, gyv, gs);
+        point_terms<NF, 4, 0, false, false>(ug[i], dax[i], day[i], T->wq[q][c], a, gxv, gyv, gs);
         const double kx = T->lift[0 * 4 + q][lane], ky = T->lift[1 * 4 + q][lane], ka = T->lift[2 * 4 + q][lane];
         const double kx8 = T->lift8[0 * 4 + q][c], ky8 = T->lift8[1 * 4 + q][c], ka8 = T->lift8[2 * 4 + q][c];
 #pragma unroll

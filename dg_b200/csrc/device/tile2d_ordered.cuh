@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(OrdDims<NY, GC>::NT, OrdDims<NY, GC>::ctas)
 #pragma unroll
         for (int iy = 0; iy < N1; ++iy) { dax += tab.B1[gy][iy] * dT[iy]; day += tab.D1[gy][iy] * Tc[4][iy]; }
         double gxv[NFL], gyv[NFL], gs;
-        point_terms<NF, NFL, NY, GC>(ug, dax, day, tab.W[gx][gy], tab, gxv, gyv, gs);
+        point_terms<NF, NFL, NY, GC, true>(ug, dax, day, tab.W[gx][gy], tab, gxv, gyv, gs);
 #pragma unroll
         for (int iy = 0; iy < N1; ++iy) {
           const double b = tab.B1[gy][iy], d = tab.D1[gy][iy];
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(OrdDims<NY, GC>::NT, OrdDims<NY, GC>::ctas)
       R[f] = sr;
     }
     double F[NF], nc;
-    phys::riemann2d_rcp<FLUX, NY, GC>(L, R, nxv, nyv, F, nc);
+    phys::riemann2d_rcp<FLUX, NY, GC, true>(L, R, nxv, nyv, F, nc);
 #pragma unroll
     for (int f = 0; f < NF; ++f) FS[(f * N1 + g) * NFACE + fc] = sgn * F[f];
     FS[(NF * N1 + g) * NFACE + fc] = nc;

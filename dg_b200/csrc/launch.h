@@ -83,7 +83,9 @@ void launch_tile2d(dgb_ctx* c, const StageArgs& s) {
                           : MODE == MODE_SSP ? map_of(c, s.Ubase) : MODE == MODE_RK4 && s.Uacc ? map_of(c, s.Uacc) : mu;
   dim3 grid(c->nx / TILE_W, c->ny / TH);
   ProfScope ps(c, KC_RESIDUAL);
-  launch_pdl(c, k, grid, dim3(TILE_W * TH), smem, a, mu, mb);
+  // (not programmatic: the kernel reads its stage base between its stores, with read-only loads; plain ones, which
+  // wait for the stores, cost a third of its time)
+  k<<<grid, dim3(TILE_W * TH), smem, c->st>>>(a, mu, mb);
 }
 
 constexpr int RES2D_TE = 16;
