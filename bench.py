@@ -17,7 +17,7 @@ device-side CFL step.  DOF = N_E * N_s * N_F = 5,898,240.
              on average for SSP-RK3) / its average device time from a profiled pass of the same steps
   cpu_baseline  the reference CPU build (oracle/_ref, compiled from the reference sources) on a
              bounded sample of the same workload, one process on one core
-  forms      plain FP64, mixed and mixed + learned indicator at equal L1 error (same protocol)
+  forms      plain FP64, mixed (at p = 2 the same FP64 kernels) and learned indicator (same protocol)
   mass_fraction  the workload with one passive mass fraction (6 fields): time per step
   gamma_model  the workload grid with Roe + hrl in both gamma models (GAMNCON, GAMCONS): time per step
   slab_local  the workload split into y-slabs with ghost rows, all in this process on one GPU
@@ -25,8 +25,8 @@ device-side CFL step.  DOF = N_E * N_s * N_F = 5,898,240.
              rows' distance from it
   tube_1d    the 1D two-fluid shock tube (1000 elements, p=2, Roe, RK4, CFL 0.4, 2000 steps): device
              time, distance from the reference's own run, the reference CPU build's time
-  learned_deploy  the learned indicator on a 1024x1024 four-quadrant problem: FP64 / mixed / mixed +
-             gated limiter, time per step and L1 density distance from the FP64 full-limiter run
+  learned_deploy  the learned indicator on a 1024x1024 four-quadrant problem: FP64 / mixed (the same kernels at
+             p = 2) / gated limiter, time per step and L1 density distance from the FP64 full-limiter run
   mixed_p3   the 2048x1024 p=3 Roe shock-bubble: FP64 and mixed throughput, per-field L1 / Linf of
              the mixed form against the FP64 run and the conserved totals after 300 steps
   ensemble   the batched ensemble (256 independent cases of uneven sizes, dgb_batch): aggregate
@@ -286,8 +286,8 @@ def cell_means(prob, U, field=0):
 
 
 def compare_forms(dgb, U0_coarse, dev, steps, warmup, flush, acc_steps=200):
-    """The forms of the solver on the benchmark workload: throughput of plain FP64, mixed and
-    mixed + learned indicator (same timing protocol as the headline), and their L1 density error
+    """The forms of the solver on the benchmark workload: throughput of plain FP64, mixed (at p = 2 the
+    same FP64 kernels) and learned indicator (same timing protocol as the headline), and their L1 density error
     after `acc_steps` fixed steps against a 2x-refined plain FP64 solution (1024 x 512, half the
     step) projected on the 512 x 256 cells."""
     from dg_b200 import learned as L
@@ -493,7 +493,7 @@ DEPLOY_N, DEPLOY_STEPS, DEPLOY_SEED = 1024, 100, 4097
 def learned_deploy(dgb, dev, timed=20, warmup=3, steps=DEPLOY_STEPS):
     """The learned indicator on its deployment problem: a seeded four-quadrant Riemann problem on
     1024 x 1024 quads, p = 2, Rusanov, m2l, SSP-RK3, CFL 0.3 (states as in the training set, a
-    problem outside it).  Plain FP64 with the full limiter, mixed with the full limiter and mixed
+    problem outside it).  Plain FP64 with the full limiter, mixed (at p = 2 the same kernels) and mixed
     with the indicator-gated limiter (threshold 0.2, band of face neighbours, scored every
     IND_EVERY steps): device time per step, and after `steps` fixed steps the L1 density distance of each
     run from the plain FP64 full-limiter run (the judge) and the flagged / band fractions."""
@@ -715,7 +715,8 @@ P3_NX, P3_NY, P3_STEPS = 2048, 1024, 300
 
 def mixed_p3(dgb, dev, steps=P3_STEPS, timed=10):
     """The p=3 configuration: shock-bubble on 2048 x 1024 quads, p = 3, Roe, m2l, SSP-RK3, CFL 0.3.
-    Throughput of the plain FP64 and the mixed form (same protocol as the headline, without the L2
+    Throughput of the plain FP64 form (whose limited cubic runs keep the order of every sum) and the mixed form
+    (FP64 kernels that do not; same protocol as the headline, without the L2
     flush: the 2.7 GB state is 21x the L2), then both advanced `steps` CFL steps from the same
     state: per-field relative L1 and Linf error of the mixed form against the FP64 run, and the
     conserved totals (domain integrals of the five fields) of both at the start and the end."""
@@ -1034,12 +1035,12 @@ def main(argv=None) -> int:
         tube = tube_1d(dgb, dev, with_reference=rank == 0 and not args.no_cpu_baseline)
 
     form_cfg = {"form": ("plain FP64" if args.form == "fp64" else
-                         "mixed: FP32 contractions/Rusanov flux on FP64 anchors, FP64 pressure, state and update")
+                         "mixed (FP32 contractions allowed; runs the FP64 kernels)")
                 + (f" + learned indicator (threshold 0.2, scored every {IND_EVERY} steps)" if args.learned else "")}
     if rank == 0:
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": dev_ms / args.steps, "higher_is_better": True,
-                "scaling": "weak", "vs_baseline": None, "dtype": "f64" if args.form == "fp64" else "f64+f32",
+                "scaling": "weak", "vs_baseline": None, "dtype": "f64",
                 "data": "synthetic",
                 "config": config(form_cfg) if (args.nx, args.ny) == (NX, NY) else config(
                     {"workload": f"profiling case {args.nx}x{args.ny} (not the benchmark workload)",
@@ -1047,9 +1048,7 @@ def main(argv=None) -> int:
                 "e2e": e2e,
                 "roofline": {"bound": "hbm", "achieved": achieved_gbs, "peak": peak, "unit": "GB/s",
                              "frac": achieved_gbs / peak, "traffic": traffic,
-                             "kernel": ("residual2d_tile_kernel<p=2,Rusanov,SSP> (fused residual + stage update)"
-                                        if args.form == "fp64" else
-                                        "residual2d_tile_mixed_kernel<p=2,Rusanov,SSP> (mixed form)"),
+                             "kernel": "residual2d_cols_kernel<p=2,Rusanov> (fused residual + stage update)",
                              "algorithmic_bytes_per_launch": BYTES_PER_DOF_STAGE * dof,
                              "algorithmic_bytes_per_stage": {"stage1": 16.0 * dof, "stage2_3": 24.0 * dof},
                              "traffic_per_stage": traffic_stages,

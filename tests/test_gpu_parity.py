@@ -116,24 +116,32 @@ def test_sensors(solvers, name):
     assert np.array_equal(s.sensors(d["Uraw"]), d["sens"])
 
 
-@pytest.mark.parametrize("limiter,order,bc", [("m2l", 2, ("periodic",) * 4), ("hrl", 1, ("reflective",) * 4),
-                                              ("m2l", 3, ("reflective", "transmissive", "reflective", "transmissive"))])
-def test_fused_limiter_matches_two_pass_limiter(limiter, order, bc, monkeypatch):
-    """The opt-in single-kernel limiter (x and y passes fused) equals the two tiled passes."""
+SIDES = ("reflective", "transmissive", "reflective", "transmissive")
+
+
+@pytest.mark.parametrize("limiter,order,bc", [
+    ("m2l", 2, ("periodic",) * 4), ("hrl", 1, ("reflective",) * 4), ("m2l", 3, SIDES), ("hrl", 3, SIDES[1:] + SIDES[:1]),
+    ("hrl", 2, SIDES[1:] + SIDES[:1]), ("m2l", 1, SIDES),
+])
+@pytest.mark.parametrize("nx,ny", [(70, 29), (30, 8), (31, 9), (29, 1), (61, 17)])
+def test_one_launch_limiter_matches_the_passes(limiter, order, bc, nx, ny, monkeypatch):
+    """The limiter with both passes in one launch (tiles of 30 columns x 8 rows, p = 3: 4) against the generic passes of
+    any element order, on extents at, below and above its tiles: alone, and in steps (whose residuals are
+    other kernels too).  Some 100 products per value: 1e-13 of the state's scale, 1e-12 after four steps."""
     import dg_b200 as dgb
-    prob = dgb.Problem.structured(2, order, 70, 29, 0.0, 2.0, 0.0, 1.0, bc, flux="rusanov", limiter=limiter, cfl=0.3)
+    prob = dgb.Problem.structured(2, order, nx, ny, 0.0, 2.0, 0.0, 1.0, bc, flux="rusanov", limiter=limiter, cfl=0.3)
     U0 = prob.init_state("shock_bubble", seed=9)
-    two = dgb.DGSolver(prob)
-    monkeypatch.setenv("DGB_FUSED_LIMITER", "1")
-    fused = dgb.DGSolver(prob)
-    monkeypatch.delenv("DGB_FUSED_LIMITER")
+    tiled = dgb.DGSolver(prob)
+    monkeypatch.setenv("DGB_NO_TILE", "1")
+    generic = dgb.DGSolver(prob)
+    monkeypatch.delenv("DGB_NO_TILE")
     try:
-        assert rel_err(fused.limit(U0), two.limit(U0)) < 1e-13
-        U1 = two.limit(U0)
-        for s in (two, fused):
+        assert rel_err(tiled.limit(U0), generic.limit(U0)) < 1e-13
+        U1 = generic.limit(U0)
+        for s in (tiled, generic):
             s.set_state(U1)
             s.advance(4, 0.0, scheme=dgb.SSPRK3)
-        assert rel_err(fused.get_state(), two.get_state()) < 1e-12
+        assert rel_err(tiled.get_state(), generic.get_state()) < 1e-12
     finally:
-        two.close()
-        fused.close()
+        tiled.close()
+        generic.close()
