@@ -1,8 +1,9 @@
 // 2D limiters of structured row-major grids (HR and m2 methods).
 //
-//   lim2d_kernel       both passes in one launch, out of place: one thread per element
-//   lim2d_*pass_*      x pass, then y pass through a global scratch: the batched ensemble, the
-//                      allocation-free limiter, primitive variables, sides with frozen data
+//   lim2d_kernel       both passes in one launch, out of place: one thread per element and slice (its body also
+//                      limits the batched ensemble)
+//   lim2d_*pass_*      x pass, then y pass through a global scratch: the allocation-free limiter, primitive
+//                      variables, more than three mass fractions
 //
 // Either way every element's moments (hr_moments) are computed once per slice and shared with the
 // neighbours that need them.
@@ -78,8 +79,8 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
         q[1][ix] = v[1][ix];
         q[2][ix] = v[2][ix];
         q[3][ix] = v[4][ix];
-        // pressure from the unlimited state (pressure kernel, physics.cu:891-958), with correctly
-        // rounded reciprocals in place of its divisions
+        // pressure from the unlimited state (pressure kernel, physics.cu:891-958), with reciprocals in place of
+        // its divisions
         const double ru = v[1][ix], rv = v[2][ix];
         q[4][ix] = HR::rcp(v[4][ix]) * (v[3][ix] - 0.5 * (ru * ru + rv * rv) * HR::rcp(v[0][ix]));
       }

@@ -115,7 +115,7 @@ constexpr bool kSfLift = DGB_SF_LIFT != 0;
 // boundary faces seen from the right/top element store -F so that every consumer forms (+F + nc)
 // on its left/bottom face and (-F + nc) on its right/top face.
 // Work items k0 <= k < k1 (x-faces first, then y-faces); item k goes to record k - rec0.
-template <int P, int FLUX, int TW, int TH, int NY, bool GC>
+template <int P, int FLUX, int TW, int TH, int NY>
 __device__ __forceinline__ void tile_face_fluxes(const double* Us, const double* HL, const double* HR,
                                                  const double* HD, const double* HU, const int* codes, double* Fs,
                                                  int tid, int nthr, int k0, int k1, int rec0) {
@@ -187,7 +187,7 @@ __device__ __forceinline__ void tile_face_fluxes(const double* Us, const double*
       R[f] = sr;
     }
     double F[NF], nc;
-    phys::riemann2d_rcp<FLUX, NY, GC, P == 3>(L, R, nxv, nyv, F, nc);
+    phys::riemann2d_rcp<FLUX, NY, false, P == 3>(L, R, nxv, nyv, F, nc);
     // boundary faces seen from the right/top element store -F so that every consumer forms
     // (+F + nc) on its left/bottom face and (-F + nc) on its right/top face
 #pragma unroll
@@ -197,11 +197,11 @@ __device__ __forceinline__ void tile_face_fluxes(const double* Us, const double*
 }
 
 // Phase 0 of a tile (origin tx0, ty0): boundary codes of the tile edges, the tile's nodal state
-// (TMA copy, or plain coalesced loads when TMA = false) and the four neighbour face-node strips into
+// (TMA copy) and the four neighbour face-node strips into
 // shared memory, by `nthr` threads.  Returns whether the tile copy arrived (CTA-uniform); a copy that
 // could not start or whose bounded wait ran out sets FLAG_TIMEOUT.  `phase` counts the mbarrier's
 // completed phases.
-template <int P, int TW, int TH, int NY, bool TMA>
+template <int P, int TW, int TH, int NY>
 __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorMap* mapU, int tx0, int ty0,
                                               unsigned char* smraw, uint32_t& phase, int tid, int nthr) {
   using Dm = TileDims<P, TW, TH, NY>;
@@ -227,14 +227,8 @@ __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorM
   __syncthreads();
   // a TMA copy must land on a 128-byte shared boundary and start on a 16-byte global column;
   // otherwise record the fault and skip the copy (the wait below then reports it)
-  const bool tma_ok = TMA && (smem_u32(Us) & 127u) == 0 && (smem_u32(Fs) & 127u) == 0 && ((tx0 * 8) & 15) == 0;
-  if constexpr (!TMA) {
-    for (int k = tid; k < NF * NS * NT; k += nthr) {  // [plane][row][column], as the tensor map lands it
-      const int q = k / NT, el = k % NT;
-      Us[k] = __ldg(a.U + (size_t)q * ld + (size_t)(ty0 + el / TW) * nx + tx0 + el % TW);
-    }
-  }
-  if (TMA && tid == 0) {
+  const bool tma_ok = (smem_u32(Us) & 127u) == 0 && (smem_u32(Fs) & 127u) == 0 && ((tx0 * 8) & 15) == 0;
+  if (tid == 0) {
     if (tma_ok) {
       mbar_arrive_expect_tx(bar, Dm::tile_bytes);
       tma_load_3d(Us, mapU, tx0, ty0, 0, bar);
@@ -261,8 +255,8 @@ __device__ __forceinline__ bool tile_stage_in(const TileArgs& a, const CUtensorM
     (side == 0 ? HD : HU)[r] = v;
   }
   if (tid == 0) {
-    bool ok = !TMA || (tma_ok && mbar_wait(bar, phase & 1, a.polls));
-    if (TMA && tma_ok && !ok) {
+    bool ok = tma_ok && mbar_wait(bar, phase & 1, a.polls);
+    if (tma_ok && !ok) {
       atomicOr(a.errflag, (unsigned)FLAG_TIMEOUT);
       mbar_wait(bar, phase & 1);
     }
@@ -299,19 +293,14 @@ __device__ __forceinline__ void point_terms(const double (&ug)[NF], double dax, 
 // barrier).  Every early return is taken by the whole CTA, after its last barrier.
 // NY passive mass fractions rho*Y_k follow the five gamma-model fields: conservative volume flux
 // rho*Y_k (u, v) (physics.cu:293-298) and the interface fluxes of phys::riemann2d_rcp.
-// GC: the GAMCONS model (fifth field rho/(gamma-1), conservative flux rho u/(gamma-1), no source;
-// physics.cu:253-281), with NY = 0.
-// TMA = false: the tile and the stage base come in by plain coalesced loads (grids whose row pitch
-// nx * 8 bytes is not a multiple of 16, which a tensor map cannot describe); same arithmetic.
-template <int P, int FLUX, int MODE, int TW, int TH, int UNROLL, int NY = 0, bool GC = false, bool TMA = true>
+template <int P, int FLUX, int MODE, int TW, int TH, int UNROLL, int NY = 0>
 __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap* mapU, const CUtensorMap* mapB,
                                             int tx0, int ty0, unsigned char* smraw, uint32_t& phase) {
-  static_assert(!(GC && NY > 0), "GAMCONS with mass fractions is not built");
   using Dm = TileDims<P, TW, TH, NY>;
   constexpr int N1 = Dm::N1, NS = Dm::NS, NF = Dm::NF, NT = Dm::NT, NXF = Dm::NXF;
-  constexpr int FS = NF + 1;             // face record: NF fluxes, ncterm
-  constexpr int NFL = 4 + NY + (GC ? 1 : 0);  // fields with a volume flux (rho, rho u, rho v, E, alpha | rho Y_k)
-  auto fld = [](int k) { return (GC || k < 4) ? k : k + 1; };
+  constexpr int FS = NF + 1;   // face record: NF fluxes, ncterm
+  constexpr int NFL = 4 + NY;  // fields with a volume flux (rho, rho u, rho v, E | rho Y_k)
+  auto fld = [](int k) { return k < 4 ? k : k + 1; };
   uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);
   int* s_ok = reinterpret_cast<int*>(smraw + 8);
   int* codes = reinterpret_cast<int*>(smraw + Dm::head_bytes);  // [L: TH][R: TH][D: TW][U: TW]
@@ -329,10 +318,10 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
   constexpr int NYF = Dm::NYF;
 
   // ---------------- phase 0: stage the tile (TMA) and the neighbour strips ----------------
-  if (!tile_stage_in<P, TW, TH, NY, TMA>(a, mapU, tx0, ty0, smraw, phase, tid, NT)) return;
+  if (!tile_stage_in<P, TW, TH, NY>(a, mapU, tx0, ty0, smraw, phase, tid, NT)) return;
 
   // ---------------- phase 1: face fluxes, each face of the tile once ----------------
-  tile_face_fluxes<P, FLUX, TW, TH, NY, GC>(Us, HL, HR, HD, HU, codes, Fs, tid, NT, 0, kSplit ? NXF : NXF + NYF, 0);
+  tile_face_fluxes<P, FLUX, TW, TH, NY>(Us, HL, HR, HD, HU, codes, Fs, tid, NT, 0, kSplit ? NXF : NXF + NYF, 0);
   __syncthreads();
 
   // ---------------- phase 2: volume terms and assembly, one thread per element ----------------
@@ -350,7 +339,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
   for (int kf = 0; kf < 4; ++kf) {
     if (kSplit && kf == 2) {
       __syncthreads();  // every thread has read its x-face records
-      tile_face_fluxes<P, FLUX, TW, TH, NY, GC>(Us, HL, HR, HD, HU, codes, Fs, tid, NT, NXF, NXF + NYF, NXF);
+      tile_face_fluxes<P, FLUX, TW, TH, NY>(Us, HL, HR, HD, HU, codes, Fs, tid, NT, NXF, NXF + NYF, NXF);
       __syncthreads();
     }
     const int yrec = kSplit ? 0 : NXF;  // first y-face record in the buffer
@@ -382,17 +371,9 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
     // the face buffer is free once every thread has read its face fluxes
     fence_proxy_async_smem();
     __syncthreads();
-    if constexpr (TMA) {
-      if (tid == 0 && need) {
-        mbar_arrive_expect_tx(bar, Dm::tile_bytes);
-        tma_load_3d(Ub, mapB, tx0, ty0, 0, bar);
-      }
-    } else if (need) {
-      const double* base = MODE == MODE_SSP ? a.Ubase : a.Uacc;
-      for (int k = tid; k < NF * NS * NT; k += NT) {
-        const int q = k / NT, el = k % NT;
-        Ub[k] = __ldg(base + (size_t)q * ld + (size_t)(ty0 + el / TW) * nx + tx0 + el % TW);
-      }
+    if (tid == 0 && need) {
+      mbar_arrive_expect_tx(bar, Dm::tile_bytes);
+      tma_load_3d(Ub, mapB, tx0, ty0, 0, bar);
     }
   }
 
@@ -437,21 +418,21 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
 #pragma unroll
       for (int iy = 0; iy < N1; ++iy) { dax += DGB_TAB2(P, B1[gy][iy]) * dT[iy]; day += DGB_TAB2(P, D1[gy][iy]) * Tc[4][iy]; }
       double gxv[NFL], gyv[NFL], gs;
-      point_terms<NF, NFL, NY, GC, P == 3>(ug, dax, day, DGB_TAB2(P, W[g]), a, gxv, gyv, gs);
+      point_terms<NF, NFL, NY, false, P == 3>(ug, dax, day, DGB_TAB2(P, W[g]), a, gxv, gyv, gs);
       if constexpr (kSfLift) {
 #pragma unroll
         for (int iy = 0; iy < N1; ++iy) {
           const double b = DGB_TAB2(P, B1[gy][iy]), d = DGB_TAB2(P, D1[gy][iy]);
 #pragma unroll
           for (int f = 0; f < NFL; ++f) { Ax[f][iy] += b * gxv[f]; Ay[f][iy] += d * gyv[f]; }
-          if (!GC) As[iy] += b * gs;
+          As[iy] += b * gs;
         }
       } else {
 #pragma unroll
         for (int t = 0; t < NS; ++t) {
 #pragma unroll
           for (int f = 0; f < NFL; ++f) r[fld(f)][t] += DGB_TAB2(P, dPx[g][t]) * gxv[f] + DGB_TAB2(P, dPy[g][t]) * gyv[f];
-          if (!GC) r[4][t] += DGB_TAB2(P, Phi[g][t]) * gs;
+          r[4][t] += DGB_TAB2(P, Phi[g][t]) * gs;
         }
       }
     }
@@ -465,7 +446,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
           const int t = ix + N1 * iy;
 #pragma unroll
           for (int f = 0; f < NFL; ++f) r[fld(f)][t] += dx * Ax[f][iy] + bx * Ay[f][iy];
-          if (!GC) r[4][t] += bx * As[iy];
+          r[4][t] += bx * As[iy];
         }
     }
   }
@@ -477,7 +458,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
     return;
   }
   if (need) {
-    if (TMA && tid == 0) {
+    if (tid == 0) {
       bool ok = mbar_wait(bar, phase & 1, a.polls);
       if (!ok) {
         atomicOr(a.errflag, (unsigned)FLAG_TIMEOUT);
@@ -485,7 +466,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
       }
       *s_ok = ok ? 1 : 0;
     }
-    if (TMA) ++phase;
+    ++phase;
     __syncthreads();
     if (!*s_ok) return;
   }
@@ -526,7 +507,7 @@ __device__ __forceinline__ void tile2d_body(const TileArgs& a, const CUtensorMap
   }
 }
 
-template <int P, int FLUX, int MODE, int TW, int TH, int NY = 0, bool GC = false, bool TMA = true>
+template <int P, int FLUX, int MODE, int TW, int TH, int NY = 0>
 __global__ void __launch_bounds__(TW * TH, 2)
     residual2d_tile_kernel(const TileArgs a, const __grid_constant__ CUtensorMap mapU,
                            const __grid_constant__ CUtensorMap mapB) {
@@ -537,7 +518,7 @@ __global__ void __launch_bounds__(TW * TH, 2)
     fence_mbar_init();
   }
   uint32_t phase = 0;
-  tile2d_body<P, FLUX, MODE, TW, TH, vol_unroll<P>(), NY, GC, TMA>(a, &mapU, &mapB, blockIdx.x * TW, blockIdx.y * TH,
+  tile2d_body<P, FLUX, MODE, TW, TH, vol_unroll<P>(), NY>(a, &mapU, &mapB, blockIdx.x * TW, blockIdx.y * TH,
                                                              smraw, phase);
   pdl_trigger();
 }

@@ -196,7 +196,7 @@ __device__ __forceinline__ bool cols_load(const ColArgs& a, const CUtensorMap* m
   // edge slot s of the tile (left, right, bottom, top): the neighbour across it -- the next element of the row or
   // column, or at the domain's edges what the neighbour table says -- and its face nodes.  A thread takes
   // node j of every field of one slot, all loads in flight.  (Offsets into a state are 32-bit counts of
-  // values: 2^32 of them in each of a context's seven buffers is more than the GPU's memory.)
+  // values: dgb_create refuses larger states.)
   const unsigned plane = ld;
   for (int k = tid; k < N1 * Dm::NEDGE; k += NT) {
     const int s = k % Dm::NEDGE, j = k / Dm::NEDGE;
@@ -382,7 +382,7 @@ __device__ __forceinline__ void cols_body(const ColArgs& a, const ColTab& tab, c
         if (code == -3) tr[1][g] = -tr[1][g];
       }
     }
-    double Ff[NF + 1][N1];  // lifted along the face; fields, then alpha as its right-hand element sees it
+    double Ff[NF + 1][N1];  // lifted along the face; fields, then alpha as its left-hand element sees it
 #pragma unroll
     for (int g = 0; g < N1; ++g) {
       double L[NF], R[NF], F2[NF], nc2;

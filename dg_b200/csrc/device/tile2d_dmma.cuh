@@ -21,12 +21,13 @@
 // The accumulators then hold M^-1 R; the stage update reads the stage base from global memory.
 // FP64 throughout: the sums run in another order than the scalar kernel's (differences of order
 // 1e-16 relative).  No mass fractions, GAMNCON, SSP and RK4 stages.
-// Measured on B200 (1024 x 512 stage launch): 15.4 warps per SM against the scalar kernel's 7.8,
-// but 298.5 us against 292 us.  The FP64 tensor rate equals the FP64 vector rate (36.9 TFLOP/s for
+// Measured on B200 (1024 x 512 stage launch): 15.4 warps per SM against the 7.8 of the scalar kernel with one thread
+// per element (tile2d.cuh), but 298.5 us against 292 us.  The FP64 tensor rate equals the FP64 vector rate (36.9 TFLOP/s for
 // both at 8+ warps per SM), so DMMA saves issue slots, not FP64 pipe time; without the scalar
 // kernel's sum factorisation the contractions need ~30 % more FMAs, and preparing the fragments
 // (tile loads, deviations, table loads, node 8, face gathers) costs what the DMMAs save in DFMA
-// instructions.  Kept as an alternative (DGB_TILE_KERNEL=dmma); the scalar kernel is the default.
+// instructions.  Kept as an alternative (DGB_TILE_KERNEL=dmma); the default is
+// residual2d_cols_kernel (50 us at 512 x 256, this one 92).
 #pragma once
 #include "tile2d.cuh"
 
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(DMMA_THREADS, 2)
   // (the first barrier inside tile_stage_in orders the table stores before their use)
   uint32_t phase = 0;
   const int tx0 = blockIdx.x * TW, ty0 = blockIdx.y * TH;
-  if (!tile_stage_in<P, TW, TH, 0, true>(a, &mapU, tx0, ty0, smraw, phase, tid, DMMA_THREADS)) return;
+  if (!tile_stage_in<P, TW, TH, 0>(a, &mapU, tx0, ty0, smraw, phase, tid, DMMA_THREADS)) return;
 
   const double* Us = reinterpret_cast<const double*>(smraw + Dm::off_tile);  // [NF*NS][NT]
   double* HL = reinterpret_cast<double*>(smraw + Dm::off_halo);
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(DMMA_THREADS, 2)
   double* HU = HD + TW * NF * N1;
   double* Fs = reinterpret_cast<double*>(smraw + Dm::off_face);
   const int* codes = reinterpret_cast<const int*>(smraw + Dm::head_bytes);
-  tile_face_fluxes<P, FLUX, TW, TH, 0, false>(Us, HL, HR, HD, HU, codes, Fs, tid, DMMA_THREADS, 0, Dm::NXF + Dm::NYF, 0);
+  tile_face_fluxes<P, FLUX, TW, TH, 0>(Us, HL, HR, HD, HU, codes, Fs, tid, DMMA_THREADS, 0, Dm::NXF + Dm::NYF, 0);
   __syncthreads();
 
   const int lane = tid & 31, warp = tid >> 5;

@@ -33,9 +33,9 @@ using namespace dgb;
 namespace {
 
 // residual tile shapes of the 2D classes: width, height (elements).  32 x 2 first: two CTAs of 256 threads
-// per SM at p = 2 (the others: one of 512), the fastest in the single-problem kernel too.  unroll is part
-// of the tuning interface; the quadrature loops are always unrolled now, so both 32 x 4 entries run
-// the same kernel.
+// per SM at p = 2 (the others: one of 512), the fastest of them (55 us per 512 x 256 launch in the single-problem
+// kernel, whose 16 x 2 tiles take 52).  unroll is part of the tuning interface; the quadrature loops are always
+// unrolled now, so both 32 x 4 entries are the same kernel and the autotuner times the first.
 struct Shape2 {
   int tw, th, unroll;
 };
@@ -494,7 +494,7 @@ extern "C" int dgb_batch_autotune(dgb_batch* b, int reps) {
     };
     std::vector<Cand> cand;
     if (k.D == 2) {
-      for (int s : k.valid_shapes)
+      for (int s : k.valid_shapes) if (kShapes2[s].unroll == 1)
         for (int ps : {0, 1}) cand.push_back({s, 0, ps});
     } else {
       for (int ch : kChunks1)

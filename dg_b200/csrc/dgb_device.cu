@@ -242,18 +242,20 @@ int residual_dispatch(dgb_ctx* c, const StageArgs& a) {
   return set_error(DGB_ERR_UNSUPPORTED, "no residual kernel for this (dim, p, flux)");
 }
 
-template <int P, int METHOD, int NY = 0>
+// both passes through X: any element order; structured grids' hrl / m2l are limit2d_out's, their prl (METHOD 1 on
+// primitive variables) is here
+template <int P, int METHOD>
 void launch_lim2d(dgb_ctx* c, double* U) {
   ProfScope ps(c, KC_LIMITER);
   const LimArgs la{c->ld, c->ne};
-  if (c->rowmajor) {
+  if (METHOD == 1 && c->rowmajor) {
     dim3 gx((c->nx + 29) / 30, c->ny), bx(32, P + 1);
-    launch_pdl(c, lim2d_xpass_tile_kernel<P, METHOD, NY>, gx, bx, 0, la, c->nx, (const double*)U,
+    launch_pdl(c, lim2d_xpass_tile_kernel<P, 1, 0>, gx, bx, 0, la, c->nx, (const double*)U,
                (const int*)c->nbr, c->X, (const DevScalars*)c->scal);
     dim3 gy((c->nx + 31) / 32, (c->ny + 3) / 4, P + 1), by(32, 6);
-    launch_pdl(c, lim2d_ypass_tile_kernel<P, METHOD, NY>, gy, by, 0, la, c->nx, c->ny, (const double*)c->X,
+    launch_pdl(c, lim2d_ypass_tile_kernel<P, 1, 0>, gy, by, 0, la, c->nx, c->ny, (const double*)c->X,
                (const int*)c->nbr, U, (const DevScalars*)c->scal);
-  } else if (NY == 0) {
+  } else {
     dim3 grid((c->ne + 127) / 128, P + 1);
     lim2d_xpass_kernel<P, METHOD><<<grid, 128, 0, c->st>>>(la, U, c->nbr, c->X, c->scal);
     lim2d_ypass_kernel<P, METHOD><<<grid, 128, 0, c->st>>>(la, c->X, c->nbr, U, c->scal);
@@ -405,17 +407,11 @@ void launch_learned_limiter(dgb_ctx* c, double* U, bool score) {
 
 // in-place limiting of a state buffer with the context's limiter (rescore: the learned indicator
 // scores U first; the time steppers score once per step and pass false)
-// hrl / m2l with NY passive mass fractions; key = p * 10 + limiter
+// 1D hrl / m2l with NY passive mass fractions; key = p * 10 + limiter
 template <int NY>
 int limit_ny(dgb_ctx* c, double* U, int key) {
-#define L2Y(P, M) case P * 10 + M: launch_lim2d<P, M, NY>(c, U); return 0;
 #define L1Y(P, M) case P * 10 + M: launch_lim1d<P, M, NY>(c, U); return 0;
-  if (c->D == 2) {
-    switch (key) { L2Y(1, 1) L2Y(1, 2) L2Y(2, 1) L2Y(2, 2) L2Y(3, 1) L2Y(3, 2) default: break; }
-  } else {
-    switch (key) { L1Y(1, 1) L1Y(1, 2) L1Y(2, 1) L1Y(2, 2) L1Y(3, 1) L1Y(3, 2) default: break; }
-  }
-#undef L2Y
+  switch (key) { L1Y(1, 1) L1Y(1, 2) L1Y(2, 1) L1Y(2, 2) L1Y(3, 1) L1Y(3, 2) default: break; }
 #undef L1Y
   return set_error(DGB_ERR_UNSUPPORTED, "limiter not available with mass fractions");
 }
@@ -867,7 +863,7 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
     // learned-indicator scoring: tcgen05 GEMMs (DGB_INDICATOR_KERNEL=mma: the mma.sync form)
     const char* ik = std::getenv("DGB_INDICATOR_KERNEL");
     c->ind_tc = !(ik && std::string(ik) == "mma");
-    // p = 2 FP64 tiled stages: the one-thread-per-element kernel; DGB_TILE_KERNEL=dmma selects the
+    // p = 2 FP64 stages: the column kernel (tile2d_cols.cuh); DGB_TILE_KERNEL=dmma selects the
     // form with the basis contractions on the FP64 tensor cores (measured slower on B200, whose
     // FP64 tensor rate equals its FP64 vector rate)
     const char* tk = std::getenv("DGB_TILE_KERNEL");
@@ -902,6 +898,10 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
   c->tiled_full = c->tile_tma && P.nx % TILE_W == 0 && P.ny % tile_h_for(P.p, P.N_Y) == 0;
   // structured grids, up to three mass fractions: the residual of tile2d_cols.cuh on any extents
   c->cols = c->rowmajor && P.p <= 3 && P.N_Y <= 3;
+  if (c->cols && c->nstate >= (1ull << 32)) {  // whose offsets into a state are 32-bit counts of values
+    delete c;
+    return set_error(DGB_ERR_UNSUPPORTED, "a state of 2^32 values or more (six buffers of that size are 206 GB)");
+  }
   // hrl / m2l: both limiter passes in one launch
   c->lim_out = c->rowmajor && (P.limiter == DGB_LIM_HRL || P.limiter == DGB_LIM_M2L) && P.N_Y <= 3;
   c->nmass = P.N_Y;
@@ -1010,7 +1010,8 @@ extern "C" int dgb_create(const dgb_problem* prob, int device, dgb_ctx** out) {
     }
   }
   if (c->cols) cols_setup(c);
-  if (c->tiled && !c->tiled_full) {
+  if (c->tiled && !c->tiled_full && (P.N_Y > 3 || P.p == 3 || c->tile_dmma)) {
+    // (of many-mass-fraction, limited cubic and DMMA residuals; the column kernel cuts its tiles instead)
     // the right strip (rows of the full tiles) and the top strip (all columns), in element order
     const int th = tile_h_for(P.p, P.N_Y), nxt = P.nx / TILE_W * TILE_W, nyt = P.ny / th * th;
     std::vector<int> left;

@@ -69,18 +69,16 @@ inline TileArgs tile_args(dgb_ctx* c, const StageArgs& s) {
   return a;
 }
 
-template <int P, int FLUX, int MODE, int NY = 0, bool GC = false, bool TMA = true>
+template <int P, int FLUX, int MODE, int NY>
 void launch_tile2d(dgb_ctx* c, const StageArgs& s) {
   constexpr int TH = tile_h_for(P, NY);
   using Dm = TileDims<P, TILE_W, TH, NY>;
   constexpr size_t smem = Dm::smem_bytes;
-  auto k = residual2d_tile_kernel<P, FLUX, MODE, TILE_W, TH, NY, GC, TMA>;
+  auto k = residual2d_tile_kernel<P, FLUX, MODE, TILE_W, TH, NY>;
   allow_dynamic_smem(k, smem);
   const TileArgs a = tile_args(c, s);
-  // (without TMA the maps are not read: the tile loads are plain)
-  const CUtensorMap& mu = TMA ? map_of(c, s.U) : c->mapA;
-  const CUtensorMap& mb = !TMA ? c->mapA
-                          : MODE == MODE_SSP ? map_of(c, s.Ubase) : MODE == MODE_RK4 && s.Uacc ? map_of(c, s.Uacc) : mu;
+  const CUtensorMap& mu = map_of(c, s.U);
+  const CUtensorMap& mb = MODE == MODE_SSP ? map_of(c, s.Ubase) : MODE == MODE_RK4 && s.Uacc ? map_of(c, s.Uacc) : mu;
   dim3 grid(c->nx / TILE_W, c->ny / TH);
   ProfScope ps(c, KC_RESIDUAL);
   // (not programmatic: the kernel reads its stage base between its stores, with read-only loads; plain ones, which
