@@ -471,10 +471,10 @@ __device__ __forceinline__ void limit_slice(int phys, const double* vL, const do
     HR::moments(vC, DC);
     HR::moments(vL, DL);
     HR::moments(vR, DR);
-    HR::limit(DL, DC, DR, lim);
+    HR::limit(DL, DC, DR, vC, lim);
   } else if (phys == 2 || phys == 3) {
     HR::moments(vC, DC);
-    HR::flat(DC, lim);
+    HR::flat(DC, vC, lim);
   } else {
     HR::mono(vC, lim);
   }

@@ -106,9 +106,9 @@ __device__ __forceinline__ void lim2d_xpass_body(const LimArgs la, int nx, const
     if (ph == 0) {
 #pragma unroll
       for (int m = 0; m < NM; ++m) { DL[m] = A[k][sl][m][tx - 1]; DR[m] = A[k][sl][m][tx + 1]; }
-      HR::limit(DL, DC, DR, lim[k]);
+      HR::limit(DL, DC, DR, q[k], lim[k]);
     } else if (ph == 2 || ph == 3) {
-      HR::flat(DC, lim[k]);
+      HR::flat(DC, q[k], lim[k]);
     } else {
       HR::mono(q[k], lim[k]);
     }
@@ -223,9 +223,9 @@ __device__ __forceinline__ void lim2d_ypass_body(const LimArgs la, int nx, int n
     if (ph == 0) {
 #pragma unroll
       for (int m = 0; m < NM; ++m) { DD[m] = B[k][m][ty - 1][tx]; DU[m] = B[k][m][ty + 1][tx]; }
-      HR::limit(DD, DC, DU, lim[k]);
+      HR::limit(DD, DC, DU, col[k], lim[k]);
     } else if (ph == 2 || ph == 3) {
-      HR::flat(DC, lim[k]);
+      HR::flat(DC, col[k], lim[k]);
     } else {
       HR::mono(col[k], lim[k]);
     }
@@ -361,10 +361,10 @@ __device__ __forceinline__ void lim2d_body(const LimArgs la, int nx, int ny, con
         DL[m] = __shfl_up_sync(0xffffffffu, DC[m], 1);
         DR[m] = __shfl_down_sync(0xffffffffu, DC[m], 1);
       }
-      HR::limit(DL, DC, DR, lim);
+      HR::limit(DL, DC, DR, q, lim);
       if (phx != 0) {
         if (phx == 4 || (METHOD == 1 && phx == 3 && k == 1)) HR::mono(q, lim);
-        else HR::flat(DC, lim);
+        else HR::flat(DC, q, lim);
       }
       HR::lag(lim, o[k]);
 #pragma unroll
@@ -424,7 +424,7 @@ __device__ __forceinline__ void lim2d_body(const LimArgs la, int nx, int ny, con
 #pragma unroll
       for (int iy = 0; iy < N1; ++iy) w[iy] = b[N1 * iy * PITCH + 32];
       moments(w, DU);
-      HR::limit(DD, DC, DU, lim);
+      HR::limit(DD, DC, DU, c, lim);
     } else if (phy == 4 || (METHOD == 1 && phy == 3 && k == 2)) {
       if constexpr (P == 3) {
 #pragma unroll
@@ -433,7 +433,7 @@ __device__ __forceinline__ void lim2d_body(const LimArgs la, int nx, int ny, con
         HR::mono(c, lim);
       }
     } else {
-      HR::flat(DC, lim);
+      HR::flat(DC, c, lim);
     }
     HR::lag(lim, o[k]);
 #pragma unroll
