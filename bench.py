@@ -969,7 +969,7 @@ def main(argv=None) -> int:
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
     peak = peaks.get("hbm_gbs", 6650.0)
     traffic, traffic_stages = None, None
-    tf = ROOT / "profiles" / "residual2d_tile_p2_512x256_traffic.json"
+    tf = ROOT / "profiles" / "residual2d_cols_p2_512x256_traffic.json"
     if tf.exists():
         tj = json.loads(tf.read_text())
         traffic = tj.get("bytes_per_launch_full_size")

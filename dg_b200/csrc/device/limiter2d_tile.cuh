@@ -288,11 +288,11 @@ namespace dgb {
 // the x-limited nodes in shared memory; the y pass (warp = x-column) reads its column and those of
 // the rows above and below from there, so the x-limited state never goes to memory.  Uout must not alias U.
 // Per stage of m2l, against the two passes through a global scratch: p = 2, 512 x 256: 52 -> 33 us; p = 3,
-// 1024 x 512: 329 -> 304 (hrl 292 -> 247; HrTab3's transforms have 16 products, with HrSums it would be 212);
+// 1024 x 512: 329 -> 315 (HrTab3's transforms have 16 products, with HrSums it would be 212);
 // p = 1, 1024 x 256: 34 -> 23.  The two passes were FP64-bound at half the memory
 // rate (2,240 FP64 instructions per p = 2 element, 1,280 now with the halo rows' second x pass) and moved
-// 35 B per value; this moves 16 plus halos (15 us at the copy rate) and waits on its loads: long
-// scoreboard 4.3 of 12 stall cycles at 36 warps per SM, FP64 pipe 37 %.
+// 35 B per value; this moves 16 plus halos (15 us at the copy rate) and waits on its loads and its dependent
+// operations: 27 warps per SM, issue 55 %, FP64 pipe 34 % (p = 3: 22 warps, 60 %, 54 %).
 // Rows per tile: more rows repeat less x work, fewer leave room for a second CTA.  p = 2: 2 rows 41 us,
 // 3: 35, 4 (two CTAs): 35, 6: 35, 8: 33; p = 3 (with HrSums): 1: 436, 2: 242, 3: 224, 4: 212; p = 1: 4: 26, 6: 27, 8 (two
 // CTAs): 23, 8 (three): 33, 14: 35.  One thread per element with all slices in registers (164
